@@ -398,7 +398,7 @@ struct BatchPlan {
   std::vector<wl::ReduceJob> rjobs;
   std::vector<float> inst;
   size_t part_total = 0, out_total = 0;
-  int flat_total = 0;
+  int reduce_blocks = 0;
 };
 
 int batch_plan(wl_ctx *ctx, int njobs, const wl_job *jobs, int points, BatchPlan *P) {
@@ -472,14 +472,11 @@ int batch_plan(wl_ctx *ctx, int njobs, const wl_job *jobs, int points, BatchPlan
       P->perm_total += (size_t)n;
     }
     wl::ReduceJob &rj = P->rjobs[i];
-    rj.n_chunks = a.n_chunks;
-    rj.cpg = J.group / lcs[i];
-    rj.lpg = J.group;
-    rj.ninst = n;
-    rj.nF = J.nF;
-    rj.first = P->flat_total;
+    rj.shape = {nullptr, a.n_chunks, J.group / lcs[i], 1, J.group, n, J.nF};
+    rj.ti = wl::reduce_instances(n, J.nF, e.Nl / J.group);
+    rj.first = P->reduce_blocks;
     rj.out_group = (double *)(uintptr_t)(out_off[i]);
-    P->flat_total += n * J.nF;
+    P->reduce_blocks += wl::reduce_blocks(rj);
     if (!wl::batch_in_kernel(kprofs[i])) {
       P->side.push_back(i);
       continue;
@@ -532,11 +529,11 @@ int batch_run(wl_ctx *ctx, int njobs, const wl_job *jobs, int flags, int points,
     a.status = ctx->status.p;
     if (a.perm) a.perm = ctx->b_perm.p + ((size_t)(uintptr_t)a.perm - 1);
     wl::ReduceJob &rj = P.rjobs[i];
-    rj.partial = a.partial;
-    const int ng = a.Nl / rj.lpg;
+    rj.shape.partial = a.partial;
+    const int ng = a.Nl / rj.shape.lpg;
     rj.out_group = ctx->b_out.p + (size_t)(uintptr_t)rj.out_group;
-    rj.out_mean = rj.out_group + (size_t)n * rj.nF * ng;
-    rj.out_sem = rj.out_mean + (size_t)n * rj.nF;
+    rj.out_mean = rj.out_group + (size_t)n * a.nF * ng;
+    rj.out_sem = rj.out_mean + (size_t)n * a.nF;
   }
   unsigned char *meta = ctx->b_meta.p;
   WL_CHECK(ctx, cudaMemcpyAsync(ctx->b_inst.p, P.inst.data(), sizeof(float) * P.inst.size(),
@@ -581,7 +578,7 @@ int batch_run(wl_ctx *ctx, int njobs, const wl_job *jobs, int flags, int points,
       const wl::SweepArgs &a = P.jobs[i];
       e = wl::launch_sweep(a.kprof, a.fermion != 0, a.nint, a, ctx->stream);
     }
-    if (e == cudaSuccess) e = wl::launch_batch_reduce(rjd, njobs, P.flat_total, ctx->stream);
+    if (e == cudaSuccess) e = wl::launch_batch_reduce(rjd, njobs, P.reduce_blocks, ctx->stream);
     return e;
   };
   cudaError_t ce = cudaEventRecord(e0, ctx->stream);
@@ -945,8 +942,8 @@ static int run_eval(wl_ctx *ctx, const Ensemble &e, int kprof, const FieldDev &f
     WL_CHECK(ctx, wl::launch_loopwarp(kprof, fermion, nint, a, ctx->stream));
     ctx->last_kind = "loop-parallel";
   }
-  WL_CHECK(ctx, wl::launch_group_reduce(ctx->partial.p, n_chunks, cpg, group, ninst, nF, dg, dm,
-                                        ds, ctx->stream));
+  const wl::ReduceShape rs = {ctx->partial.p, n_chunks, cpg, 1, group, ninst, nF};
+  WL_CHECK(ctx, wl::launch_group_reduce(rs, dg, dm, ds, ctx->stream));
   return WL_OK;
 }
 
@@ -1466,8 +1463,8 @@ int wl_eval_plain(wl_ctx *ctx, int handle, const wl_field *field, int ninst, con
     WL_CHECK(ctx, wl::launch_plain(kprof, field->fermion != 0, field->nint, a, i, ctx->stream));
   WL_CHECK(ctx, cudaEventRecord(e1, ctx->stream));
   double *dg = ctx->out.p, *dm = dg + (size_t)ninst * nF * ng, *ds = dm + (size_t)ninst * nF;
-  WL_CHECK(ctx, wl::launch_group_reduce(ctx->partial.p, e.Nl, group, group, ninst, nF, dg, dm, ds,
-                                        ctx->stream));
+  const wl::ReduceShape rs = {ctx->partial.p, e.Nl, group, 1, group, ninst, nF};
+  WL_CHECK(ctx, wl::launch_group_reduce(rs, dg, dm, ds, ctx->stream));
   WL_CHECK(ctx, cudaEventSynchronize(e1));
   float ms = 0.0f;
   cudaEventElapsedTime(&ms, e0, e1);

@@ -8,6 +8,7 @@
 // host orders tiles by decreasing cost so the queue drains evenly.
 #include "wl_device.cuh"
 #include "wl_internal.h"
+#include "wl_reduce.cuh"
 #include "wl_sweep.cuh"
 
 namespace wl {
@@ -120,42 +121,23 @@ __global__ void __launch_bounds__(kSweepThreads, kBatchMinBlocks)
   }
 }
 
-// one thread per (job, instance, flux value); jobs located by binary search
-__global__ void batch_reduce_kernel(const ReduceJob *__restrict__ jobs, int njobs, int total) {
-  const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= total) return;
+// the jobs' reductions as one launch: a CTA's job by binary search
+__global__ void __launch_bounds__(kReduceThreads)
+    batch_reduce_kernel(const ReduceJob *__restrict__ jobs, int njobs) {
+  const int b = blockIdx.x;
   int lo = 0, hi = njobs - 1;
   while (lo < hi) {
     const int mid = (lo + hi + 1) / 2;
-    if (jobs[mid].first <= idx) lo = mid;
+    if (jobs[mid].first <= b) lo = mid;
     else hi = mid - 1;
   }
   const ReduceJob J = jobs[lo];
-  const int local = idx - J.first;
-  const int inst = local % J.ninst, j = local / J.ninst;
-  const int ng = J.n_chunks / J.cpg;
-  const double inv = 1.0 / (double)J.lpg;
-  double mean = 0.0;
-  for (int g = 0; g < ng; ++g) {
-    double s0 = 0.0, s1 = 0.0, s2 = 0.0;
-    for (int c = g * J.cpg; c < (g + 1) * J.cpg; ++c) {
-      const size_t b = ((size_t)(c * J.nF + j) * 3) * J.ninst + inst;
-      s0 += J.partial[b];
-      s1 += J.partial[b + J.ninst];
-      s2 += J.partial[b + 2 * (size_t)J.ninst];
-    }
-    const double v = 1.0 + (8.0 / 3.0 * (s0 * inv) - 2.0 * (s1 * inv) + 1.0 / 3.0 * (s2 * inv));
-    J.out_group[((size_t)inst * J.nF + j) * ng + g] = v;
-    mean += v;
-  }
-  mean /= (double)ng;
-  double ss = 0.0;
-  for (int g = 0; g < ng; ++g) {
-    const double v = J.out_group[((size_t)inst * J.nF + j) * ng + g];
-    ss += (v - mean) * (v - mean);
-  }
-  J.out_mean[(size_t)inst * J.nF + j] = mean;
-  J.out_sem[(size_t)inst * J.nF + j] = ng > 1 ? sqrt(ss / ((double)ng * (ng - 1.0))) : 0.0;
+  const int nx = (J.shape.ninst + J.ti - 1) / J.ti;
+  reduce_block(J.shape, (b - J.first) % nx * J.ti, (b - J.first) / nx, J.ti, J.out_group,
+               [&](size_t at, double mean, double sem) {
+                 J.out_mean[at] = mean;
+                 J.out_sem[at] = sem;
+               });
 }
 
 // The plain per-instance kernel: one thread per loop walking its points from
@@ -273,9 +255,8 @@ cudaError_t launch_batch(const BatchArgs &a, int grid, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-cudaError_t launch_batch_reduce(const ReduceJob *jobs, int njobs, int total, cudaStream_t s) {
-  const int bs = 128;
-  batch_reduce_kernel<<<(total + bs - 1) / bs, bs, 0, s>>>(jobs, njobs, total);
+cudaError_t launch_batch_reduce(const ReduceJob *jobs, int njobs, int blocks, cudaStream_t s) {
+  batch_reduce_kernel<<<blocks, kReduceThreads, 0, s>>>(jobs, njobs);
   return cudaGetLastError();
 }
 

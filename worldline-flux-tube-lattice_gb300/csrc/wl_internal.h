@@ -69,11 +69,32 @@ inline __host__ __device__ int sweep_tile_instances(int kprof, int nint) {
 struct BatchTile {
   int job, tile_x, chunk, cost;
 };
-struct ReduceJob {  // per job: where its partial sums and outputs live
+// Partial sums [n_chunks * inner][nF][3][ninst] of one job: cpg chunks per group
+// of lpg loops, each chunk one sum (inner = 1) or its inner loops one by one.
+struct ReduceShape {
   const double *partial;
-  double *out_group, *out_mean, *out_sem;
-  int n_chunks, cpg, lpg, ninst, nF, first;  // first: flat (instance, F) index
+  int n_chunks, cpg, inner, lpg, ninst, nF;
 };
+constexpr int kReduceThreads = 256;
+// Instances per CTA of a reduction: 32 (a warp reads 256 contiguous bytes)
+// when that fills the chip, else fewer, down to the 4 of a 32-byte sector, so
+// that more CTAs run and more groups are summed at once.
+inline int reduce_instances(int ninst, int nF, int ng) {
+  int ti = 32;
+  while (ti > 1 && ti / 2 >= ninst) ti /= 2;
+  while (ti > 4 && (long long)((ninst + ti - 1) / ti) * nF < 304 && kReduceThreads / ti < ng)
+    ti /= 2;
+  return ti;
+}
+struct ReduceJob {  // per job: where its partial sums and outputs live
+  ReduceShape shape;
+  double *out_group, *out_mean, *out_sem;
+  int ti, first;  // instances per CTA, first CTA of the job
+};
+// CTAs of one job's reduction
+inline int reduce_blocks(const ReduceJob &r) {
+  return (r.shape.ninst + r.ti - 1) / r.ti * r.shape.nF;
+}
 struct BatchArgs {
   const SweepArgs *jobs;
   const BatchTile *tiles;
@@ -81,7 +102,7 @@ struct BatchArgs {
   int *counter;  // next tile to take
 };
 cudaError_t launch_batch(const BatchArgs &a, int grid, cudaStream_t s);
-cudaError_t launch_batch_reduce(const ReduceJob *jobs, int njobs, int total, cudaStream_t s);
+cudaError_t launch_batch_reduce(const ReduceJob *jobs, int njobs, int blocks, cudaStream_t s);
 // largest number of batch-kernel CTAs resident per SM
 int batch_max_ctas_per_sm();
 // every profile batches; the heavy ones (periodic, spline, fixflux) are not
@@ -122,9 +143,8 @@ cudaError_t launch_loopwarp(int profile, bool fermion, int nint, const LoopArgs 
                             cudaStream_t s);
 
 // partial sums -> per-group <W>, mean and SEM over groups
-cudaError_t launch_group_reduce(const double *partial, int n_chunks, int chunks_per_group,
-                                int loops_per_group, int ninst, int nF, double *out_group,
-                                double *out_mean, double *out_sem, cudaStream_t s);
+cudaError_t launch_group_reduce(const ReduceShape &r, double *out_group, double *out_mean,
+                                double *out_sem, cudaStream_t s);
 
 // EV(): mean over an index list of per-loop W factors (partial with
 // ninst = 1, nF = 1) and the Richardson combination; writes one double.

@@ -4,6 +4,7 @@
 
 #include "wl_device.cuh"
 #include "wl_internal.h"
+#include "wl_reduce.cuh"
 
 namespace wl {
 
@@ -47,47 +48,15 @@ cudaError_t launch_loopwarp(int profile, bool fermion, int nint, const LoopArgs 
 }
 
 // ---------------------------------------------------------- reductions --
-// One thread per (instance, flux value): group sums over the group's chunks
-// in chunk order (the result of an instance does not depend on how many
-// other instances share the launch), the Richardson combination
-// 8/3 W_N - 2 W_N/2 + 1/3 W_N/4 (Integrand.c:400), then mean and standard
-// error over the groups.  The partial sums hold W - 1 per loop; the weights
-// sum to one, so <W> = 1 + the same combination of the deviations.
-__global__ void group_reduce_kernel(const double *__restrict__ partial, int n_chunks,
-                                    int cpg, int lpg, int ninst, int nF,
-                                    double *__restrict__ out_group,
-                                    double *__restrict__ out_mean,
-                                    double *__restrict__ out_sem) {
-  const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= ninst * nF) return;
-  const int inst = idx % ninst, j = idx / ninst;
-  const int ng = n_chunks / cpg;
-  const double inv = 1.0 / (double)lpg;
-  auto group_value = [&](int g) {
-    double s0 = 0.0, s1 = 0.0, s2 = 0.0;
-    for (int c = g * cpg; c < (g + 1) * cpg; ++c) {
-      const size_t base = ((size_t)(c * nF + j) * 3) * ninst + inst;
-      s0 += partial[base];
-      s1 += partial[base + ninst];
-      s2 += partial[base + 2 * (size_t)ninst];
-    }
-    return 1.0 + (8.0 / 3.0 * (s0 * inv) - 2.0 * (s1 * inv) + 1.0 / 3.0 * (s2 * inv));
-  };
-  double mean = 0.0;
-  for (int g = 0; g < ng; ++g) {
-    const double v = group_value(g);
-    if (out_group) out_group[((size_t)inst * nF + j) * ng + g] = v;
-    mean += v;
-  }
-  mean /= (double)ng;
-  double ss = 0.0;
-  for (int g = 0; g < ng; ++g) {
-    const double v = out_group ? out_group[((size_t)inst * nF + j) * ng + g] : group_value(g);
-    ss += (v - mean) * (v - mean);
-  }
-  if (out_mean) out_mean[(size_t)inst * nF + j] = mean;
-  if (out_sem)
-    out_sem[(size_t)inst * nF + j] = ng > 1 ? sqrt(ss / ((double)ng * (ng - 1.0))) : 0.0;
+// <W> per group (Integrand.c:400), mean and standard error over the groups
+__global__ void __launch_bounds__(kReduceThreads)
+    group_reduce_kernel(const ReduceShape R, int ti, double *__restrict__ out_group,
+                        double *__restrict__ out_mean, double *__restrict__ out_sem) {
+  reduce_block(R, blockIdx.x * ti, blockIdx.y, ti, out_group,
+               [&](size_t at, double mean, double sem) {
+                 if (out_mean) out_mean[at] = mean;
+                 if (out_sem) out_sem[at] = sem;
+               });
 }
 
 // ------------------------------------------------ lattice instance order --
@@ -152,12 +121,11 @@ cudaError_t launch_order_instances(const float *cx, const float *cy, const float
   return cudaGetLastError();
 }
 
-cudaError_t launch_group_reduce(const double *partial, int n_chunks, int cpg, int lpg,
-                                int ninst, int nF, double *out_group, double *out_mean,
+cudaError_t launch_group_reduce(const ReduceShape &r, double *out_group, double *out_mean,
                                 double *out_sem, cudaStream_t s) {
-  const int n = ninst * nF, bs = 128;
-  group_reduce_kernel<<<(n + bs - 1) / bs, bs, 0, s>>>(partial, n_chunks, cpg, lpg, ninst,
-                                                        nF, out_group, out_mean, out_sem);
+  const int ti = reduce_instances(r.ninst, r.nF, r.n_chunks / r.cpg);
+  const dim3 grid((r.ninst + ti - 1) / ti, r.nF);
+  group_reduce_kernel<<<grid, kReduceThreads, 0, s>>>(r, ti, out_group, out_mean, out_sem);
   return cudaGetLastError();
 }
 

@@ -195,7 +195,7 @@ extern "C" int wl_eval_noalloc(const float *dev_loops, int Nl, int ppl, const wl
     ce = wl::launch_loopwarp(kprof, field->fermion != 0, field->nint, a, s);
   }
   if (ce == cudaSuccess)
-    ce = wl::launch_group_reduce(partial, n_chunks, cpg, group, ninst, nF, dev_out_group,
+    ce = wl::launch_group_reduce({partial, n_chunks, cpg, 1, group, ninst, nF}, dev_out_group,
                                  dev_out_mean, dev_out_sem, s);
   int st = 0;
   if (ce == cudaSuccess) ce = cudaMemcpyAsync(&st, status, sizeof(int), cudaMemcpyDeviceToHost, s);

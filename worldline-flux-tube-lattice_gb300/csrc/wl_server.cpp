@@ -489,15 +489,11 @@ bool admit(wl_server *s) {
     if (R->kprof == wl::kLattice) a.perm = (const int *)(dmem + R->o_perm);
     wl::ReduceJob &rj = R->rj;
     memset(&rj, 0, sizeof(rj));
-    rj.partial = d_part;
     rj.out_group = d_out;
     rj.out_mean = d_out + (size_t)n * nF * R->ng;
     rj.out_sem = rj.out_mean + (size_t)n * nF;
-    rj.n_chunks = R->n_chunks;
-    rj.cpg = R->q.group / R->lc;
-    rj.lpg = R->q.group;
-    rj.ninst = n;
-    rj.nF = nF;
+    rj.shape = {d_part, R->n_chunks, R->q.group / R->lc, 1, R->q.group, n, nF};
+    rj.ti = wl::reduce_instances(n, nF, R->ng);
     rj.first = 0;
     memcpy(pin + R->p_args, &a, sizeof(a));
     memcpy(pin + R->p_rj, &rj, sizeof(rj));
@@ -685,7 +681,7 @@ void launch_quantum(wl_server *s, int k) {
     ck(cudaStreamWaitEvent(st, s->ev_stop[k ^ 1], 0), "wait other stream");
     for (Req *R : closing) {
       const wl::ReduceJob *d_rj = (const wl::ReduceJob *)(R->dmem + R->o_rj);
-      ck(wl::launch_batch_reduce(d_rj, 1, R->ninst * R->q.nF, st), "reduce");
+      ck(wl::launch_batch_reduce(d_rj, 1, wl::reduce_blocks(R->rj), st), "reduce");
       char *po = R->pin + R->p_out;
       ck(cudaMemcpyAsync(po, R->dmem, sizeof(int), cudaMemcpyDeviceToHost, st), "status read");
       const double *src;
