@@ -398,45 +398,112 @@ __device__ __forceinline__ void step_normals(uint2 key, int k, int lg, double n[
   }
 }
 
-// One thread per loop.  A discrete Brownian bridge of unit proper time:
-// increments N(0, 2/N) per component (the kinetic weight exp(-1/4 int xdot^2)
-// of a unit loop), x_k = y_k - (k/N) y_N, then the mean is removed.  Two
-// passes over the same counter-based draws avoid storing the walk.
-__global__ void vloops_kernel(uint64_t seed, int first, int Nl, int ppl,
-                              float4 *__restrict__ out) {
-  const int l = blockIdx.x * blockDim.x + threadIdx.x;
-  if (l >= Nl) return;
+// A discrete Brownian bridge of unit proper time: increments N(0, 2/N) per
+// component (the kinetic weight exp(-1/4 int xdot^2) of a unit loop), x_k =
+// y_k - (k/N) y_N, then the mean is removed.  One CTA per loop: the draws are
+// counter-based, so every thread draws its own run of `per` consecutive
+// steps, the walk is the exclusive scan of the threads' sums (FP64, in thread
+// order) and the mean follows from the scan.  The increments wait for y_N in
+// shared memory (32 bytes a step) where they fit, else they are drawn again.
+//
+// Bound by the FP64 pipe (2 lanes per SM per clock; a log, a square root and
+// a sincospi for two of a step's four normals).  Generating, evaluating and
+// releasing 2048 loops of 1024 points took 12.6 ms with one thread per loop,
+// both passes drawing (11.4 ms of it the generator, the same for any loop count
+// up to the chip's threads), and takes 2.05 ms with one CTA per loop.
+constexpr int kVloopMaxThreads = 256;
+constexpr int kVloopMaxWarps = kVloopMaxThreads / 32;
+constexpr size_t kVloopMaxSmem = 200 * 1024;
+
+__global__ void __launch_bounds__(kVloopMaxThreads)
+    vloops_kernel(uint64_t seed, int first, int ppl, int keep, float4 *__restrict__ out) {
+  extern __shared__ __align__(16) double inc[];  // [ppl][4] when kept
+  __shared__ double wsum[kVloopMaxWarps][8];
+  const int l = blockIdx.x, t = threadIdx.x, lane = t & 31, w = t >> 5;
   const uint2 key = make_uint2((uint32_t)seed, (uint32_t)(seed >> 32));
   const double sigma = sqrt(2.0 / (double)ppl);
+  const int per = (ppl + blockDim.x - 1) / blockDim.x;
+  const int k0 = min(ppl, t * per), k1 = min(ppl, k0 + per);
+  // this thread's part of the walk: its end, and the sum of its points
   double y[4] = {0, 0, 0, 0}, sy[4] = {0, 0, 0, 0};
-  for (int k = 0; k < ppl; ++k) {
+  for (int k = k0; k < k1; ++k) {
     double n[4];
     step_normals(key, k, first + l, n);
+#pragma unroll
     for (int d = 0; d < 4; ++d) {
+      if (keep) inc[4 * (size_t)k + d] = n[d];
       sy[d] += y[d];
-      y[d] += sigma * n[d];
+      y[d] = fma(sigma, n[d], y[d]);
     }
   }
+  // exclusive scan of the ends over the CTA's threads
+  double pre[4], tot[4];
+#pragma unroll
+  for (int d = 0; d < 4; ++d) {
+    double s = y[d];
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const double u = __shfl_up_sync(0xffffffffu, s, off);
+      if (lane >= off) s += u;
+    }
+    if (lane == 31) wsum[w][d] = s;
+    pre[d] = __shfl_up_sync(0xffffffffu, s, 1);
+    if (lane == 0) pre[d] = 0.0;
+  }
+  __syncthreads();
+  const int nw = blockDim.x >> 5;
+#pragma unroll
+  for (int d = 0; d < 4; ++d) {
+    double base = 0.0;
+    tot[d] = 0.0;
+    for (int v = 0; v < nw; ++v) {
+      if (v < w) base += wsum[v][d];
+      tot[d] += wsum[v][d];
+    }
+    pre[d] += base;
+    // sum of the points: each of this thread's lies pre above its own walk
+    double s = fma((double)(k1 - k0), pre[d], sy[d]);
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
+    if (lane == 0) wsum[w][4 + d] = s;
+  }
+  __syncthreads();
   // mean of x_k = (1/N) sum y_k - y_N (N-1)/(2N)
   double mean[4];
-  for (int d = 0; d < 4; ++d)
-    mean[d] = sy[d] / (double)ppl - y[d] * ((double)(ppl - 1) / (2.0 * ppl));
-  double yy[4] = {0, 0, 0, 0};
+#pragma unroll
+  for (int d = 0; d < 4; ++d) {
+    double s = 0.0;
+    for (int v = 0; v < nw; ++v) s += wsum[v][4 + d];
+    mean[d] = s / (double)ppl - tot[d] * ((double)(ppl - 1) / (2.0 * ppl));
+  }
   float4 *o = out + (size_t)l * ppl;
-  for (int k = 0; k < ppl; ++k) {
+  for (int k = k0; k < k1; ++k) {
     const double fk = (double)k / (double)ppl;
-    o[k] = make_float4((float)(yy[0] - fk * y[0] - mean[0]), (float)(yy[1] - fk * y[1] - mean[1]),
-                       (float)(yy[2] - fk * y[2] - mean[2]), (float)(yy[3] - fk * y[3] - mean[3]));
+    o[k] = make_float4((float)(pre[0] - fk * tot[0] - mean[0]), (float)(pre[1] - fk * tot[1] - mean[1]),
+                       (float)(pre[2] - fk * tot[2] - mean[2]), (float)(pre[3] - fk * tot[3] - mean[3]));
     double n[4];
-    step_normals(key, k, first + l, n);
-    for (int d = 0; d < 4; ++d) yy[d] += sigma * n[d];
+    if (keep)
+#pragma unroll
+      for (int d = 0; d < 4; ++d) n[d] = inc[4 * (size_t)k + d];
+    else
+      step_normals(key, k, first + l, n);
+#pragma unroll
+    for (int d = 0; d < 4; ++d) pre[d] = fma(sigma, n[d], pre[d]);
   }
 }
 
 cudaError_t launch_vloops(uint64_t seed, int first, int Nl, int ppl, float4 *out,
                           cudaStream_t s) {
-  const int bs = 64;
-  vloops_kernel<<<(Nl + bs - 1) / bs, bs, 0, s>>>(seed, first, Nl, ppl, out);
+  int threads = 32;
+  while (threads < ppl && threads < kVloopMaxThreads) threads *= 2;
+  const size_t bytes = sizeof(double) * 4 * (size_t)ppl;
+  const int keep = bytes <= kVloopMaxSmem;
+  if (keep && bytes > 48 * 1024) {
+    const cudaError_t e = cudaFuncSetAttribute(
+        vloops_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kVloopMaxSmem);
+    if (e != cudaSuccess) return e;
+  }
+  vloops_kernel<<<Nl, threads, keep ? bytes : 0, s>>>(seed, first, ppl, keep, out);
   return cudaGetLastError();
 }
 
