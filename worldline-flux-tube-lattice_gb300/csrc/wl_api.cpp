@@ -398,14 +398,18 @@ struct BatchPlan {
   std::vector<wl::ReduceJob> rjobs;
   std::vector<float> inst;
   size_t part_total = 0, out_total = 0;
+  bool split = false;  // some job's partial sums are stored loop by loop
   int reduce_blocks = 0;
 };
 
-int batch_plan(wl_ctx *ctx, int njobs, const wl_job *jobs, int points, BatchPlan *P) {
+int batch_plan(wl_ctx *ctx, int njobs, const wl_job *jobs, int points, bool may_split,
+               BatchPlan *P) {
   size_t inst_total = 0;
   std::vector<size_t> inst_off(njobs), part_off(njobs), out_off(njobs);
   std::vector<int> lcs(njobs), kprofs(njobs);
   std::vector<FieldDev> fds(njobs);
+  std::vector<wl::SweepArgs> cut(njobs);
+  double items = 0.0;
   for (int i = 0; i < njobs; ++i) {
     const wl_job &J = jobs[i];
     Ensemble e;
@@ -419,10 +423,28 @@ int batch_plan(wl_ctx *ctx, int njobs, const wl_job *jobs, int points, BatchPlan
     lcs[i] = batch_loops_per_tile(points, e.ppl, J.group);
     inst_off[i] = inst_total;
     inst_total += (size_t)wl::kInstArrays * J.ninst;
-    part_off[i] = P->part_total;
-    P->part_total += (size_t)(e.Nl / lcs[i]) * J.nF * 3 * J.ninst;
+    cut[i].ninst = J.ninst;
+    cut[i].nF = J.nF;
+    cut[i].ppl = e.ppl;
+    cut[i].chunk_loops = lcs[i];
+    cut[i].n_chunks = e.Nl / lcs[i];
+    items += wl::sweep_chunk_items(cut[i], kprofs[i], J.field.nint);
     out_off[i] = P->out_total;
     P->out_total += (size_t)J.ninst * J.nF * (e.Nl / J.group + 2);
+  }
+  // units over the whole launch (a heavy profile's own launch follows it)
+  P->split = false;
+  for (int i = 0; i < njobs; ++i) {
+    const wl_job &J = jobs[i];
+    wl::sweep_units(cut[i], kprofs[i], J.field.fermion != 0, J.field.nint,
+                    !may_split ? wl::kNoSplit
+                    : wl::batch_in_kernel(kprofs[i])
+                        ? items
+                        : wl::sweep_chunk_items(cut[i], kprofs[i], J.field.nint));
+    const int rows = cut[i].n_chunks * (cut[i].per_loop ? lcs[i] : 1);
+    P->split |= cut[i].per_loop && lcs[i] > 1;
+    part_off[i] = P->part_total;
+    P->part_total += (size_t)rows * J.nF * 3 * J.ninst;
   }
   P->inst.resize(inst_total);
   P->jobs.resize(njobs);
@@ -452,13 +474,16 @@ int batch_plan(wl_ctx *ctx, int njobs, const wl_job *jobs, int points, BatchPlan
     a.Nl = e.Nl;
     a.ppl = e.ppl;
     a.ninst = n;
+    a.chunk_loops = cut[i].chunk_loops;
+    a.n_chunks = cut[i].n_chunks;
+    a.unit_loops = cut[i].unit_loops;
+    a.n_units = cut[i].n_units;
+    a.per_loop = cut[i].per_loop;
     // device pointers are patched in after the buffers are sized (offsets now)
     a.cx = (const float *)(uintptr_t)(inst_off[i]);
     a.nF = J.nF;
     fill_flux(a, &J.field, J.nF, J.F);
     a.field = fds[i];
-    a.chunk_loops = lcs[i];
-    a.n_chunks = e.Nl / lcs[i];
     a.partial = (double *)(uintptr_t)(part_off[i]);
     a.wait_tries = 1u << 22;
     a.kprof = kprofs[i];
@@ -472,7 +497,8 @@ int batch_plan(wl_ctx *ctx, int njobs, const wl_job *jobs, int points, BatchPlan
       P->perm_total += (size_t)n;
     }
     wl::ReduceJob &rj = P->rjobs[i];
-    rj.shape = {nullptr, a.n_chunks, J.group / lcs[i], 1, J.group, n, J.nF};
+    rj.shape = {nullptr, a.n_chunks, J.group / lcs[i], a.per_loop ? lcs[i] : 1,
+                J.group, n,          J.nF};
     rj.ti = wl::reduce_instances(n, J.nF, e.Nl / J.group);
     rj.first = P->reduce_blocks;
     rj.out_group = (double *)(uintptr_t)(out_off[i]);
@@ -483,8 +509,11 @@ int batch_plan(wl_ctx *ctx, int njobs, const wl_job *jobs, int points, BatchPlan
     }
     const int per_tile = wl::sweep_tile_instances(kprofs[i], J.field.nint);
     const int tiles_x = (n + per_tile - 1) / per_tile;
-    const int cost = lcs[i] * e.ppl * (per_tile / wl::kSweepThreads);
-    for (int c = 0; c < a.n_chunks; ++c)
+    a.n_tiles = (n + per_tile / wl::kSweepWarps - 1) / (per_tile / wl::kSweepWarps);
+    const int cost = (int)fmin(
+        2e9, wl::profile_weight(kprofs[i], a.fermion, a.nint) * a.unit_loops * e.ppl *
+                 (per_tile / wl::kSweepThreads));
+    for (int c = 0; c < a.n_units; ++c)
       for (int t = 0; t < tiles_x; ++t) P->tiles.push_back({i, t, c, cost});
   }
   // longest tiles first: the queue then drains evenly (LPT order); ties keep
@@ -497,8 +526,13 @@ int batch_plan(wl_ctx *ctx, int njobs, const wl_job *jobs, int points, BatchPlan
 int batch_run(wl_ctx *ctx, int njobs, const wl_job *jobs, int flags, int points, int ctas,
               bool copy_out) {
   BatchPlan P;
-  int r = batch_plan(ctx, njobs, jobs, points, &P);
+  int r = batch_plan(ctx, njobs, jobs, points, true, &P);
   if (r) return r;
+  if (P.split && ctx->b_part.reserve(P.part_total) != cudaSuccess) {
+    cudaGetLastError();  // loop by loop needs more memory than whole chunks
+    P = BatchPlan();
+    if ((r = batch_plan(ctx, njobs, jobs, points, false, &P))) return r;
+  }
   if (P.tiles.empty() && P.side.empty()) return fail(ctx, WL_ERR_INVALID, "empty batch");
   const size_t jobs_bytes = sizeof(wl::SweepArgs) * njobs;
   const size_t tiles_bytes = sizeof(wl::BatchTile) * P.tiles.size();
@@ -884,29 +918,38 @@ static int run_eval(wl_ctx *ctx, const Ensemble &e, int kprof, const FieldDev &f
     n_chunks = e.Nl;
     cpg = group;
   }
-  const size_t npart = (size_t)n_chunks * nF * 3 * ninst;
+  wl::SweepArgs a;
+  memset(&a, 0, sizeof(a));
+  if (use_sweep) {
+    a.ppl = e.ppl;
+    a.ninst = ninst;
+    a.nF = nF;
+    a.chunk_loops = e.Nl / n_chunks;
+    a.n_chunks = n_chunks;
+    wl::sweep_units(a, kprof, fermion, nint, wl::sweep_chunk_items(a, kprof, nint));
+    // loop by loop needs chunk_loops times the memory: by chunks if there is none
+    if (a.per_loop && ctx->partial.reserve((size_t)e.Nl * nF * 3 * ninst) != cudaSuccess) {
+      cudaGetLastError();
+      wl::sweep_units(a, kprof, fermion, nint, wl::kNoSplit);
+    }
+  }
+  const int inner = a.per_loop ? a.chunk_loops : 1;
+  const size_t npart = (size_t)n_chunks * inner * nF * 3 * ninst;
   if (ctx->partial.reserve(npart) != cudaSuccess) {
     cudaGetLastError();
     return fail(ctx, WL_ERR_NOMEM, "cannot allocate %zu partial sums", npart);
   }
   const float *di = ctx->inst.p;
   if (use_sweep) {
-    wl::SweepArgs a;
-    memset(&a, 0, sizeof(a));
     a.loops = e.dev;
     a.Nl = e.Nl;
-    a.ppl = e.ppl;
-    a.ninst = ninst;
     a.cx = di;
     a.cy = di + ninst;
     a.rtT = di + 2 * ninst;
     a.tqh = di + 3 * ninst;
     a.tql = di + 4 * ninst;
-    a.nF = nF;
     fill_flux(a, field, nF, host_F);
     a.field = fd;
-    a.chunk_loops = e.Nl / n_chunks;
-    a.n_chunks = n_chunks;
     a.partial = ctx->partial.p;
     a.status = ctx->status.p;
     a.wait_tries = 1u << 22;
@@ -923,26 +966,26 @@ static int run_eval(wl_ctx *ctx, const Ensemble &e, int kprof, const FieldDev &f
     WL_CHECK(ctx, wl::launch_sweep(kprof, fermion, nint, a, ctx->stream));
     ctx->last_kind = "instance-parallel";
   } else {
-    wl::LoopArgs a;
-    memset(&a, 0, sizeof(a));
-    a.loops = e.dev;
-    a.Nl = e.Nl;
-    a.ppl = e.ppl;
-    a.ninst = ninst;
-    a.cx = di;
-    a.cy = di + ninst;
-    a.rtT = di + 2 * ninst;
-    a.tqh = di + 3 * ninst;
-    a.tql = di + 4 * ninst;
-    a.nF = nF;
-    fill_flux(a, field, nF, host_F);
-    a.field = fd;
-    a.partial = ctx->partial.p;
-    a.bbox = bbox;
-    WL_CHECK(ctx, wl::launch_loopwarp(kprof, fermion, nint, a, ctx->stream));
+    wl::LoopArgs b;
+    memset(&b, 0, sizeof(b));
+    b.loops = e.dev;
+    b.Nl = e.Nl;
+    b.ppl = e.ppl;
+    b.ninst = ninst;
+    b.cx = di;
+    b.cy = di + ninst;
+    b.rtT = di + 2 * ninst;
+    b.tqh = di + 3 * ninst;
+    b.tql = di + 4 * ninst;
+    b.nF = nF;
+    fill_flux(b, field, nF, host_F);
+    b.field = fd;
+    b.partial = ctx->partial.p;
+    b.bbox = bbox;
+    WL_CHECK(ctx, wl::launch_loopwarp(kprof, fermion, nint, b, ctx->stream));
     ctx->last_kind = "loop-parallel";
   }
-  const wl::ReduceShape rs = {ctx->partial.p, n_chunks, cpg, 1, group, ninst, nF};
+  const wl::ReduceShape rs = {ctx->partial.p, n_chunks, cpg, inner, group, ninst, nF};
   WL_CHECK(ctx, wl::launch_group_reduce(rs, dg, dm, ds, ctx->stream));
   return WL_OK;
 }

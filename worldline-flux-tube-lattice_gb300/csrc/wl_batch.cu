@@ -1,11 +1,11 @@
 // wl_batch.cu -- persistent multi-job sweep and its batched reduction.
 //
 // Many evaluations of uneven size (different ensembles, profiles, flux
-// values, instance counts, loops per tile) run as one launch: every CTA takes
-// tiles from a global queue (atomicAdd on a counter) until it is empty and
-// runs the same per-tile code as the single-job sweep (sweep_tile), so a
-// job's partial sums -- and its results -- do not depend on the batch.  The
-// host orders tiles by decreasing cost so the queue drains evenly.
+// values, instance counts, loops per tile) run as one launch: every warp takes
+// units from a global queue (atomicAdd on a counter) until it is empty and
+// runs the same code as the single-job sweep (warp_unit), so a job's partial
+// sums -- and its results -- do not depend on the batch.  The host orders tiles
+// by decreasing cost so the queue drains evenly.
 #include "wl_device.cuh"
 #include "wl_internal.h"
 #include "wl_reduce.cuh"
@@ -15,109 +15,87 @@ namespace wl {
 
 namespace {
 
-// One tile of a job: packed pairs (256 instances) for the light profiles at
-// 4 and 50 intervals -- as the single-job sweep, so such a job's results match
-// it bit for bit -- one instance per thread otherwise (sweep_tile_instances).
+// One warp's unit of a job: loop pairs for the light profiles at 4 and 50
+// intervals, two instances per lane for the lattice at 4 -- as the single-job
+// sweep, so such a job's loops match it bit for bit -- one instance per lane
+// otherwise.
+// A called function per kind: each is allocated registers on its own (inlined,
+// the 28 of them spilled 420 bytes and the kernel ran an uneven batch of six
+// jobs in 43.9 ms; called, and with the lattice units first, 20.0 ms; CTA tiles
+// of 256 instances, 33 ms).
+template <int P, bool FERM, int NINT, bool PAIR>
+__device__ __noinline__ bool unit_called(const SweepArgs &A, int tile, int l0, int l1, size_t row,
+                                         WarpStage &W) {
+  if constexpr (P == kLattice && PAIR)
+    return warp_unit_lattice<FERM, false>(A, tile, l0, l1, row, W);
+  else
+    return warp_unit<P, FERM, NINT, PAIR>(A, tile, l0, l1, row, W);
+}
 template <bool FERM, int NINT>
-__device__ __forceinline__ void run_tile(int kprof, const SweepArgs &A, int tx, int chunk,
-                                         const SweepShared &S, double (*sacc2)[kPairTile],
-                                         float (*tot)[kSweepThreads], int &consumed) {
-  if constexpr (NINT == 0) {
-    switch (kprof) {
-      case kSmooth: sweep_tile<kSmooth, FERM, NINT>(A, tx, chunk, S, consumed); break;
-      case kGaussian: sweep_tile<kGaussian, FERM, NINT>(A, tx, chunk, S, consumed); break;
-      case kStep: sweep_tile<kStep, FERM, NINT>(A, tx, chunk, S, consumed); break;
-      case kQuadratic: sweep_tile<kQuadratic, FERM, NINT>(A, tx, chunk, S, consumed); break;
-      case kLattice: sweep_tile<kLattice, FERM, NINT>(A, tx, chunk, S, consumed); break;
-      default: break;
-    }
-  } else {
-    switch (kprof) {
-      case kSmooth:
-        sweep_tile2<kSmooth, FERM, NINT>(A, tx, chunk, S.full_bar, sacc2, S.bad, S.ring,
-                                         consumed);
-        break;
-      case kGaussian:
-        sweep_tile2<kGaussian, FERM, NINT>(A, tx, chunk, S.full_bar, sacc2, S.bad, S.ring,
-                                           consumed);
-        break;
-      case kStep:
-        sweep_tile2<kStep, FERM, NINT>(A, tx, chunk, S.full_bar, sacc2, S.bad, S.ring,
-                                       consumed);
-        break;
-      case kQuadratic:
-        sweep_tile2<kQuadratic, FERM, NINT>(A, tx, chunk, S.full_bar, sacc2, S.bad, S.ring,
-                                            consumed);
-        break;
-      case kLattice:
-        if constexpr (NINT == 4)
-          sweep_tile_lat<FERM, false>(A, tx, chunk, S.full_bar, sacc2, tot, S.bad, S.ring,
-                                      consumed);
-        break;
-      default: break;
-    }
+__device__ __forceinline__ bool run_unit(const SweepArgs &A, int tile, int l0, int l1, size_t row,
+                                         WarpStage &W) {
+  constexpr bool kPair = true;  // loop pairs
+  switch (A.kprof) {
+    case kSmooth: return unit_called<kSmooth, FERM, NINT, kPair>(A, tile, l0, l1, row, W);
+    case kGaussian: return unit_called<kGaussian, FERM, NINT, kPair>(A, tile, l0, l1, row, W);
+    case kStep: return unit_called<kStep, FERM, NINT, kPair>(A, tile, l0, l1, row, W);
+    case kQuadratic: return unit_called<kQuadratic, FERM, NINT, kPair>(A, tile, l0, l1, row, W);
+    case kLattice:
+      if constexpr (NINT == 4) return unit_called<kLattice, FERM, 4, true>(A, tile, l0, l1, row, W);
+      if constexpr (NINT == 0)
+        return unit_called<kLattice, FERM, NINT, false>(A, tile, l0, l1, row, W);
+      return true;
+    default: return true;
   }
 }
 
 constexpr int kBatchMinBlocks = 4;
 
+// Every warp takes units from the queue (a tile holds one unit for each of its
+// CTA's four warps' instances) and works alone, its job's parameters in shared
+// memory.
 __global__ void __launch_bounds__(kSweepThreads, kBatchMinBlocks)
     batch_kernel(const __grid_constant__ BatchArgs B) {
-  extern __shared__ __align__(128) float4 ring[];
-  __shared__ __align__(8) uint64_t full_bar[kSweepStages];
-  __shared__ int sm_bad;
-  // FP64 W - 1 sums: [kMaxF * 3][kPairTile] for pair tiles, the first
-  // [kMaxF * 3][kSweepThreads] of it for one-instance tiles
-  __shared__ double sacc2[kMaxF * 3][kPairTile];
-  __shared__ float lat_tot[kLatTotRows][kSweepThreads];  // lattice tiles' loop totals
-  __shared__ __align__(16) SweepArgs job;
-  __shared__ int cur[4];
-  const SweepShared S = {full_bar, reinterpret_cast<double(*)[kSweepThreads]>(&sacc2[0][0]),
-                         &sm_bad, ring};
-  sweep_shared_init(S);
-  int consumed = 0;
+  extern __shared__ __align__(128) unsigned char smem[];
+  __shared__ __align__(8) uint64_t bars[kSweepWarps];
+  __shared__ __align__(16) SweepArgs jobs[kSweepWarps];
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  SweepArgs &job = jobs[w];
+  WarpStage W = warp_stage(smem, bars, kLatStageBytes);
+  warp_stage_init(W.bar);
+  int have = -1;  // the job whose parameters this warp holds
   for (;;) {
-    if (threadIdx.x == 0) {
-      const int t = atomicAdd(B.counter, 1);
-      cur[0] = t;
-      if (t < B.ntiles) {
-        const BatchTile d = B.tiles[t];
-        cur[1] = d.job;
-        cur[2] = d.tile_x;
-        cur[3] = d.chunk;
-      }
-    }
-    __syncthreads();
-    const int t = cur[0];
-    if (t >= B.ntiles) break;
-    {  // the tile's job parameters, copied word by word
-      const int *src = reinterpret_cast<const int *>(B.jobs + cur[1]);
+    int t = 0;
+    if (lane == 0) t = atomicAdd(B.counter, 1);
+    t = __shfl_sync(0xffffffffu, t, 0);
+    if (t / kSweepWarps >= B.ntiles) break;
+    const BatchTile d = B.tiles[t / kSweepWarps];
+    if (d.job != have) {  // copied word by word
+      const int *src = reinterpret_cast<const int *>(B.jobs + d.job);
       int *dst = reinterpret_cast<int *>(&job);
-      for (int w = threadIdx.x; w < (int)(sizeof(SweepArgs) / 4); w += kSweepThreads)
-        dst[w] = src[w];
+      for (int i = lane; i < (int)(sizeof(SweepArgs) / 4); i += 32) dst[i] = src[i];
+      __syncwarp();
+      have = d.job;
     }
-    __syncthreads();
-    const int tx = cur[2], chunk = cur[3];
+    const int tile = d.tile_x * kSweepWarps + t % kSweepWarps;
+    if (tile >= job.n_tiles) continue;
+    int l0, l1;
+    const size_t row = unit_loops(job, d.chunk, l0, l1);
     // 4 and 50 intervals (the reference's): unrolled, pairs for the light
     // profiles; any other count at run time
     const bool n50 = job.nint == 50 && light_profile(job.kprof);
+    bool ok;
     if (job.fermion) {
-      if (job.nint == 4)
-        run_tile<true, 4>(job.kprof, job, tx, chunk, S, sacc2, lat_tot, consumed);
-      else if (n50)
-        run_tile<true, 50>(job.kprof, job, tx, chunk, S, sacc2, lat_tot, consumed);
-      else
-        run_tile<true, 0>(job.kprof, job, tx, chunk, S, sacc2, lat_tot, consumed);
+      if (job.nint == 4) ok = run_unit<true, 4>(job, tile, l0, l1, row, W);
+      else if (n50) ok = run_unit<true, 50>(job, tile, l0, l1, row, W);
+      else ok = run_unit<true, 0>(job, tile, l0, l1, row, W);
     } else {
-      if (job.nint == 4)
-        run_tile<false, 4>(job.kprof, job, tx, chunk, S, sacc2, lat_tot, consumed);
-      else if (n50)
-        run_tile<false, 50>(job.kprof, job, tx, chunk, S, sacc2, lat_tot, consumed);
-      else
-        run_tile<false, 0>(job.kprof, job, tx, chunk, S, sacc2, lat_tot, consumed);
+      if (job.nint == 4) ok = run_unit<false, 4>(job, tile, l0, l1, row, W);
+      else if (n50) ok = run_unit<false, 50>(job, tile, l0, l1, row, W);
+      else ok = run_unit<false, 0>(job, tile, l0, l1, row, W);
     }
-    if (sm_bad) break;  // a copy timed out: the status is set, stop taking tiles
-    __syncthreads();    // cur[] and job are rewritten next
+    if (!ok) break;  // a copy timed out: the status is set, stop taking units
+    __syncwarp();    // the job's parameters may be rewritten next
   }
 }
 
@@ -229,19 +207,18 @@ bool batch_in_kernel(int kprof) { return light_profile(kprof) || kprof == kLatti
 
 bool plain_supports(int kprof) { return light_profile(kprof) || kprof == kLattice; }
 
-// the kernel's static shared memory (the FP64 sums and the lattice totals,
-// 37 KiB) and its ring (16 KiB) exceed the 48 KiB a launch gets without
-// opting in; the attribute is per device, so it is set before every use
+// the lattice units' staging may pass the 48 KiB a launch gets without opting
+// in; the attribute is per device, so it is set before every use
 static cudaError_t batch_smem_optin() {
   return cudaFuncSetAttribute(batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)sweep_smem_bytes());
+                              (int)sweep_lat_smem_bytes());
 }
 
 int batch_max_ctas_per_sm() {
   int n = 0;
   if (batch_smem_optin() != cudaSuccess ||
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, batch_kernel, kSweepThreads,
-                                                    sweep_smem_bytes()) != cudaSuccess) {
+                                                    sweep_lat_smem_bytes()) != cudaSuccess) {
     cudaGetLastError();
     return 1;
   }
@@ -251,7 +228,7 @@ int batch_max_ctas_per_sm() {
 cudaError_t launch_batch(const BatchArgs &a, int grid, cudaStream_t s) {
   const cudaError_t e = batch_smem_optin();
   if (e != cudaSuccess) return e;
-  batch_kernel<<<grid, kSweepThreads, sweep_smem_bytes(), s>>>(a);
+  batch_kernel<<<grid, kSweepThreads, sweep_lat_smem_bytes(), s>>>(a);
   return cudaGetLastError();
 }
 

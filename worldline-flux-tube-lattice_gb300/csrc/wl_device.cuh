@@ -136,6 +136,14 @@ struct Profile<kSmooth> {  // f = r2/(l2+r2): f/r2 = 1/(l2+r2), f' = l2 (f/r2)^2
   static constexpr bool kHeavy = false;
 };
 
+// The smooth profile takes |z|^2 only as l2 + max(|z|^2, clampA).  Where
+// l2 + clampA rounds to l2 (the reference's 1e-8 at lambda^2 > 0.25) or there
+// is no clamp, the maximum changes no bit of that sum and is left out: one of
+// the ten instructions a segment spends beside its FP32 arithmetic and
+// reciprocals (2 % of the 4-interval sweep).
+template <>
+struct Profile<kSmoothWide> : Profile<kSmooth> {};
+
 template <>
 struct Profile<kStep> {  // intEV.cu:267-272, 368-373
   static __device__ __forceinline__ void eval(float r2, const FieldDev &F, float &g,
@@ -442,7 +450,7 @@ __device__ __noinline__ float2 segment_fixflux(float zix, float ziy, float zjx, 
 // profile evaluates on l2 + rho^2, else 0)
 template <int P>
 __device__ __forceinline__ float profile_shift(const FieldDev &F) {
-  if constexpr (P == kSmooth)
+  if constexpr (smooth_profile(P))
     return Profile<P>::shift(F);
   else
     return 0.0f;
@@ -473,7 +481,7 @@ __device__ __forceinline__ float profile_shift(const FieldDev &F) {
 #endif
 template <int P, bool FERM, int NINT, bool PAIR = false>
 constexpr int soft_rcp_period() {
-  if constexpr (P == kSmooth && NINT >= 8) {
+  if constexpr (smooth_profile(P) && NINT >= 8) {
     if constexpr (PAIR)
       return FERM ? WL_SOFT_RCP_PAIR_SPINOR : WL_SOFT_RCP_PAIR_SCALAR;
     else
@@ -575,7 +583,7 @@ __device__ __forceinline__ float2 rcp_newton2(float2 d) {
 // the light profiles on a pair: g = f/rho^2 and fp = f'/fp_scale as in eval
 template <int P>
 __device__ __forceinline__ void eval2(float2 r2, const FieldDev &F, float2 &g, float2 &fp) {
-  if constexpr (P == kSmooth) {
+  if constexpr (smooth_profile(P)) {
     g = rcp2(r2);
     fp = mul2(g, g);
   } else if constexpr (P == kGaussian) {  // as Profile<kGaussian>::eval, per half
@@ -610,7 +618,7 @@ __device__ __forceinline__ void segment2(float2 zix, float2 ziy, float2 zjx, flo
   float2 b = fma2(zix, dx, mul2(ziy, dy));
   float2 c = fma2(dx, dx, mul2(dy, dy));
   const float2 xyyx = fma2(zix, zjy, neg2(mul2(ziy, zjx)));
-  a = max2(a, F.clampA);
+  if (P != kSmoothWide) a = max2(a, F.clampA);
   b = max2(b, F.clampB);
   c = max2(c, F.clampC);
   const float2 as = add2(a, f2(profile_shift<P>(F)));
@@ -625,7 +633,7 @@ __device__ __forceinline__ void segment2(float2 zix, float2 ziy, float2 zjx, flo
   // as explicit fma (the square of each later node fused into the running
   // sum), so no sum of two products is left for the compiler to contract
   // one way or the other.
-  constexpr bool kSq = (P == kSmooth);
+  constexpr bool kSq = smooth_profile(P);
   float2 so, se, fo, fe;
 #pragma unroll
   for (int j = 1; j < NINT; j++) {
@@ -656,6 +664,63 @@ __device__ __forceinline__ void segment2(float2 zix, float2 ziy, float2 zjx, flo
   }
 }
 
+// segment() with a run-time interval count on a pair.  Each half as segment()
+// rounds it; the smooth profile's f' = g^2 enters the sums as a fused
+// multiply-add, except in a loop's opening and closing segments (EDGE), where
+// the square is rounded first: the two roundings the scalar kernel was compiled
+// to, made explicit so that results keep their bits.
+template <int P, bool FERM, bool EDGE>
+__device__ __forceinline__ void segment2_rt(float2 zix, float2 ziy, float2 zjx, float2 zjy,
+                                            const FieldDev &F, float2 &ph, float2 &sp) {
+  static_assert(!Profile<P>::kHeavy, "pairs: light profiles");
+  const float2 dx = add2(zjx, neg2(zix)), dy = add2(zjy, neg2(ziy));
+  float2 a = fma2(zix, zix, mul2(ziy, ziy));
+  float2 b = fma2(zix, dx, mul2(ziy, dy));
+  float2 c = fma2(dx, dx, mul2(dy, dy));
+  const float2 xyyx = fma2(zix, zjy, neg2(mul2(ziy, zjx)));
+  a = max2(a, F.clampA);
+  b = max2(b, F.clampB);
+  c = max2(c, F.clampC);
+  const float2 b2 = add2(b, b);
+  const float2 as = add2(a, f2(profile_shift<P>(F)));
+  const float2 ae = add2(add2(as, b2), c);
+  constexpr bool kSq = smooth_profile(P);
+  const float h = F.h;
+  auto node = [&](float j, float2 &g, float2 &fp) {
+    const float2 t = f2(j * h);  // the reference's (float)j * h (intEV.cu:436)
+    eval2<P>(fma2(fma2(c, t, b2), t, as), F, g, fp);
+  };
+  auto acc = [&](float2 &sg, float2 &sf, float2 g, float2 fp) {
+    sg = add2(sg, g);
+    if (!FERM) return;
+    if (kSq && EDGE)
+      sf = make_float2(__fadd_rn(sf.x, __fmul_rn(g.x, g.x)),
+                       __fadd_rn(sf.y, __fmul_rn(g.y, g.y)));
+    else
+      sf = kSq ? fma2(g, g, sf) : add2(sf, fp);
+  };
+  float2 g0, f0, g1, f1;
+  eval2<P>(as, F, g0, f0);
+  eval2<P>(ae, F, g1, f1);
+  float2 so, fo, se = f2(0.f), fe = f2(0.f);
+  node(1.0f, so, fo);
+  float j = 2.0f;
+#pragma unroll 2
+  for (int k = F.nint / 2 - 1; k > 0; --k, j += 2.0f) {
+    float2 ge, pe, go, po;
+    node(j, ge, pe);
+    node(j + 1.0f, go, po);
+    acc(se, fe, ge, pe);
+    acc(so, fo, go, po);
+  }
+  const float2 S = fma2(f2(4.0f), so, fma2(f2(2.0f), se, add2(g0, g1)));
+  ph = fma2(xyyx, S, ph);
+  if (FERM) {
+    const float2 f01 = kSq ? fma2(g0, g0, f1) : add2(f0, f1);
+    sp = add2(sp, fma2(f2(4.0f), fo, fma2(f2(2.0f), fe, f01)));
+  }
+}
+
 // segment2 as a called function for many intervals: one copy of the long
 // node sequence instead of one per call site of the sweep (a dozen), which
 // keeps the kernel within the instruction cache; the sums travel by value
@@ -669,10 +734,12 @@ __device__ __noinline__ float4 segment2_called(float2 zix, float2 ziy, float2 zj
   segment2<P, FERM, NINT>(zix, ziy, zjx, zjy, F, ph, sp);
   return make_float4(ph.x, ph.y, sp.x, sp.y);
 }
-template <int P, bool FERM, int NINT>
+template <int P, bool FERM, int NINT, bool EDGE>
 __device__ __forceinline__ void seg2(float2 zix, float2 ziy, float2 zjx, float2 zjy,
                                      const FieldDev &F, float2 &ph, float2 &sp) {
-  if constexpr (NINT >= WL_SEG2_CALL_MIN) {
+  if constexpr (NINT == 0) {
+    segment2_rt<P, FERM, EDGE>(zix, ziy, zjx, zjy, F, ph, sp);
+  } else if constexpr (NINT >= WL_SEG2_CALL_MIN) {
     const float4 r = segment2_called<P, FERM, NINT>(zix, ziy, zjx, zjy, F,
                                                     make_float4(ph.x, ph.y, sp.x, sp.y));
     ph = make_float2(r.x, r.y);

@@ -12,18 +12,14 @@ namespace wl {
 // device-side status codes written to the status word of a launch
 enum : int { kDevOk = 0, kDevTimeout = 1, kDevBadInstance = 2 };
 
-// Instance-parallel sweep: one thread per (instance), one CTA per
-// (instance tile, chunk of loops); the chunk's loops are streamed through a
-// shared-memory ring by bulk copies and every thread walks every point.
-constexpr int kSweepThreads = 128;   // instances per CTA
-// resident CTAs per SM the light-profile sweep is compiled for (register cap
-// 65536 / (128 * blocks)); the lattice profiles use 4
-#ifndef WL_SWEEP_MIN_BLOCKS
-#define WL_SWEEP_MIN_BLOCKS 6
-#endif
-constexpr int kSweepMinBlocks = WL_SWEEP_MIN_BLOCKS;
-constexpr int kSweepStages = 4;      // shared-memory ring depth
-constexpr int kSweepChunkPts = 256;  // points per bulk copy (4 KiB)
+// Instance-parallel sweep: one lane per instance, one warp per (32 instances,
+// unit of loops); every warp streams its loops through shared memory by bulk
+// copies and works alone (wl_sweep.cuh).
+constexpr int kSweepThreads = 128;
+constexpr int kSweepWarps = kSweepThreads / 32;
+constexpr int kLandPts = 256;  // points of a warp's landing zone (4 KiB)
+// warps resident on the chip: 152 SMs x 4 CTAs (128 registers a thread)
+constexpr int kSweepSlots = 152 * 4 * kSweepWarps;
 
 struct SweepArgs {
   const float4 *loops;  // [Nl][ppl]
@@ -37,9 +33,13 @@ struct SweepArgs {
   // double-float per-flux constants: cph = F h/3, csp = F h/3 fp_scale
   float cph_hi[kMaxF], cph_lo[kMaxF], csp_hi[kMaxF], csp_lo[kMaxF];
   FieldDev field;
-  int chunk_loops;   // loops per CTA
+  int chunk_loops;   // loops per partial sum
   int n_chunks;      // Nl / chunk_loops
-  double *partial;   // [n_chunks][nF][3][ninst]
+  int unit_loops;    // loops per warp unit
+  int n_units;
+  int per_loop;      // the partial sums are stored loop by loop
+  int n_tiles;       // warps per unit (set at launch)
+  double *partial;   // [n_chunks][nF][3][ninst], per_loop: [Nl][nF][3][ninst]
   int *status;       // kDevOk / kDevTimeout
   uint32_t wait_tries;
   int kprof, fermion, nint;  // kernel selection inside the persistent batch kernel
@@ -49,19 +49,75 @@ struct SweepArgs {
   const int *perm;
 };
 
-// The single-job sweep runs the light profiles at 4 and 50 intervals two
-// instances per thread as packed f32x2 pairs (256 per CTA of 128 threads),
-// and the lattice at 4 intervals two instances per thread (their images in
-// packed pairs), everything else one per thread; so do the tiles of the
-// persistent batch kernel: instances per batch tile.
 inline __host__ __device__ bool light_profile(int kprof) {
   return kprof == kSmooth || kprof == kStep || kprof == kQuadratic || kprof == kGaussian;
 }
-inline __host__ __device__ int sweep_tile_instances(int kprof, int nint) {
-  return (((nint == 4 || nint == 50) && light_profile(kprof)) || (nint == 4 && kprof == kLattice))
-             ? 2 * kSweepThreads
-             : kSweepThreads;
+// two loops per lane as packed f32x2 pairs (wl_sweep.cuh)
+inline __host__ __device__ bool sweep_loop_pairs(int kprof, int nint) {
+  (void)nint;
+  return light_profile(kprof);
 }
+// instances per warp (the lattice at 4 intervals: two per lane)
+inline __host__ __device__ int warp_instances(int kprof, int nint) {
+  return nint == 4 && kprof == kLattice ? 64 : 32;
+}
+// instances per batch tile (one CTA's warps)
+inline __host__ __device__ int sweep_tile_instances(int kprof, int nint) {
+  return kSweepWarps * warp_instances(kprof, nint);
+}
+
+// Device time of one tile-point relative to the smooth profile at 4
+// intervals (tile order, processor-sharing split and rate estimates only): the
+// node count times the profile's cost relative to the smooth one at the same
+// interval count, measured on the GB300 through wl_eval (512 instances on
+// Nl 1024 x ppl 1024, scalar QED) at 4, 8 and 50 intervals and interpolated
+// linearly in nint between them (flat outside).
+inline double profile_weight(int kprof, int fermion, int nint) {
+  double r[3] = {1.0, 1.0, 1.0};  // at 4, 8, 50 intervals
+  switch (kprof) {
+    case kGaussian: r[0] = 1.6; r[1] = 1.94; r[2] = 3.95; break;
+    case kLattice: r[0] = r[1] = r[2] = 8.0; break;
+    case kPeriodic: r[0] = r[1] = 30.4; r[2] = 70.8; break;
+    case kSpline: r[0] = r[1] = 12.6; r[2] = 29.2; break;
+    case kFixflux:
+    case kFixfluxFF: r[0] = r[1] = 180.0; r[2] = 400.0; break;
+    default: break;
+  }
+  double w;
+  if (nint <= 4) w = r[0];
+  else if (nint <= 8) w = r[0] + (r[1] - r[0]) * (nint - 4) / 4.0;
+  else if (nint <= 50) w = r[1] + (r[2] - r[1]) * (nint - 8) / 42.0;
+  else w = r[2];
+  return (fermion ? w * 1.15 : w) * (nint + 1) / 5.0;
+}
+
+// warp units of a sweep by whole chunks
+inline double sweep_chunk_items(const SweepArgs &a, int kprof, int nint) {
+  const int per = warp_instances(kprof, nint);
+  return (double)((a.ninst + per - 1) / per) * a.n_chunks;
+}
+// How the loops of a sweep are cut into warp units.  By whole chunks of
+// chunk_loops (one partial sum per chunk), or, where that gives the launch too
+// few units to fill the chip evenly, into the smallest units (a loop, or the
+// two of a packed pair) whose loops are stored one by one; the reduction adds
+// them in the same order, so a result does not depend on the choice.
+//   items: the launch's units by whole chunks.  Chunks leave about half a wave
+// of warps idle at the end, 0.5 / waves of the time; loop by loop costs 48 nF
+// bytes of HBM traffic per (loop, instance), 6 nF / ppl of the time of its ppl
+// segments at the measured rates (8.5e11 segments/s of weight 1, 6.8 TB/s).
+// Above 16 waves the partial sums would also outgrow the gain (0.24 GB per flux
+// value).  Measured: 96 instances x 3 fluxes on 5120 x 2048 points (1 wave)
+// 1.20 ms against 3.14 ms in 128-thread tiles of 256 instances.
+inline void sweep_units(SweepArgs &a, int kprof, int fermion, int nint, double items) {
+  const int loops = a.n_chunks * a.chunk_loops, unit = sweep_loop_pairs(kprof, nint) ? 2 : 1;
+  const bool split = items <= 16.0 * kSweepSlots &&
+                     items * 12.0 * a.nF <
+                         (double)kSweepSlots * a.ppl * profile_weight(kprof, fermion, nint);
+  a.per_loop = a.chunk_loops == 1 || split;
+  a.unit_loops = a.per_loop ? unit : a.chunk_loops;
+  a.n_units = (loops + a.unit_loops - 1) / a.unit_loops;
+}
+constexpr double kNoSplit = 1e300;  // items of a launch that keeps whole chunks
 
 // Persistent multi-job sweep: a queue of tiles (job, instance tile, loop
 // chunk) drained by one CTA per slot; jobs differ in ensemble, profile,
@@ -204,11 +260,13 @@ cudaError_t launch_loop_bbox(const float4 *loops, int Nl, int ppl, float4 *out, 
 cudaError_t launch_vloops(uint64_t seed, int first, int Nl, int ppl, float4 *out,
                           cudaStream_t s);
 
-// bytes of dynamic shared memory of the sweep kernel
 constexpr int kInstArrays = 5;  // cx, cy, rtT, tq_hi, tq_lo
 
-constexpr size_t sweep_smem_bytes() {
-  return (size_t)kSweepStages * kSweepChunkPts * sizeof(float4);
+// per CTA: each warp's landing zone and compact piece
+constexpr size_t sweep_smem_bytes() { return (size_t)kSweepWarps * kLandPts * (16 + 8); }
+// lattice at 4 intervals: landing zone, compact points, block boxes, loop totals
+constexpr size_t sweep_lat_smem_bytes() {
+  return (size_t)kSweepWarps * (kLandPts * 16 + (kLandPts + 8) * 16 + 8 * 16 + 24 * 32 * 4);
 }
 
 }  // namespace wl

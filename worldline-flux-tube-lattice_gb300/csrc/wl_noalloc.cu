@@ -123,7 +123,8 @@ extern "C" int wl_eval_noalloc(const float *dev_loops, int Nl, int ppl, const wl
   const size_t inst_off = 256;
   const size_t inst_bytes = (size_t)wl::kInstArrays * ninst * sizeof(float);
   const size_t part_off = (inst_off + inst_bytes + 255) & ~(size_t)255;
-  const size_t need = part_off + (size_t)n_chunks * nF * 3 * ninst * sizeof(double);
+  const size_t part_bytes = (size_t)n_chunks * nF * 3 * ninst * sizeof(double);
+  const size_t need = part_off + part_bytes;
   if (need > kScratchBytes)
     return nfail(WL_ERR_INVALID,
                  "the request needs %s%lld bytes of scratch, more than the fixed %lld "
@@ -155,6 +156,7 @@ extern "C" int wl_eval_noalloc(const float *dev_loops, int Nl, int ppl, const wl
   cudaError_t ce = cudaMemsetAsync(status, 0, sizeof(int), s);
   if (ce == cudaSuccess)
     ce = wl::launch_instance_setup(dev_cx, dev_cy, dev_T, ninst, ppl, inst, status, s);
+  int inner = 1;
   if (ce == cudaSuccess && use_sweep) {
     wl::SweepArgs a;
     memset(&a, 0, sizeof(a));
@@ -172,6 +174,12 @@ extern "C" int wl_eval_noalloc(const float *dev_loops, int Nl, int ppl, const wl
     a.field = fd;
     a.chunk_loops = lc;
     a.n_chunks = n_chunks;
+    // loop by loop (as wl_eval_device) only where that fits the scratch too
+    wl::sweep_units(a, kprof, field->fermion != 0, field->nint,
+                    part_off + part_bytes * lc <= kScratchBytes
+                        ? wl::sweep_chunk_items(a, kprof, field->nint)
+                        : wl::kNoSplit);
+    if (a.per_loop) inner = lc;
     a.partial = partial;
     a.status = status;
     a.wait_tries = 1u << 22;
@@ -195,7 +203,7 @@ extern "C" int wl_eval_noalloc(const float *dev_loops, int Nl, int ppl, const wl
     ce = wl::launch_loopwarp(kprof, field->fermion != 0, field->nint, a, s);
   }
   if (ce == cudaSuccess)
-    ce = wl::launch_group_reduce({partial, n_chunks, cpg, 1, group, ninst, nF}, dev_out_group,
+    ce = wl::launch_group_reduce({partial, n_chunks, cpg, inner, group, ninst, nF}, dev_out_group,
                                  dev_out_mean, dev_out_sem, s);
   int st = 0;
   if (ce == cudaSuccess) ce = cudaMemcpyAsync(&st, status, sizeof(int), cudaMemcpyDeviceToHost, s);

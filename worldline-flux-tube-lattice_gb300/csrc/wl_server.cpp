@@ -53,31 +53,6 @@ constexpr size_t kAlign = 256;
 
 size_t up(size_t x) { return (x + kAlign - 1) & ~(kAlign - 1); }
 
-// Device time of one tile-point relative to the smooth profile at 4
-// intervals (the processor-sharing split and the rate estimate only): the
-// node count times the profile's cost relative to the smooth one at the same
-// interval count, measured on the GB300 through wl_eval (512 instances on
-// Nl 1024 x ppl 1024, scalar QED) at 4, 8 and 50 intervals and interpolated
-// linearly in nint between them (flat outside).
-double profile_weight(int kprof, int fermion, int nint) {
-  double r[3] = {1.0, 1.0, 1.0};  // at 4, 8, 50 intervals
-  switch (kprof) {
-    case wl::kGaussian: r[0] = 1.6; r[1] = 1.94; r[2] = 3.95; break;
-    case wl::kLattice: r[0] = r[1] = r[2] = 8.0; break;
-    case wl::kPeriodic: r[0] = r[1] = 30.4; r[2] = 70.8; break;
-    case wl::kSpline: r[0] = r[1] = 12.6; r[2] = 29.2; break;
-    case wl::kFixflux:
-    case wl::kFixfluxFF: r[0] = r[1] = 180.0; r[2] = 400.0; break;
-    default: break;
-  }
-  double w;
-  if (nint <= 4) w = r[0];
-  else if (nint <= 8) w = r[0] + (r[1] - r[0]) * (nint - 4) / 4.0;
-  else if (nint <= 50) w = r[1] + (r[2] - r[1]) * (nint - 8) / 42.0;
-  else w = r[2];
-  return (fermion ? w * 1.15 : w) * (nint + 1) / 5.0;
-}
-
 struct SrvEnsemble {
   uint64_t seed = 0;
   int Nl = 0, ppl = 0;
@@ -98,6 +73,7 @@ struct Req {
   bool done = false;
   // sizes
   int ninst = 0, lc = 0, n_chunks = 0, ng = 0, tiles_x = 0;
+  int unit_loops = 0, n_units = 0, per_loop = 0;
   long long ntiles = 0, next_tile = 0;
   size_t dbytes = 0, pbytes = 0;  // device / pinned footprint
   size_t o_rj = 0, o_inst = 0, o_perm = 0, o_part = 0, o_out = 0, o_aux = 0;  // device offsets
@@ -246,9 +222,20 @@ int check_request(wl_server *s, const wl_request *q, Req *R) {
   R->n_chunks = q->Nl / R->lc;
   const int per_tile = wl::sweep_tile_instances(R->kprof, q->field.nint);
   R->tiles_x = (n + per_tile - 1) / per_tile;
-  R->ntiles = (long long)R->n_chunks * R->tiles_x;
-  R->tile_work = (double)R->lc * q->ppl * per_tile *
-                 profile_weight(R->kprof, q->field.fermion != 0, q->field.nint);
+  {
+    wl::SweepArgs a;
+    memset(&a, 0, sizeof(a));
+    a.ninst = n;
+    a.chunk_loops = R->lc;
+    a.n_chunks = R->n_chunks;
+    wl::sweep_units(a, R->kprof, q->field.fermion != 0, q->field.nint, wl::kNoSplit);
+    R->unit_loops = a.unit_loops;
+    R->n_units = a.n_units;
+    R->per_loop = a.per_loop;
+  }
+  R->ntiles = (long long)R->n_units * R->tiles_x;
+  R->tile_work = (double)R->unit_loops * q->ppl * per_tile *
+                 wl::profile_weight(R->kprof, q->field.fermion != 0, q->field.nint);
   R->segments = (double)n * q->Nl * q->ppl;
   const size_t n_part = (size_t)R->n_chunks * nF * 3 * n;
   const size_t n_out = (size_t)n * nF * (ng + 2);
@@ -479,6 +466,11 @@ bool admit(wl_server *s) {
     a.field = R->fd;
     a.chunk_loops = R->lc;
     a.n_chunks = R->n_chunks;
+    a.unit_loops = R->unit_loops;
+    a.n_units = R->n_units;
+    a.per_loop = R->per_loop;
+    const int per_warp = wl::warp_instances(R->kprof, R->q.field.nint);
+    a.n_tiles = (n + per_warp - 1) / per_warp;
     a.partial = d_part;
     a.status = d_status;
     a.wait_tries = 1u << 22;
@@ -624,8 +616,7 @@ void launch_quantum(wl_server *s, int k) {
       if (R->next_tile >= R->ntiles) closing.push_back(R);
       continue;
     }
-    const int cost = R->lc * R->q.ppl *
-                     (wl::sweep_tile_instances(R->kprof, R->q.field.nint) / wl::kSweepThreads);
+    const int cost = (int)fmin(2e9, R->tile_work / wl::kSweepThreads);
     for (long long c = 0; c < take[i] && n < kMaxQuantumTiles; ++c) {
       const long long t = R->next_tile++;
       h[n++] = {R->slot, (int)(t % R->tiles_x), (int)(t / R->tiles_x), cost};
@@ -668,7 +659,7 @@ void launch_quantum(wl_server *s, int k) {
     wl::SweepArgs a = R->args;
     a.loops += (size_t)x.c0 * R->lc * R->q.ppl;
     a.partial += (size_t)x.c0 * R->q.nF * 3 * R->ninst;
-    a.n_chunks = x.nc;
+    a.n_chunks = a.n_units = x.nc;  // heavy profiles: a unit is a chunk
     ck(wl::launch_sweep(R->kprof, R->q.field.fermion != 0, R->q.field.nint, a, st),
        "sweep launch");
   }

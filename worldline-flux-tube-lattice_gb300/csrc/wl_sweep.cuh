@@ -4,16 +4,17 @@
 // (ExpectValue -> WilsonLoop, intEV.cu:508-582) and the EVMean factors
 // (Integrand.c:352-390), and write FP64 partial sums of the W factors.
 //
-// sweep_kernel (instance-parallel): thread = instance (centre of mass,
-//   proper time), CTA = 128 instances x a chunk of loops.  The chunk's loops
-//   are streamed through a 4-stage shared-memory ring with bulk copies
-//   (cp.async.bulk + mbarrier); every thread walks every point of the staged
-//   loop, so each shared-memory load is a warp-wide broadcast and the loop
-//   data is read from HBM once per CTA.  Within a loop the points are visited
-//   in order; the three sub-loops (N/2: odd points, N/4a: i = 0 mod 4,
-//   N/4b: i = 2 mod 4; intEV.cu:461-506) advance together, one group of four
-//   points (four segments) at a time, and each segment adds to its sub-loop
-//   in the reference's order.  Phases accumulate in FP32 with Kahan
+// sweep kernels (instance-parallel): lane = instance (centre of mass, proper
+//   time), warp = 32 instances x a unit of loops.  Every warp works alone: it
+//   streams its own loops through shared memory with bulk copies
+//   (cp.async.bulk + mbarrier, the next piece in flight while one is walked),
+//   and every lane walks every staged point, so each shared-memory load is a
+//   warp-wide broadcast and the ensemble comes from HBM about once per launch
+//   (the warps of other instances read it from L2).  Within a loop the points
+//   are visited in order; the three sub-loops (N/2: odd points, N/4a: i = 0
+//   mod 4, N/4b: i = 2 mod 4; intEV.cu:461-506) advance together, one group of
+//   four points (four segments) at a time, and each segment adds to its
+//   sub-loop in the reference's order.  Phases accumulate in FP32 with Kahan
 //   compensation per block of 8 groups; W factors accumulate in FP64.
 //
 // loopwarp_kernel (loop-parallel): warp = (loop, instance), lanes over the
@@ -29,118 +30,216 @@ namespace wl {
 static_assert(kSweepThreads == 32 * kFfWarps && kLoopWarps == kFfWarps,
               "fixflux queues: 4 warps per CTA");
 
-// Shared-memory state of the sweep, reused by consecutive tiles of a CTA.
-struct SweepShared {
-  uint64_t *full_bar;                  // [kSweepStages] mbarriers
-  double (*sacc)[kSweepThreads];       // [kMaxF * 3][kSweepThreads] FP64 W - 1 sums
-  int *bad;                            // a stage copy timed out
-  float4 *ring;                        // [kSweepStages][kSweepChunkPts]
+// ------------------------------------------------------ staging per warp --
+// A warp's staging area: the landing zone of its bulk copies and the compact
+// copy of a piece's coordinates that the lanes walk.  `copies` counts the
+// pieces this warp has waited for (its barrier's phase continues across units).
+struct WarpStage {
+  float4 *land;   // [kLandPts] float4 points as the ensemble holds them
+  float4 *comp;   // the piece's coordinates, laid out for its walk
+  uint64_t *bar;  // the warp's mbarrier
+  uint32_t copies;
 };
 
-__device__ __forceinline__ void sweep_shared_init(const SweepShared &S) {
-  if (threadIdx.x == 0) {
-    for (int st = 0; st < kSweepStages; ++st) mbar_init(&S.full_bar[st], 1);
+__device__ __forceinline__ void warp_stage_init(uint64_t *bar) {
+  if ((threadIdx.x & 31) == 0) {
+    mbar_init(bar, 1);
     fence_mbar_init();
-    *S.bad = 0;
   }
-  __syncthreads();
+  __syncwarp();
 }
 
-// One tile: instances [tile_x * kSweepThreads, +kSweepThreads) of A over the
-// loops of chunk `chunk`.  `consumed` counts the stage copies this CTA has
-// waited for before (the ring's barrier phases continue across tiles).
-// Returns false if a copy timed out (status set, nothing written).
-template <int P, bool FERM, int NINT>
-__device__ __forceinline__ bool sweep_tile(const SweepArgs &A, int tile_x, int chunk,
-                                           const SweepShared &S, int &consumed) {
-  const int tid = threadIdx.x;
-  const int slot = tile_x * kSweepThreads + tid;
+// Waits (bounded) for the piece in flight; on a time-out waits once more, so
+// that the copy does not land after the warp has left, and reports.
+__device__ __forceinline__ bool warp_stage_wait(const SweepArgs &A, WarpStage &W) {
+  const uint32_t par = W.copies & 1u;
+  const bool ok = mbar_wait_bounded(W.bar, par, A.wait_tries);
+  if (!__all_sync(0xffffffffu, ok)) {
+    mbar_wait_bounded(W.bar, par, A.wait_tries);
+    if ((threadIdx.x & 31) == 0) atomicExch(A.status, kDevTimeout);
+    return false;
+  }
+  ++W.copies;
+  return true;
+}
+
+// W - 1 of one loop at one instance into the partial sums: stored on its own
+// (per_loop) or added to its chunk's sum, which the same lane keeps in loop
+// order (acc: not the chunk's first loop).
+__device__ __forceinline__ void put_loop(const SweepArgs &A, size_t row, int j, int ic, bool acc,
+                                         double d0, double d1, double d2) {
+  double *o = A.partial + (row * A.nF + j) * 3 * A.ninst + ic;
+  const size_t n = (size_t)A.ninst;
+  if (acc) {
+    d0 += o[0];
+    d1 += o[n];
+    d2 += o[2 * n];
+  }
+  o[0] = d0;
+  o[n] = d1;
+  o[2 * n] = d2;
+}
+
+// scalar and pair arithmetic of the walk under one name
+__device__ __forceinline__ float vset(float, float a) { return a; }
+__device__ __forceinline__ float2 vset(float2, float a) { return f2(a); }
+__device__ __forceinline__ float vfma(float a, float b, float c) { return fmaf(a, b, c); }
+__device__ __forceinline__ float2 vfma(float2 a, float2 b, float2 c) { return fma2(a, b, c); }
+__device__ __forceinline__ void vkahan(float &s, float &c, float x) { kahan_add(s, c, x); }
+__device__ __forceinline__ void vkahan(float2 &s, float2 &c, float2 x) { kahan_add2(s, c, x); }
+__device__ __forceinline__ float vlane(float v, int) { return v; }
+__device__ __forceinline__ float vlane(float2 v, int h) { return h ? v.y : v.x; }
+template <bool PAIR>
+struct Vec {
+  using T = float;
+};
+template <>
+struct Vec<true> {
+  using T = float2;
+};
+
+// one segment; EDGE: a loop's opening or a closing segment
+template <int P, bool FERM, int NINT, bool EDGE = false>
+__device__ __forceinline__ void vseg(float zix, float ziy, float zjx, float zjy,
+                                     const FieldDev &F, const ImgRange &img, float &ph,
+                                     float &sp) {
+  seg<P, FERM, NINT>(zix, ziy, zjx, zjy, F, img, ph, sp);
+}
+template <int P, bool FERM, int NINT, bool EDGE = false>
+__device__ __forceinline__ void vseg(float2 zix, float2 ziy, float2 zjx, float2 zjy,
+                                     const FieldDev &F, const ImgRange &, float2 &ph,
+                                     float2 &sp) {
+  seg2<P, FERM, NINT, EDGE>(zix, ziy, zjx, zjy, F, ph, sp);
+}
+
+// Kahan blocks: 8 groups, counted from the loop's first walked group (1) up to
+// group 64 and from multiples of 64 groups (256 points) after it
+__device__ __forceinline__ int block_end(int q) {
+  return q < 64 ? min(((q - 1) & ~7) + 9, 64) : (q & ~7) + 8;
+}
+
+// One unit of a warp: instances [32 tile, +32), one per lane, over loops
+// [l0, l1).  PAIR: the lane walks loops l and l + 1 together as a packed pair:
+// every FP32 operation of a segment is one f32x2 operation on the two loops
+// (each half rounds as the scalar walk does), and the staged piece interleaves
+// the two loops' coordinates (x, x', y, y'), so that one 16-byte broadcast load
+// gives both operands already packed.
+//   Bound by the SM's dispatch: a packed operation takes two of its cycles, so
+// a pair-segment of the smooth spinor profile spends 68 on FP32 arithmetic, 10
+// on reciprocals (80 on the MUFU) and ~13 on clamps, loads and loop control.
+// Tiles of 256 instances on one loop (two per thread, a CTA barrier per piece)
+// left lanes dead below 256 instances and slots empty below ~600 CTAs.
+// Measured, 256-instance tiles -> warp units: 96 instances x 3 fluxes on 5120 x
+// 2048 points 3.14 -> 1.15 ms; 8192 instances there 101.3 -> 98.6 ms (8.8e11
+// segments/s); smooth scalar at 50 intervals, 3160 instances on 5120 x 1024,
+// 152.3 -> 143.5 ms.  Run-time interval counts, one instance per thread -> loop
+// pairs: Gaussian spinor at 16 intervals, 333 instances on 1500 x 516, 4.83 ->
+// 2.65 ms.  One lane per instance, one CTA per chunk -> one warp per loop, 50
+// intervals: periodic, 128 instances on 1024 x 512, 103 -> 32.7 ms; fixflux, 64
+// instances on 512 x 512, 375 -> 92 ms.
+//   row: the partial-sum row of loop l0 (per_loop) or of the unit's chunk.
+// Returns false if a copy timed out.
+template <int P, bool FERM, int NINT, bool PAIR>
+__device__ __forceinline__ bool warp_unit(const SweepArgs &A, int tile, int l0, int l1,
+                                          size_t row, WarpStage &W) {
+  using V = typename Vec<PAIR>::T;
+  constexpr int kStep = PAIR ? 2 : 1;          // loops walked together
+  constexpr int kPiece = kLandPts / kStep;     // points per staged piece
+  // groups in straight-line code: 4 where they fit the registers (smooth, the
+  // scalar step profile: 2-5 % over 2), 2 elsewhere (4 there up to 11 %
+  // slower), 1 around a run-time node loop
+  constexpr int kUnroll = NINT == 0 ? 1 : NINT == 4 && (smooth_profile(P) || (P == kStep && !FERM)) ? 4 : 2;
+  const int lane = threadIdx.x & 31;
+  const int slot = tile * 32 + lane;
   const bool live = slot < A.ninst;
   const int sl = live ? slot : A.ninst - 1;
-  // every per-instance read and the partial-sum write go through ic: a
-  // thread's result does not depend on which slot it runs in
+  // every per-instance read and the partial-sum write go through ic: a lane's
+  // result does not depend on which slot it runs in
   const int ic = A.perm ? A.perm[sl] : sl;
-  const int l0 = chunk * A.chunk_loops;
-  const int nck = (A.ppl + kSweepChunkPts - 1) / kSweepChunkPts;
-  const int K = A.chunk_loops * nck;
-  float4 *const ring = S.ring;
-  uint64_t *const full_bar = S.full_bar;
-
-  const float cx = A.cx[ic], cy = A.cy[ic], s = A.rtT[ic];
   const FieldDev &F = A.field;
-  const df tq = {A.tqh[ic], A.tql[ic]};
-  const int base = consumed;
+  const V cx = vset(V(), A.cx[ic]), cy = vset(V(), A.cy[ic]), s = vset(V(), A.rtT[ic]);
 
-  auto issue = [&](int k) {  // chunk k -> stage (base + k) % kSweepStages
-    const int st = (base + k) % kSweepStages;
-    const int l = l0 + k / nck, c = k % nck;
-    const int p0 = c * kSweepChunkPts;
-    const int np = min(kSweepChunkPts, A.ppl - p0);
-    const uint32_t bytes = (uint32_t)np * (uint32_t)sizeof(float4);
-    mbar_arrive_expect_tx(&full_bar[st], bytes);
-    bulk_g2s(ring + st * kSweepChunkPts, A.loops + (size_t)l * A.ppl + p0, bytes,
-             &full_bar[st]);
+  auto issue = [&](int l, int p0) {  // points p0.. of the kStep loops from l
+    const uint32_t bytes = (uint32_t)(min(kPiece, A.ppl - p0) * (int)sizeof(float4));
+    const bool two = PAIR && l + 1 < l1;
+    mbar_arrive_expect_tx(W.bar, two ? 2 * bytes : bytes);
+    const float4 *src = A.loops + (size_t)l * A.ppl + p0;
+    bulk_g2s(W.land, src, bytes, W.bar);
+    if (two) bulk_g2s(W.land + kPiece, src + A.ppl, bytes, W.bar);
   };
-  if (tid == 0)
-    for (int k = 0; k < K && k < kSweepStages; ++k) issue(k);
+  if (lane == 0) issue(l0, 0);
 
+  // running sums of the current loops: phase and spin, each with compensation
+  V ph[3], pc[3], sp[3], sc[3], bp[3], bs[3];
+  const V zero = vset(V(), 0.f);
+  // previous point of each sub-loop
+  V zAx = zero, zAy = zero, zBx = zero, zBy = zero, zOx = zero, zOy = zero;
 #pragma unroll
-  for (int r = 0; r < kMaxF * 3; ++r) S.sacc[r][tid] = 0.0;
-
-  // running sums of the current loop: phase and spin, each with compensation
-  float ph[3] = {0.f, 0.f, 0.f}, pc[3] = {0.f, 0.f, 0.f};
-  float sp[3] = {0.f, 0.f, 0.f}, sc[3] = {0.f, 0.f, 0.f};
-  // previous point of each sub-loop and the first points (closing segments)
-  float zAx = 0.f, zAy = 0.f, zBx = 0.f, zBy = 0.f, zOx = 0.f, zOy = 0.f;
-  float z0x = 0.f, z0y = 0.f, z1x = 0.f, z1y = 0.f, z2x = 0.f, z2y = 0.f;
+  for (int r = 0; r < 3; ++r) ph[r] = pc[r] = sp[r] = sc[r] = bp[r] = bs[r] = zero;
   ImgRange img = {0, -1, 0, -1, 1};  // lattice images of the current loop
+  const int nq = A.ppl >> 2;
 
-  int k = 0;
-  for (; k < K; ++k) {
-    const int st = (base + k) % kSweepStages;
-    const uint32_t par = (uint32_t)((base + k) / kSweepStages) & 1u;
-    if (!mbar_wait_bounded(&full_bar[st], par, A.wait_tries)) *S.bad = 1;
+  int l = l0, p0 = 0;  // the piece's loops and first point
+#pragma unroll 1
+  while (l < l1) {
+    const int np = min(kPiece, A.ppl - p0);
+    const bool last = p0 + kPiece >= A.ppl;
+    if (!warp_stage_wait(A, W)) return false;
+    // compact copy of the piece, then the landing zone is free for the next
+    if constexpr (PAIR) {
+      const int o = l + 1 < l1 ? kPiece : 0;
+      for (int i = lane; i < np; i += 32) {
+        const float2 a = *reinterpret_cast<const float2 *>(W.land + i);
+        const float2 b = *reinterpret_cast<const float2 *>(W.land + o + i);
+        W.comp[i] = make_float4(a.x, b.x, a.y, b.y);
+      }
+    } else {
+      for (int i = lane; i < np; i += 32)
+        reinterpret_cast<float2 *>(W.comp)[i] = *reinterpret_cast<const float2 *>(W.land + i);
+    }
+    __syncwarp();
+    const int ln = last ? l + kStep : l, pn = last ? 0 : p0 + kPiece;
+    if (lane == 0 && ln < l1) issue(ln, pn);
 
-    const int c = k % nck;
-    const int p0 = c * kSweepChunkPts;
-    const int p1 = min(A.ppl, p0 + kSweepChunkPts);
-    const float2 *pts = reinterpret_cast<const float2 *>(ring + st * kSweepChunkPts);
-    auto pt = [&](int p, float &x, float &y) {
-      const float2 v = pts[2 * (p - p0)];  // (x, y) of the float4 point
-      x = fmaf(s, v.x, cx);
-      y = fmaf(s, v.y, cy);
+    auto pt = [&](int p, V &x, V &y) {
+      if constexpr (PAIR) {
+        const float4 v = W.comp[p - p0];
+        x = fma2(s, make_float2(v.x, v.y), cx);
+        y = fma2(s, make_float2(v.z, v.w), cy);
+      } else {
+        const float2 v = reinterpret_cast<const float2 *>(W.comp)[p - p0];
+        x = fmaf(s, v.x, cx);
+        y = fmaf(s, v.y, cy);
+      }
     };
 
     int q = p0 >> 2;
-    const int qend = p1 >> 2;
-    if (c == 0) {  // first chunk of a loop: points 0..3 open the sub-loops
+    const int qend = (p0 + np) >> 2;
+    if (p0 == 0) {  // first piece of a loop: points 0..3 open the sub-loops
 #pragma unroll
-      for (int r = 0; r < 3; ++r) ph[r] = pc[r] = sp[r] = sc[r] = 0.f;
-      if constexpr (P == kLattice) img = image_range(A.bbox[l0 + k / nck], s, cx, cy, F);
-      float z3x, z3y;
-      pt(0, z0x, z0y);
+      for (int r = 0; r < 3; ++r) ph[r] = pc[r] = sp[r] = sc[r] = zero;
+      if constexpr (P == kLattice && !PAIR)
+        img = image_range(A.bbox[l], A.rtT[ic], A.cx[ic], A.cy[ic], F);
+      V z1x, z1y;
+      pt(0, zAx, zAy);
       pt(1, z1x, z1y);
-      pt(2, z2x, z2y);
-      pt(3, z3x, z3y);
-      seg<P, FERM, NINT>(z1x, z1y, z3x, z3y, F, img, ph[0], sp[0]);  // N/2: 1 -> 3
-      zAx = z0x; zAy = z0y;
-      zBx = z2x; zBy = z2y;
-      zOx = z3x; zOy = z3y;
+      pt(2, zBx, zBy);
+      pt(3, zOx, zOy);
+      vseg<P, FERM, NINT, true>(z1x, z1y, zOx, zOy, F, img, ph[0], sp[0]);  // N/2: 1 -> 3
       q = 1;
     }
     while (q < qend) {
-      const int qe = min(q + 8, qend);
-      float bp0 = 0.f, bp1 = 0.f, bp2 = 0.f, bs0 = 0.f, bs1 = 0.f, bs2 = 0.f;
+      const int be = min(block_end(q), nq), qe = min(be, qend);
       auto group = [&](int qq) {
-        float P0x, P0y, P1x, P1y, P2x, P2y, P3x, P3y;
+        V P0x, P0y, P1x, P1y, P2x, P2y, P3x, P3y;
         pt(4 * qq, P0x, P0y);
         pt(4 * qq + 1, P1x, P1y);
         pt(4 * qq + 2, P2x, P2y);
         pt(4 * qq + 3, P3x, P3y);
-        seg<P, FERM, NINT>(zAx, zAy, P0x, P0y, F, img, bp2, bs2);  // N/4a: 4q-4 -> 4q
-        seg<P, FERM, NINT>(zOx, zOy, P1x, P1y, F, img, bp0, bs0);  // N/2 : 4q-1 -> 4q+1
-        seg<P, FERM, NINT>(zBx, zBy, P2x, P2y, F, img, bp1, bs1);  // N/4b: 4q-2 -> 4q+2
-        seg<P, FERM, NINT>(P1x, P1y, P3x, P3y, F, img, bp0, bs0);  // N/2 : 4q+1 -> 4q+3
+        vseg<P, FERM, NINT>(zAx, zAy, P0x, P0y, F, img, bp[2], bs[2]);  // N/4a: 4q-4 -> 4q
+        vseg<P, FERM, NINT>(zOx, zOy, P1x, P1y, F, img, bp[0], bs[0]);  // N/2 : 4q-1 -> 4q+1
+        vseg<P, FERM, NINT>(zBx, zBy, P2x, P2y, F, img, bp[1], bs[1]);  // N/4b: 4q-2 -> 4q+2
+        vseg<P, FERM, NINT>(P1x, P1y, P3x, P3y, F, img, bp[0], bs[0]);  // N/2 : 4q+1 -> 4q+3
         zAx = P0x; zAy = P0y;
         zBx = P2x; zBy = P2y;
         zOx = P3x; zOy = P3y;
@@ -149,71 +248,71 @@ __device__ __forceinline__ bool sweep_tile(const SweepArgs &A, int tile_x, int c
 #pragma unroll 1
         for (; q < qe; ++q) group(q);
       } else {
-#pragma unroll 2
+#pragma unroll kUnroll
         for (; q < qe; ++q) group(q);
       }
-      kahan_add(ph[0], pc[0], bp0);
-      kahan_add(ph[1], pc[1], bp1);
-      kahan_add(ph[2], pc[2], bp2);
-      if (FERM) {
-        kahan_add(sp[0], sc[0], bs0);
-        kahan_add(sp[1], sc[1], bs1);
-        kahan_add(sp[2], sc[2], bs2);
+      if (q == be) {  // the block is complete (it may span two pieces)
+#pragma unroll
+        for (int r = 0; r < 3; ++r) {
+          vkahan(ph[r], pc[r], bp[r]);
+          if (FERM) vkahan(sp[r], sc[r], bs[r]);
+          bp[r] = bs[r] = zero;
+        }
       }
     }
 
-    if (c == nck - 1) {  // last chunk: closing segments back to points 1, 0, 2
-      float tp0 = 0.f, tp1 = 0.f, tp2 = 0.f, ts0 = 0.f, ts1 = 0.f, ts2 = 0.f;
-      seg<P, FERM, NINT>(zOx, zOy, z1x, z1y, F, img, tp0, ts0);  // N/2 : N-1 -> 1
-      seg<P, FERM, NINT>(zBx, zBy, z2x, z2y, F, img, tp1, ts1);  // N/4b: N-2 -> 2
-      seg<P, FERM, NINT>(zAx, zAy, z0x, z0y, F, img, tp2, ts2);  // N/4a: N-4 -> 0
-      kahan_add(ph[0], pc[0], tp0);
-      kahan_add(ph[1], pc[1], tp1);
-      kahan_add(ph[2], pc[2], tp2);
-      kahan_add(sp[0], sc[0], ts0);
-      kahan_add(sp[1], sc[1], ts1);
-      kahan_add(sp[2], sc[2], ts2);
-      const df G[3] = {fast_two_sum(ph[0], -pc[0]), fast_two_sum(ph[1], -pc[1]),
-                       fast_two_sum(ph[2], -pc[2])};
-      const df H[3] = {fast_two_sum(sp[0], -sc[0]), fast_two_sum(sp[1], -sc[1]),
-                       fast_two_sum(sp[2], -sc[2])};
-      loop_epilogue<FERM>(G, H, A.cph_hi, A.cph_lo, A.csp_hi, A.csp_lo, tq, A.nF,
-                          [&](int j, double w0, double w1, double w2) {
-                            S.sacc[3 * j][tid] += w0;
-                            S.sacc[3 * j + 1][tid] += w1;
-                            S.sacc[3 * j + 2][tid] += w2;
-                          });
+    if (last) {  // last piece: closing segments back to points 1, 0, 2
+      // (read again from the ensemble: kept since the first piece they would
+      // hold six registers, twelve on a pair, through the whole walk)
+      V tp[3] = {zero, zero, zero}, ts[3] = {zero, zero, zero};
+      const float2 *g = reinterpret_cast<const float2 *>(A.loops + (size_t)l * A.ppl);
+      auto gpt = [&](int p, V &x, V &y) {
+        const float2 a = __ldg(&g[2 * p]);
+        if constexpr (PAIR) {
+          const float2 b = l + 1 < l1 ? __ldg(&g[2 * ((size_t)A.ppl + p)]) : a;
+          x = fma2(s, make_float2(a.x, b.x), cx);
+          y = fma2(s, make_float2(a.y, b.y), cy);
+        } else {
+          x = fmaf(s, a.x, cx);
+          y = fmaf(s, a.y, cy);
+        }
+      };
+      V zx, zy;
+      gpt(1, zx, zy);
+      vseg<P, FERM, NINT, true>(zOx, zOy, zx, zy, F, img, tp[0], ts[0]);  // N/2 : N-1 -> 1
+      gpt(2, zx, zy);
+      vseg<P, FERM, NINT, true>(zBx, zBy, zx, zy, F, img, tp[1], ts[1]);  // N/4b: N-2 -> 2
+      gpt(0, zx, zy);
+      vseg<P, FERM, NINT, true>(zAx, zAy, zx, zy, F, img, tp[2], ts[2]);  // N/4a: N-4 -> 0
+#pragma unroll
+      for (int r = 0; r < 3; ++r) {
+        vkahan(ph[r], pc[r], tp[r]);
+        vkahan(sp[r], sc[r], ts[r]);
+      }
+      const df tq = {A.tqh[ic], A.tql[ic]};
+#pragma unroll 1
+      for (int h = 0; h < kStep; ++h) {  // per-loop epilogue of each half
+        if (l + h >= l1) break;
+        const df G[3] = {fast_two_sum(vlane(ph[0], h), -vlane(pc[0], h)),
+                         fast_two_sum(vlane(ph[1], h), -vlane(pc[1], h)),
+                         fast_two_sum(vlane(ph[2], h), -vlane(pc[2], h))};
+        const df H[3] = {fast_two_sum(vlane(sp[0], h), -vlane(sc[0], h)),
+                         fast_two_sum(vlane(sp[1], h), -vlane(sc[1], h)),
+                         fast_two_sum(vlane(sp[2], h), -vlane(sc[2], h))};
+        const size_t at = A.per_loop ? row + (l - l0) + h : row;
+        const bool acc = !A.per_loop && l + h > l0;
+        loop_epilogue<FERM>(G, H, A.cph_hi, A.cph_lo, A.csp_hi, A.csp_lo, tq, A.nF,
+                            [&](int j, double w0, double w1, double w2) {
+                              if (live) put_loop(A, at, j, ic, acc, w0, w1, w2);
+                            });
+      }
     }
-
-    __syncthreads();  // every thread is done with stage st
-    if (*S.bad) break;
-    if (tid == 0 && k + kSweepStages < K) issue(k + kSweepStages);
-  }
-
-  if (*S.bad) {
-    // a copy did not arrive in time: wait (bounded) for the copies still in
-    // flight so that none lands after the CTA exits, report, write nothing
-    if (tid == 0) {
-      const int kend = min(K, k + kSweepStages);
-      for (int kk = k; kk < kend; ++kk)
-        mbar_wait_bounded(&full_bar[(base + kk) % kSweepStages],
-                          (uint32_t)((base + kk) / kSweepStages) & 1u, A.wait_tries);
-      atomicExch(A.status, kDevTimeout);
-    }
-    consumed = base + K;
-    return false;
-  }
-  consumed = base + K;
-
-  if (live) {
-    for (int r = 0; r < A.nF * 3; ++r)
-      A.partial[((size_t)chunk * A.nF * 3 + r) * A.ninst + ic] = S.sacc[r][tid];
+    __syncwarp();  // every lane is done with the compact piece
+    l = ln;
+    p0 = pn;
   }
   return true;
 }
-
-// instances of a packed-pair tile (two per thread)
-constexpr int kPairTile = 2 * kSweepThreads;
 
 // ------------------------------------------------ lattice, images outer --
 // One segment u_i -> u_j for two images at once (packed pair; u = the loop
@@ -322,8 +421,8 @@ constexpr float kLatFarChunk = 19.0f;
 // large-x form: the walk skips the small-x polynomial and its selects.
 constexpr float kLatMidChunk = 0.55f;
 constexpr int kLatSub = 32;  // staged points per far-test box
-constexpr int kLatNSub = kSweepChunkPts / kLatSub;
-static_assert(kSweepChunkPts % kLatSub == 0 && kLatSub % 4 == 0, "whole groups per box");
+constexpr int kLatNSub = kLandPts / kLatSub;
+static_assert(kLandPts % kLatSub == 0 && kLatSub % 4 == 0, "whole groups per box");
 
 // the rarely taken opening / closing segments as one called copy
 template <bool FERM>
@@ -334,71 +433,65 @@ __device__ __noinline__ float4 lat_seg2_called(float2 uix, float2 uiy, float2 uj
   return make_float4(ph.x, ph.y, sp.x, sp.y);
 }
 
-// Lattice tile at 4 intervals with the images outer: two instances A, B per
-// thread (slots t and t + 128 of the tile's instance order, 256 per CTA).  For
-// every staged chunk of a loop, the images of the two (loop, instance) pairs
-// walk all of the chunk's segments two at a time as packed f32x2 pairs:
-// A's image p beside B's image p while both have one, then the longer
-// list's remaining images two at a time -- ceil((K_A + K_B) / 2) walks, and
-// at step p the lanes of a warp hold images in the same position relative
-// to similar instances.  A loop point minus an image centre is
-// image-independent up to the shift, so the walk starts from the raw
-// unit-loop points (reloaded from L2, the same address for every thread);
-// per image pair the walk is uniform across the warp (no per-segment image
-// loop, no row logic).  An instance's images are its range of image_range()
-// flattened row by row (k -> m0 + k / w, n0 + k % w), its rows trimmed to
-// the |R| disk where the range crosses it; an unused half is computed and
-// not added.  Each image's walk
-// over the chunk is summed in FP32 and added once, in image order, to its
-// instance's Kahan-compensated loop totals: an instance's sums do not depend
-// on its partner or on the tile's other instances.
+// Lattice unit of a warp at 4 intervals with the images outer: two instances
+// A, B per lane (slots t and t + 32 of the unit's 64 in the instance order),
+// one loop at a time.  For every staged piece of a loop, the images of the two
+// (loop, instance) pairs walk all of the piece's segments two at a time as
+// packed f32x2 pairs: A's image p beside B's image p while both have one, then
+// the longer list's remaining images two at a time -- ceil((K_A + K_B) / 2)
+// walks, and at step p the lanes of a warp hold images in the same position
+// relative to similar instances.  A loop point minus an image centre is
+// image-independent up to the shift, so the walk starts from the raw unit-loop
+// points, staged with each coordinate twice (x, x, y, y) so that one 16-byte
+// broadcast load gives both packed operands; per image pair the walk is uniform
+// across the warp (no per-segment image loop, no row logic).  An instance's
+// images are its range of image_range() flattened row by row (k -> m0 + k / w,
+// n0 + k % w), its rows trimmed to the |R| disk where the range crosses it; an
+// unused half is computed and not added.  Each image's walk over the piece is
+// summed in FP32 and added once, in image order, to its instance's
+// Kahan-compensated loop totals: an instance's sums do not depend on its
+// partner or on the unit's other instances.  Warps do not wait for one another:
+// the image counts of a CTA's four warps differ, and a barrier per piece (128
+// threads, 256 instances per tile) held them to the largest; 512 instances on
+// 1024 x 1024 points, a = 5 lambda, spinor: 29.0 -> 18.0 ms alone.
 
-// shared-memory rows of the lattice tile's loop totals: [instance A/B][phase,
-// its compensation, spin, its compensation][sub-loop] x 128 threads (kept out
-// of registers: they are touched once per image walk)
+// shared-memory rows of the loop totals: [instance A/B][phase, its
+// compensation, spin, its compensation][sub-loop] x 32 lanes (kept out of
+// registers: they are touched once per image walk)
 constexpr int kLatTotRows = 2 * 4 * 3;
+// compact points of a lattice piece: the 4 before it, the piece, the loop's first 4
+constexpr int kLatPts = kLandPts + 8, kLatFirst = kLandPts + 4;
 
 // MIDWALK: walk the blocks between near and far with the large-x form alone
 // (the single-job kernel; inside the persistent batch kernel the extra walk
-// measured 3 % slower on the uneven batch, so its tiles keep two walks --
+// measured 3 % slower on the uneven batch, so its units keep two walks --
 // the sums are the same bits either way)
 template <bool FERM, bool MIDWALK>
-__device__ __forceinline__ bool sweep_tile_lat(const SweepArgs &A, int tile_x, int chunk,
-                                               uint64_t *full_bar, double (*sacc)[kPairTile],
-                                               float (*tot)[kSweepThreads], int *bad,
-                                               float4 *ring, int &consumed) {
-  const int tid = threadIdx.x;
-  // slots t and t + 128: a tile holding 128 or fewer instances gives each
-  // thread at most one (the lanes of a warp still hold consecutive slots)
-  const int sA = tile_x * kPairTile + tid, sB = sA + kSweepThreads;
+__device__ __forceinline__ bool warp_unit_lat(const SweepArgs &A, int tile, int l0, int l1,
+                                              size_t row, WarpStage &W, float (*tot)[32],
+                                              float4 *box) {
+  const int lane = threadIdx.x & 31;
+  // slots t and t + 32: a unit holding 32 or fewer instances gives each lane
+  // at most one (the lanes of a warp still hold consecutive slots)
+  const int sA = tile * 64 + lane, sB = sA + 32;
   const bool liveA = sA < A.ninst, liveB = sB < A.ninst;
   const int slA = liveA ? sA : A.ninst - 1, slB = liveB ? sB : A.ninst - 1;
   const int iA = A.perm ? A.perm[slA] : slA, iB = A.perm ? A.perm[slB] : slB;
-  const int l0 = chunk * A.chunk_loops;
-  const int nck = (A.ppl + kSweepChunkPts - 1) / kSweepChunkPts;
-  const int K = A.chunk_loops * nck;
+  const int npc = (A.ppl + kLandPts - 1) / kLandPts;
+  const int K = (l1 - l0) * npc;
   const FieldDev &F = A.field;
-  const int base = consumed;
 
   auto issue = [&](int k) {
-    const int st = (base + k) % kSweepStages;
-    const int l = l0 + k / nck, c = k % nck;
-    const int p0 = c * kSweepChunkPts;
-    const int np = min(kSweepChunkPts, A.ppl - p0);
-    const uint32_t bytes = (uint32_t)np * (uint32_t)sizeof(float4);
-    mbar_arrive_expect_tx(&full_bar[st], bytes);
-    bulk_g2s(ring + st * kSweepChunkPts, A.loops + (size_t)l * A.ppl + p0, bytes, &full_bar[st]);
+    const int l = l0 + k / npc, p0 = k % npc * kLandPts;
+    const uint32_t bytes = (uint32_t)(min(kLandPts, A.ppl - p0) * (int)sizeof(float4));
+    mbar_arrive_expect_tx(W.bar, bytes);
+    bulk_g2s(W.land, A.loops + (size_t)l * A.ppl + p0, bytes, W.bar);
   };
-  if (tid == 0)
-    for (int k = 0; k < K && k < kSweepStages; ++k) issue(k);
-#pragma unroll
-  for (int r = 0; r < kMaxF * 3; ++r) sacc[r][tid] = sacc[r][tid + kSweepThreads] = 0.0;
+  if (lane == 0) issue(0);
 
   const float2 il2 = f2(F.inv_l2);
-  // per warp: the staged chunk's far-test boxes (xmin, xmax, ymin, ymax)
-  __shared__ float4 lat_box[kSweepThreads / 32][kLatNSub];
   // loop totals per instance (h = 0: A, 1: B), Kahan-compensated, in tot[]
-  auto T = [&](int h, int v, int r) -> float & { return tot[(h * 4 + v) * 3 + r][tid]; };
+  auto T = [&](int h, int v, int r) -> float & { return tot[(h * 4 + v) * 3 + r][lane]; };
   auto tot_add = [&](int h, int r, float vp, float vs) {
     float a = T(h, 0, r), ac = T(h, 1, r);
     kahan_add(a, ac, vp);
@@ -412,57 +505,63 @@ __device__ __forceinline__ bool sweep_tile_lat(const SweepArgs &A, int tile_x, i
     }
   };
 
-  int k = 0;
-  for (; k < K; ++k) {
-    const int st = (base + k) % kSweepStages;
-    const uint32_t par = (uint32_t)((base + k) / kSweepStages) & 1u;
-    if (!mbar_wait_bounded(&full_bar[st], par, A.wait_tries)) *bad = 1;
-    const int c = k % nck;
-    const int l = l0 + k / nck;
-    const int p0 = c * kSweepChunkPts;
-    const int p1 = min(A.ppl, p0 + kSweepChunkPts);
-    const float2 *pts = reinterpret_cast<const float2 *>(ring + st * kSweepChunkPts);
-    // (x, y) of loop point p: staged points from shared memory, others from L2
-    const float2 *gl = reinterpret_cast<const float2 *>(A.loops + (size_t)l * A.ppl);
-    auto raw = [&](int p) { return pts[2 * (p - p0)]; };
-    auto graw = [&](int p) { return __ldg(&gl[2 * p]); };
+#pragma unroll 1
+  for (int k = 0; k < K; ++k) {
+    const int c = k % npc;
+    const int l = l0 + k / npc;
+    const int p0 = c * kLandPts;
+    const int np = min(kLandPts, A.ppl - p0), p1 = p0 + np;
+    if (!warp_stage_wait(A, W)) return false;
+    // compact points: the last 4 of the piece before stay in front of this one
+    // (a piece that another follows is full), the first 4 of the loop behind
+    if (c > 0) {
+      float4 v;
+      if (lane < 4) v = W.comp[kLandPts + lane];
+      __syncwarp();
+      if (lane < 4) W.comp[lane] = v;
+    }
+    for (int i = lane; i < np; i += 32) {
+      const float2 a = *reinterpret_cast<const float2 *>(W.land + i);
+      const float4 v = make_float4(a.x, a.x, a.y, a.y);
+      W.comp[4 + i] = v;
+      if (c == 0 && i < 4) W.comp[kLatFirst + i] = v;
+    }
+    __syncwarp();
+    if (lane == 0 && k + 1 < K) issue(k + 1);
     if (c == 0) {
 #pragma unroll
-      for (int w = 0; w < kLatTotRows; ++w) tot[w][tid] = 0.f;
+      for (int w = 0; w < kLatTotRows; ++w) tot[w][lane] = 0.f;
     }
-    const bool last = c == nck - 1;
+    const bool last = c == npc - 1;
     // bounding boxes (unit loop) of the points each block of kLatSub staged
     // points' segments touch: the block's points and the four before it (the
-    // previous chunk's for the first block); each warp reduces its own copy
-    {
-      const int lane = tid & 31, w = tid >> 5;
+    // previous piece's for the first block)
 #pragma unroll 1
-      for (int b = 0; b < kLatNSub; ++b) {
-        const int lo = max(p0 + b * kLatSub - 4, c == 0 ? p0 : p0 - 4);
-        const int hi = min(p0 + (b + 1) * kLatSub, p1);
-        float x0 = INFINITY, x1 = -INFINITY, y0 = INFINITY, y1 = -INFINITY;
-        for (int i = lo + lane; i < hi; i += 32) {
-          const float2 v = i >= p0 ? raw(i) : graw(i);
-          x0 = fminf(x0, v.x);
-          x1 = fmaxf(x1, v.x);
-          y0 = fminf(y0, v.y);
-          y1 = fmaxf(y1, v.y);
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-          x0 = fminf(x0, __shfl_xor_sync(0xffffffffu, x0, o));
-          x1 = fmaxf(x1, __shfl_xor_sync(0xffffffffu, x1, o));
-          y0 = fminf(y0, __shfl_xor_sync(0xffffffffu, y0, o));
-          y1 = fmaxf(y1, __shfl_xor_sync(0xffffffffu, y1, o));
-        }
-        if (lane == 0) lat_box[w][b] = make_float4(x0, x1, y0, y1);
+    for (int b = 0; b < kLatNSub; ++b) {
+      const int lo = max(b * kLatSub - 4, c == 0 ? 0 : -4);
+      const int hi = min((b + 1) * kLatSub, np);
+      float x0 = INFINITY, x1 = -INFINITY, y0 = INFINITY, y1 = -INFINITY;
+      for (int i = lo + lane; i < hi; i += 32) {
+        const float4 v = W.comp[4 + i];
+        x0 = fminf(x0, v.x);
+        x1 = fmaxf(x1, v.x);
+        y0 = fminf(y0, v.z);
+        y1 = fmaxf(y1, v.z);
       }
-      __syncwarp();
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        x0 = fminf(x0, __shfl_xor_sync(0xffffffffu, x0, o));
+        x1 = fmaxf(x1, __shfl_xor_sync(0xffffffffu, x1, o));
+        y0 = fminf(y0, __shfl_xor_sync(0xffffffffu, y0, o));
+        y1 = fmaxf(y1, __shfl_xor_sync(0xffffffffu, y1, o));
+      }
+      if (lane == 0) box[b] = make_float4(x0, x1, y0, y1);
     }
+    __syncwarp();
     // the nearest point of block b's box, scaled and shifted as U() maps the
     // points (fma(s, w, c - R) is monotone in w), is far from the image centre
     auto block_x = [&](int b, float sc, float crx, float cry) {
-      const float4 bb = lat_box[tid >> 5][b];
+      const float4 bb = box[b];
       const float lx = fmaf(sc, bb.x, crx), hx = fmaf(sc, bb.y, crx);
       const float ly = fmaf(sc, bb.z, cry), hy = fmaf(sc, bb.w, cry);
       const float ex = fmaxf(fmaxf(lx, -hx), 0.0f), ey = fmaxf(fmaxf(ly, -hy), 0.0f);
@@ -475,7 +574,7 @@ __device__ __forceinline__ bool sweep_tile_lat(const SweepArgs &A, int tile_x, i
     const int widA = max(gA.n1 - gA.n0 + 1, 1), widB = max(gB.n1 - gB.n0 + 1, 1);
     // row m of a range trimmed to the disk m^2 + n^2 <= (rimage/a)^2 (the
     // criterion image_range uses for `inside`)
-    auto row = [&](const ImgRange &g, int m, int &lo, int &hi) {
+    auto row_of = [&](const ImgRange &g, int m, int &lo, int &hi) {
       const float mm = (float)(m * m);
       int nx = (int)floorf(sqrtf(fmaxf(F.rimg2 - mm, 0.0f)));
       while (nx >= 0 && mm + (float)(nx * nx) > F.rimg2) --nx;
@@ -486,19 +585,20 @@ __device__ __forceinline__ bool sweep_tile_lat(const SweepArgs &A, int tile_x, i
     auto count = [&](const ImgRange &g, int wid) {
       if (g.m1 < g.m0 || g.n1 < g.n0) return 0;
       if (g.inside) return (g.m1 - g.m0 + 1) * wid;
-      int c = 0;
+      int n = 0;
       for (int m = g.m0; m <= g.m1; ++m) {
         int lo, hi;
-        row(g, m, lo, hi);
-        c += max(hi - lo + 1, 0);
+        row_of(g, m, lo, hi);
+        n += max(hi - lo + 1, 0);
       }
-      return c;
+      return n;
     };
     // a slot past the tile's instances walks nothing
     const int nA = liveA ? count(gA, widA) : 0, nB = liveB ? count(gB, widB) : 0;
     const int mn = min(nA, nB), mx = max(nA, nB);
     const int steps = mn + (mx - mn + 1) / 2;
     const int qa = c == 0 ? 1 : (p0 >> 2), qend = p1 >> 2;
+    const float4 *const pts = W.comp + 4 - p0;  // loop point p of the piece
     for (int p = 0; p < steps; ++p) {
       // the step's two images: (A p, B p), then the longer list two at a time
       int jx, jy;
@@ -524,7 +624,7 @@ __device__ __forceinline__ bool sweep_tile_lat(const SweepArgs &A, int tile_x, i
           nn = g.n0;
           for (int mr = g.m0; mr <= g.m1; ++mr) {
             int lo, hi;
-            row(g, mr, lo, hi);
+            row_of(g, mr, lo, hi);
             const int cnt = max(hi - lo + 1, 0);
             if (jj < cnt) {
               m = mr;
@@ -547,35 +647,35 @@ __device__ __forceinline__ bool sweep_tile_lat(const SweepArgs &A, int tile_x, i
       const float2 s2 = make_float2(sx, sy);
       const float2 crx = make_float2(cxx, cxy), cry = make_float2(cyx, cyy);
       // point minus image centre, scaled: u = s w + (c - R)
-      auto U = [&](float2 w, float2 &ux, float2 &uy) {
-        ux = fma2(s2, f2(w.x), crx);
-        uy = fma2(s2, f2(w.y), cry);
+      auto U = [&](const float4 &w, float2 &ux, float2 &uy) {
+        ux = fma2(s2, make_float2(w.x, w.y), crx);
+        uy = fma2(s2, make_float2(w.z, w.w), cry);
       };
       float2 bp[3] = {f2(0.f), f2(0.f), f2(0.f)}, bs[3] = {f2(0.f), f2(0.f), f2(0.f)};
       float2 uAx, uAy, uBx, uBy, uOx, uOy;
       if (c == 0) {  // the N/2 sub-loop's first segment 1 -> 3; sub-loops open at 0, 2, 3
         float2 u1x, u1y, u3x, u3y;
-        U(raw(1), u1x, u1y);
-        U(raw(3), u3x, u3y);
+        U(pts[1], u1x, u1y);
+        U(pts[3], u3x, u3y);
         const float4 r = lat_seg2_called<FERM>(u1x, u1y, u3x, u3y, il2,
                                                make_float4(0.f, 0.f, 0.f, 0.f));
         bp[0] = make_float2(r.x, r.y);
         bs[0] = make_float2(r.z, r.w);
-        U(raw(0), uAx, uAy);
-        U(raw(2), uBx, uBy);
+        U(pts[0], uAx, uAy);
+        U(pts[2], uBx, uBy);
         uOx = u3x;
         uOy = u3y;
-      } else {  // the previous chunk's last points of each sub-loop
-        U(graw(p0 - 4), uAx, uAy);
-        U(graw(p0 - 2), uBx, uBy);
-        U(graw(p0 - 1), uOx, uOy);
+      } else {  // the previous piece's last points of each sub-loop
+        U(pts[p0 - 4], uAx, uAy);
+        U(pts[p0 - 2], uBx, uBy);
+        U(pts[p0 - 1], uOx, uOy);
       }
       auto group4 = [&](int q, auto &&segf) {
         float2 P0x, P0y, P1x, P1y, P2x, P2y, P3x, P3y;
-        U(raw(4 * q), P0x, P0y);
-        U(raw(4 * q + 1), P1x, P1y);
-        U(raw(4 * q + 2), P2x, P2y);
-        U(raw(4 * q + 3), P3x, P3y);
+        U(pts[4 * q], P0x, P0y);
+        U(pts[4 * q + 1], P1x, P1y);
+        U(pts[4 * q + 2], P2x, P2y);
+        U(pts[4 * q + 3], P3x, P3y);
         segf(uAx, uAy, P0x, P0y, 2);  // N/4a: 4q-4 -> 4q
         segf(uOx, uOy, P1x, P1y, 0);  // N/2 : 4q-1 -> 4q+1
         segf(uBx, uBy, P2x, P2y, 1);  // N/4b: 4q-2 -> 4q+2
@@ -618,33 +718,37 @@ __device__ __forceinline__ bool sweep_tile_lat(const SweepArgs &A, int tile_x, i
       if (last) {  // closing segments back to points 1, 2, 0
         float2 ux, uy;
         float4 r;
-        U(graw(1), ux, uy);
+        U(W.comp[kLatFirst + 1], ux, uy);
         r = lat_seg2_called<FERM>(uOx, uOy, ux, uy, il2,
                                   make_float4(bp[0].x, bp[0].y, bs[0].x, bs[0].y));
         bp[0] = make_float2(r.x, r.y);
         bs[0] = make_float2(r.z, r.w);
-        U(graw(2), ux, uy);
+        U(W.comp[kLatFirst + 2], ux, uy);
         r = lat_seg2_called<FERM>(uBx, uBy, ux, uy, il2,
                                   make_float4(bp[1].x, bp[1].y, bs[1].x, bs[1].y));
         bp[1] = make_float2(r.x, r.y);
         bs[1] = make_float2(r.z, r.w);
-        U(graw(0), ux, uy);
+        U(W.comp[kLatFirst], ux, uy);
         r = lat_seg2_called<FERM>(uAx, uAy, ux, uy, il2,
                                   make_float4(bp[2].x, bp[2].y, bs[2].x, bs[2].y));
         bp[2] = make_float2(r.x, r.y);
         bs[2] = make_float2(r.z, r.w);
       }
-      // each image's chunk sums into its instance's totals, in image order
+      // each image's piece sums into its instance's totals, in image order
 #pragma unroll
       for (int r = 0; r < 3; ++r) {
         if (okx) tot_add(bx ? 1 : 0, r, bp[r].x, bs[r].x);
         if (oky) tot_add(by ? 1 : 0, r, bp[r].y, bs[r].y);
       }
     }
+    __syncwarp();
     if (last) {
+      const size_t at = A.per_loop ? row + (l - l0) : row;
+      const bool acc = !A.per_loop && l > l0;
 #pragma unroll 1
       for (int h = 0; h < 2; ++h) {  // per-loop epilogue of each instance
-        const int ih = h ? iB : iA, col = tid + h * kSweepThreads;
+        const int ih = h ? iB : iA;
+        const bool live = h ? liveB : liveA;
         const df G[3] = {fast_two_sum(T(h, 0, 0), -T(h, 1, 0)),
                          fast_two_sum(T(h, 0, 1), -T(h, 1, 1)),
                          fast_two_sum(T(h, 0, 2), -T(h, 1, 2))};
@@ -654,241 +758,65 @@ __device__ __forceinline__ bool sweep_tile_lat(const SweepArgs &A, int tile_x, i
         const df tq = {A.tqh[ih], A.tql[ih]};
         loop_epilogue<FERM>(G, H, A.cph_hi, A.cph_lo, A.csp_hi, A.csp_lo, tq, A.nF,
                             [&](int j, double d0, double d1, double d2) {
-                              sacc[3 * j][col] += d0;
-                              sacc[3 * j + 1][col] += d1;
-                              sacc[3 * j + 2][col] += d2;
+                              if (live) put_loop(A, at, j, ih, acc, d0, d1, d2);
                             });
       }
     }
-    __syncthreads();
-    if (*bad) break;
-    if (tid == 0 && k + kSweepStages < K) issue(k + kSweepStages);
-  }
-  if (*bad) {
-    if (tid == 0) {
-      const int kend = min(K, k + kSweepStages);
-      for (int kk = k; kk < kend; ++kk)
-        mbar_wait_bounded(&full_bar[(base + kk) % kSweepStages],
-                          (uint32_t)((base + kk) / kSweepStages) & 1u, A.wait_tries);
-      atomicExch(A.status, kDevTimeout);
-    }
-    consumed = base + K;
-    return false;
-  }
-  consumed = base + K;
-  for (int r = 0; r < A.nF * 3; ++r) {
-    double *o = A.partial + ((size_t)chunk * A.nF * 3 + r) * A.ninst;
-    if (liveA) o[iA] = sacc[r][tid];
-    if (liveB) o[iB] = sacc[r][tid + kSweepThreads];
+    __syncwarp();  // every lane is done with the compact piece
   }
   return true;
 }
 
-// The same tile on packed pairs: thread t runs instances t and t + 128 of a
-// tile of kPairTile, every FP32 operation of the segments as one f32x2
-// operation on the pair (each half rounds as the scalar sweep does); the
-// per-loop epilogue runs per half.  Light profiles with a fixed interval count.
-template <int P, bool FERM, int NINT>
-__device__ __forceinline__ bool sweep_tile2(const SweepArgs &A, int tile_x, int chunk,
-                                            uint64_t *full_bar, double (*sacc)[kPairTile],
-                                            int *bad, float4 *ring, int &consumed) {
-  const int tid = threadIdx.x;
-  const int sA = tile_x * kPairTile + tid, sB = sA + kSweepThreads;
-  const bool liveA = sA < A.ninst, liveB = sB < A.ninst;
-  const int iA = liveA ? sA : A.ninst - 1, iB = liveB ? sB : A.ninst - 1;
-  const int l0 = chunk * A.chunk_loops;
-  const int nck = (A.ppl + kSweepChunkPts - 1) / kSweepChunkPts;
-  const int K = A.chunk_loops * nck;
-  const float2 cx = make_float2(A.cx[iA], A.cx[iB]), cy = make_float2(A.cy[iA], A.cy[iB]);
-  const float2 s = make_float2(A.rtT[iA], A.rtT[iB]);
-  const FieldDev &F = A.field;
-  const int base = consumed;
+// ------------------------------------------------------------- kernels --
+// bytes of dynamic shared memory per warp
+constexpr int kStageBytes = kLandPts * 16 + kLandPts * 8;
+constexpr int kLatStageBytes =
+    kLandPts * 16 + kLatPts * 16 + kLatTotRows * 32 * 4 + kLatNSub * 16;
+static_assert(kSweepWarps * kStageBytes == (int)sweep_smem_bytes() &&
+                  kSweepWarps * kLatStageBytes == (int)sweep_lat_smem_bytes(),
+              "the launch's shared memory");
 
-  auto issue = [&](int k) {
-    const int st = (base + k) % kSweepStages;
-    const int l = l0 + k / nck, c = k % nck;
-    const int p0 = c * kSweepChunkPts;
-    const int np = min(kSweepChunkPts, A.ppl - p0);
-    const uint32_t bytes = (uint32_t)np * (uint32_t)sizeof(float4);
-    mbar_arrive_expect_tx(&full_bar[st], bytes);
-    bulk_g2s(ring + st * kSweepChunkPts, A.loops + (size_t)l * A.ppl + p0, bytes,
-             &full_bar[st]);
-  };
-  if (tid == 0)
-    for (int k = 0; k < K && k < kSweepStages; ++k) issue(k);
-#pragma unroll
-  for (int r = 0; r < kMaxF * 3; ++r) sacc[r][tid] = sacc[r][tid + kSweepThreads] = 0.0;
-
-  float2 ph[3], pc[3], sp[3], sc[3];
-  float2 zAx = f2(0.f), zAy = f2(0.f), zBx = f2(0.f), zBy = f2(0.f), zOx = f2(0.f), zOy = f2(0.f);
-  float2 z0x = f2(0.f), z0y = f2(0.f), z1x = f2(0.f), z1y = f2(0.f), z2x = f2(0.f), z2y = f2(0.f);
-#pragma unroll
-  for (int r = 0; r < 3; ++r) ph[r] = pc[r] = sp[r] = sc[r] = f2(0.f);
-
-  int k = 0;
-  for (; k < K; ++k) {
-    const int st = (base + k) % kSweepStages;
-    const uint32_t par = (uint32_t)((base + k) / kSweepStages) & 1u;
-    if (!mbar_wait_bounded(&full_bar[st], par, A.wait_tries)) *bad = 1;
-    const int c = k % nck;
-    const int p0 = c * kSweepChunkPts;
-    const int p1 = min(A.ppl, p0 + kSweepChunkPts);
-    const float2 *pts = reinterpret_cast<const float2 *>(ring + st * kSweepChunkPts);
-    auto pt = [&](int p, float2 &x, float2 &y) {
-      const float2 v = pts[2 * (p - p0)];
-      x = fma2(s, f2(v.x), cx);
-      y = fma2(s, f2(v.y), cy);
-    };
-    int q = p0 >> 2;
-    const int qend = p1 >> 2;
-    if (c == 0) {
-#pragma unroll
-      for (int r = 0; r < 3; ++r) ph[r] = pc[r] = sp[r] = sc[r] = f2(0.f);
-      float2 z3x, z3y;
-      pt(0, z0x, z0y);
-      pt(1, z1x, z1y);
-      pt(2, z2x, z2y);
-      pt(3, z3x, z3y);
-      seg2<P, FERM, NINT>(z1x, z1y, z3x, z3y, F, ph[0], sp[0]);
-      zAx = z0x; zAy = z0y;
-      zBx = z2x; zBy = z2y;
-      zOx = z3x; zOy = z3y;
-      q = 1;
-    }
-    while (q < qend) {
-      const int qe = min(q + 8, qend);
-      float2 bp0 = f2(0.f), bp1 = f2(0.f), bp2 = f2(0.f), bs0 = f2(0.f), bs1 = f2(0.f),
-             bs2 = f2(0.f);
-#pragma unroll 2
-      for (; q < qe; ++q) {
-        float2 P0x, P0y, P1x, P1y, P2x, P2y, P3x, P3y;
-        pt(4 * q, P0x, P0y);
-        pt(4 * q + 1, P1x, P1y);
-        pt(4 * q + 2, P2x, P2y);
-        pt(4 * q + 3, P3x, P3y);
-        seg2<P, FERM, NINT>(zAx, zAy, P0x, P0y, F, bp2, bs2);
-        seg2<P, FERM, NINT>(zOx, zOy, P1x, P1y, F, bp0, bs0);
-        seg2<P, FERM, NINT>(zBx, zBy, P2x, P2y, F, bp1, bs1);
-        seg2<P, FERM, NINT>(P1x, P1y, P3x, P3y, F, bp0, bs0);
-        zAx = P0x; zAy = P0y;
-        zBx = P2x; zBy = P2y;
-        zOx = P3x; zOy = P3y;
-      }
-      kahan_add2(ph[0], pc[0], bp0);
-      kahan_add2(ph[1], pc[1], bp1);
-      kahan_add2(ph[2], pc[2], bp2);
-      if (FERM) {
-        kahan_add2(sp[0], sc[0], bs0);
-        kahan_add2(sp[1], sc[1], bs1);
-        kahan_add2(sp[2], sc[2], bs2);
-      }
-    }
-    if (c == nck - 1) {
-      float2 tp0 = f2(0.f), tp1 = f2(0.f), tp2 = f2(0.f), ts0 = f2(0.f), ts1 = f2(0.f),
-             ts2 = f2(0.f);
-      seg2<P, FERM, NINT>(zOx, zOy, z1x, z1y, F, tp0, ts0);
-      seg2<P, FERM, NINT>(zBx, zBy, z2x, z2y, F, tp1, ts1);
-      seg2<P, FERM, NINT>(zAx, zAy, z0x, z0y, F, tp2, ts2);
-      kahan_add2(ph[0], pc[0], tp0);
-      kahan_add2(ph[1], pc[1], tp1);
-      kahan_add2(ph[2], pc[2], tp2);
-      kahan_add2(sp[0], sc[0], ts0);
-      kahan_add2(sp[1], sc[1], ts1);
-      kahan_add2(sp[2], sc[2], ts2);
-#pragma unroll 1
-      for (int h = 0; h < 2; ++h) {  // per-loop epilogue of each half
-        auto lane = [h](float2 v) { return h ? v.y : v.x; };
-        const int ih = h ? iB : iA, col = tid + h * kSweepThreads;
-        const df G[3] = {fast_two_sum(lane(ph[0]), -lane(pc[0])),
-                         fast_two_sum(lane(ph[1]), -lane(pc[1])),
-                         fast_two_sum(lane(ph[2]), -lane(pc[2]))};
-        const df H[3] = {fast_two_sum(lane(sp[0]), -lane(sc[0])),
-                         fast_two_sum(lane(sp[1]), -lane(sc[1])),
-                         fast_two_sum(lane(sp[2]), -lane(sc[2]))};
-        const df tq = {A.tqh[ih], A.tql[ih]};
-        loop_epilogue<FERM>(G, H, A.cph_hi, A.cph_lo, A.csp_hi, A.csp_lo, tq, A.nF,
-                            [&](int j, double w0, double w1, double w2) {
-                              sacc[3 * j][col] += w0;
-                              sacc[3 * j + 1][col] += w1;
-                              sacc[3 * j + 2][col] += w2;
-                            });
-      }
-    }
-    __syncthreads();
-    if (*bad) break;
-    if (tid == 0 && k + kSweepStages < K) issue(k + kSweepStages);
-  }
-  if (*bad) {
-    if (tid == 0) {
-      const int kend = min(K, k + kSweepStages);
-      for (int kk = k; kk < kend; ++kk)
-        mbar_wait_bounded(&full_bar[(base + kk) % kSweepStages],
-                          (uint32_t)((base + kk) / kSweepStages) & 1u, A.wait_tries);
-      atomicExch(A.status, kDevTimeout);
-    }
-    consumed = base + K;
-    return false;
-  }
-  consumed = base + K;
-  for (int r = 0; r < A.nF * 3; ++r) {
-    double *o = A.partial + ((size_t)chunk * A.nF * 3 + r) * A.ninst;
-    if (liveA) o[iA] = sacc[r][tid];
-    if (liveB) o[iB] = sacc[r][tid + kSweepThreads];
-  }
-  return true;
+__device__ __forceinline__ WarpStage warp_stage(unsigned char *smem, uint64_t *bars, int bytes) {
+  const int w = threadIdx.x >> 5;
+  float4 *const land = reinterpret_cast<float4 *>(smem + w * bytes);
+  return WarpStage{land, land + kLandPts, bars + w, 0u};
 }
 
-template <int P, bool FERM, int NINT>
+// the lattice's totals and block boxes behind its compact points
+template <bool FERM, bool MIDWALK>
+__device__ __forceinline__ bool warp_unit_lattice(const SweepArgs &A, int tile, int l0, int l1,
+                                                  size_t row, WarpStage &W) {
+  float4 *const box = W.comp + kLatPts;
+  return warp_unit_lat<FERM, MIDWALK>(A, tile, l0, l1, row, W,
+                                      reinterpret_cast<float(*)[32]>(box + kLatNSub), box);
+}
+
+// loops [l0, l1) of unit u and the partial-sum row of its first
+__device__ __forceinline__ size_t unit_loops(const SweepArgs &A, int u, int &l0, int &l1) {
+  l0 = u * A.unit_loops;
+  l1 = min(l0 + A.unit_loops, A.n_chunks * A.chunk_loops);
+  return A.per_loop ? (size_t)l0 : (size_t)u;
+}
+
+// warp -> (unit, instance tile), the tiles of a unit on consecutive warps
+template <int P, bool FERM, int NINT, bool PAIR>
 __global__ void __launch_bounds__(kSweepThreads, 4)
-    sweep2_kernel(const __grid_constant__ SweepArgs A) {
-  extern __shared__ __align__(128) float4 ring[];
-  __shared__ __align__(8) uint64_t full_bar[kSweepStages];
-  __shared__ int sm_bad;
-  __shared__ double sacc[kMaxF * 3][kPairTile];
-  if (threadIdx.x == 0) {
-    for (int st = 0; st < kSweepStages; ++st) mbar_init(&full_bar[st], 1);
-    fence_mbar_init();
-    sm_bad = 0;
-  }
-  __syncthreads();
-  int consumed = 0;
-  sweep_tile2<P, FERM, NINT>(A, blockIdx.x, blockIdx.y, full_bar, sacc, &sm_bad, ring, consumed);
-}
-
-template <int P, bool FERM, int NINT>
-__global__ void __launch_bounds__(kSweepThreads,
-                                  (Profile<P>::kHeavy || P == kLattice) ? 4 : kSweepMinBlocks)
     sweep_kernel(const __grid_constant__ SweepArgs A) {
-  extern __shared__ __align__(128) float4 ring[];  // [kSweepStages][kSweepChunkPts]
-  __shared__ __align__(8) uint64_t full_bar[kSweepStages];
-  __shared__ int sm_bad;
-  // FP64 W-factor sums per (flux value, factor, instance): kept in shared
-  // memory (touched once per loop) so they do not hold 24 registers
-  __shared__ double sacc[kMaxF * 3][kSweepThreads];
-  const SweepShared S = {full_bar, sacc, &sm_bad, ring};
-  sweep_shared_init(S);
-  int consumed = 0;
-  sweep_tile<P, FERM, NINT>(A, blockIdx.x, blockIdx.y, S, consumed);
-}
-
-// the lattice at 4 intervals: images outer, two instances per thread
-template <bool FERM>
-__global__ void __launch_bounds__(kSweepThreads, 4)
-    sweep_lat_kernel(const __grid_constant__ SweepArgs A) {
-  extern __shared__ __align__(128) float4 ring[];
-  __shared__ __align__(8) uint64_t full_bar[kSweepStages];
-  __shared__ int sm_bad;
-  __shared__ double sacc[kMaxF * 3][kPairTile];
-  __shared__ float tot[kLatTotRows][kSweepThreads];
-  if (threadIdx.x == 0) {
-    for (int st = 0; st < kSweepStages; ++st) mbar_init(&full_bar[st], 1);
-    fence_mbar_init();
-    sm_bad = 0;
-  }
-  __syncthreads();
-  int consumed = 0;
-  sweep_tile_lat<FERM, true>(A, blockIdx.x, blockIdx.y, full_bar, sacc, tot, &sm_bad, ring,
-                             consumed);
+  extern __shared__ __align__(128) unsigned char smem[];
+  __shared__ __align__(8) uint64_t bars[kSweepWarps];
+  const unsigned item = blockIdx.x * kSweepWarps + (threadIdx.x >> 5);
+  const unsigned u = item / (unsigned)A.n_tiles;
+  if (u >= (unsigned)A.n_units) return;  // whole warp
+  constexpr bool kLat4 = P == kLattice && PAIR;
+  WarpStage W = warp_stage(smem, bars, kLat4 ? kLatStageBytes : kStageBytes);
+  warp_stage_init(W.bar);
+  int l0, l1;
+  const size_t row = unit_loops(A, u, l0, l1);
+  const int tile = item % (unsigned)A.n_tiles;
+  if constexpr (kLat4)
+    warp_unit_lattice<FERM, true>(A, tile, l0, l1, row, W);
+  else
+    warp_unit<P, FERM, NINT, PAIR>(A, tile, l0, l1, row, W);
 }
 
 template <int P, bool FERM, int NINT>
@@ -962,63 +890,50 @@ __global__ void __launch_bounds__(kLoopWarps * 32)
 }
 
 // instantiation + dispatch over (fermion, nint) for one profile
+template <int P, bool FERM, int NINT, bool PAIR>
+cudaError_t sweep_launch(SweepArgs a, cudaStream_t s) {
+  constexpr bool kLat4 = P == kLattice && PAIR;
+  const int per = kLat4 ? 64 : 32;
+  a.n_tiles = (a.ninst + per - 1) / per;
+  const long long items = (long long)a.n_tiles * a.n_units;
+  const long long ctas = (items + kSweepWarps - 1) / kSweepWarps;
+  if (ctas > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
+  constexpr size_t smem = kLat4 ? sweep_lat_smem_bytes() : sweep_smem_bytes();
+  auto k = sweep_kernel<P, FERM, NINT, PAIR>;
+  if (smem > 48 * 1024) {  // a per-device attribute
+    const cudaError_t e =
+        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+  }
+  k<<<(unsigned)ctas, kSweepThreads, smem, s>>>(a);
+  return cudaGetLastError();
+}
+
 template <int P>
 cudaError_t sweep_dispatch(bool fermion, int nint, const SweepArgs &a, cudaStream_t s) {
-  const dim3 grid((a.ninst + kSweepThreads - 1) / kSweepThreads, a.n_chunks);
-  const size_t smem = sweep_smem_bytes();
-  const dim3 grid2((a.ninst + kPairTile - 1) / kPairTile, a.n_chunks);
-  if constexpr (P == kSmooth || P == kStep || P == kQuadratic || P == kGaussian) {
-    if (nint == 4) {  // packed pairs
-      if (fermion)
-        sweep2_kernel<P, true, 4><<<grid2, kSweepThreads, smem, s>>>(a);
-      else
-        sweep2_kernel<P, false, 4><<<grid2, kSweepThreads, smem, s>>>(a);
-      return cudaGetLastError();
-    }
+  constexpr bool kLight = P == kSmooth || P == kStep || P == kQuadratic || P == kGaussian;
+  if constexpr (P == kSmooth) {
+    const float c = a.field.clampA;
+    if (nint == 4 && (c < 0.0f || a.field.l2 + c == a.field.l2))
+      return fermion ? sweep_launch<kSmoothWide, true, 4, true>(a, s)
+                     : sweep_launch<kSmoothWide, false, 4, true>(a, s);
   }
-#ifndef WL_PAIRS50
-#define WL_PAIRS50 1
-#endif
-  if constexpr ((P == kSmooth || P == kStep || P == kQuadratic || P == kGaussian) && WL_PAIRS50) {
-    if (nint == 50) {  // the reference's interval count: packed pairs (smooth:
-                       // a share of the reciprocals on the FP32 pipe); measured
-                       // over one instance per thread: smooth +3 % / +7 %
-                       // (scalar / spinor), Gaussian +56 % / +54 %, step
-                       // +4 % / +31 %, quadratic +35 % / +24 %
-      if (fermion)
-        sweep2_kernel<P, true, 50><<<grid2, kSweepThreads, smem, s>>>(a);
-      else
-        sweep2_kernel<P, false, 50><<<grid2, kSweepThreads, smem, s>>>(a);
-      return cudaGetLastError();
-    }
+#define WL_SWEEP_CASE(NI, PAIR)                                     \
+  if (NI == 0 || nint == NI)                                        \
+    return fermion ? sweep_launch<P, true, NI, PAIR>(a, s)          \
+                   : sweep_launch<P, false, NI, PAIR>(a, s);
+  if constexpr (kLight || P == kLattice) {
+    WL_SWEEP_CASE(4, true)  // light: packed pairs; lattice: images outer
   }
-  // one instance per thread: other interval counts at run time (a
-  // run-time-interval pair kernel measured 26 % slower than the unrolled
-  // scalar 50), the lattice at 4 too, and the heavy profiles; the scalar 50
-  // serves the loop-parallel kernel
-#define WL_SWEEP_CASE(FE, NI)                                                      \
-  if (fermion == FE && (NI == 0 || nint == NI)) {                                  \
-    sweep_kernel<P, FE, NI><<<grid, kSweepThreads, smem, s>>>(a);                  \
-    return cudaGetLastError();                                                     \
+  if constexpr (kLight) {
+    // the reference's interval count: packed pairs too (smooth: a share of the
+    // reciprocals on the FP32 pipe); measured over one instance per thread:
+    // smooth +20 % / +13 % (scalar / spinor), Gaussian +56 % / +54 %, step
+    // +4 % / +31 %, quadratic +35 % / +24 %
+    WL_SWEEP_CASE(50, true)
   }
-  if constexpr (P == kLattice) {
-    if (nint == 4) {  // images outer, two instances per thread
-      // static shared memory (37 KiB) plus the ring exceeds the 48 KiB a
-      // launch gets without opting in (a per-device attribute)
-      auto k = fermion ? sweep_lat_kernel<true> : sweep_lat_kernel<false>;
-      const cudaError_t e =
-          cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      if (e != cudaSuccess) return e;
-      k<<<grid2, kSweepThreads, smem, s>>>(a);
-      return cudaGetLastError();
-    }
-  }
-  if constexpr (!Profile<P>::kHeavy && P != kLattice) {
-    WL_SWEEP_CASE(true, 50)
-    WL_SWEEP_CASE(false, 50)
-  }
-  WL_SWEEP_CASE(true, 0)
-  WL_SWEEP_CASE(false, 0)
+  // other interval counts, the heavy profiles one loop at a time
+  WL_SWEEP_CASE(0, kLight)
 #undef WL_SWEEP_CASE
   return cudaErrorInvalidValue;
 }

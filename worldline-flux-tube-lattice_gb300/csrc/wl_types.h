@@ -15,8 +15,10 @@ enum : int {
   kSpline = 5,     // tabulated profile of periodic.c (clamped cubic spline)
   kFixflux = 6,
   kFixfluxFF = 7,  // fixflux with the intEVff.cu phi/chi fits
-  kLattice = 8     // square lattice of Gaussian tubes (image sum)
+  kLattice = 8,    // square lattice of Gaussian tubes (image sum)
+  kSmoothWide = 9  // kSmooth where the clamp of |z|^2 cannot act (kernels only)
 };
+constexpr bool smooth_profile(int p) { return p == kSmooth || p == kSmoothWide; }
 
 constexpr int kMaxF = 4;  // flux values sharing one geometric pass
 
