@@ -301,15 +301,20 @@ __device__ __forceinline__ bool fixflux_cf(float r2, const FieldDev &F, float &a
     x = 2.0f * (rho - n * a) / F.lam;
     if (x <= (FF ? -1.0f : -0.999f) || !(x * x < (FF ? 1.0f : 0.999f))) return false;
   }
-  arg = -1.0f / (1.0f - x * x);
+  arg = -1.0f / fmaf(-x, x, 1.0f);
   return true;
 }
 
 // FixfluxProfile::eval with the node's fraction value E given (used only
-// where fixflux_cf says the node needs it)
-template <bool FF>
-__device__ __forceinline__ void fixflux_eval(float r2, const FieldDev &F, float E, float &g,
-                                             float &fp) {
+// where fixflux_cf says the node needs it).  f is a called function and few
+// nodes are unrolled around it: its exponentials, sine and cosines are long,
+// and with eight inlined copies the warps of an SM waited for instructions 3.8
+// cycles per issue (64 instances on 512 x 512 points, spinor, 50 intervals:
+// 88.9 -> 42.2 ms; unrolled by 8 around the call 47.0).  Where a 1 - x^2 and
+// the sum in f' are rounded once or twice is written out: the roundings of the
+// kernel as it was inlined, so that results keep their bits.
+template <bool FF, bool FERM>
+__device__ __noinline__ float fixflux_f(float r2, const FieldDev &F, float E) {
   const float a = F.a, lam = F.lam, lml = F.lml, aml = F.aml;
   const float rho = sqrtf(r2);
   const float n = floorf((rho + 0.5f * a) / a);
@@ -324,7 +329,8 @@ __device__ __forceinline__ void fixflux_eval(float r2, const FieldDev &F, float 
     f = (1.0f - 0.75f * lml) * phi + 3.0f * r2 / (a * a) * lml;
   } else {
     const float x = 2.0f * (rho - n * a) / lam;
-    const float onemx2 = 1.0f - x * x, x2 = x * x, x4 = x2 * x2;
+    const float x2 = x * x, x4 = x2 * x2;
+    const float onemx2 = FERM && !FF ? fmaf(-x, x, 1.0f) : __fsub_rn(1.0f, __fmul_rn(x, x));
     float chi;
     if (x <= (FF ? -1.0f : -0.999f)) {
       chi = 0.0f;
@@ -345,12 +351,24 @@ __device__ __forceinline__ void fixflux_eval(float r2, const FieldDev &F, float 
     f = 1.0f + 0.75f * (4.0f * r2 / (a * a) - 1.0f) * lml + 3.0f * n * (n - 1.0f) * aml;
     f += 3.0f * lam / (0.443991f * a) * aml * chi;
   }
-  g = f / r2;
+  return f;
+}
+
+template <bool FF, bool FERM>
+__device__ __forceinline__ void fixflux_eval(float r2, const FieldDev &F, float E, float &g,
+                                             float &fp) {
+  const float a = F.a, lam = F.lam, lml = F.lml, aml = F.aml;
+  const float rho = sqrtf(r2);
+  const float n = floorf((rho + 0.5f * a) / a);
+  g = fixflux_f<FF, FERM>(r2, F, E) / r2;
   const float bbg = 3.0f / (a * a) * lml;
-  if (rho <= 0.5f * a)
-    fp = bbg + 2.0f / (F.l2 * 0.0742478f) * (1.0f - 0.75f * lml) * bump_d(2.0f * rho / lam);
-  else
-    fp = bbg + 6.0f / (0.443991f * lam * a) * aml * bump_d(2.0f * (rho - n * a) / lam);
+  const bool in = rho <= 0.5f * a;
+  const float om = fmaf(-0.75f, lml, 1.0f);
+  const float k = in ? 2.0f / (F.l2 * 0.0742478f) * om : 6.0f / (0.443991f * lam * a) * aml;
+  const float x = in ? 2.0f * rho / lam : 2.0f * (rho - n * a) / lam;
+  const float xx = __fmul_rn(x, x);
+  const float bump = xx < 0.999f ? expf(-1.0f / __fsub_rn(1.0f, xx)) : 0.0f;
+  fp = __fadd_rn(bbg, __fmul_rn(k, bump));
 }
 
 // nodes per gathering batch of the fixflux segment
@@ -415,7 +433,7 @@ __device__ __noinline__ float2 segment_fixflux(float zix, float ziy, float zjx, 
     __syncwarp(act);
     for (int q = rank; q < base; q += nact) cfq[w][q] = expint_lentz(cfq[w][q]);
     __syncwarp(act);
-#pragma unroll
+#pragma unroll 4
     for (int kk = 0; kk < kFfBatch; ++kk) {  // each lane's nodes, in order
       const int k = k0 + kk;
       if (k > n) break;
@@ -423,7 +441,7 @@ __device__ __noinline__ float2 segment_fixflux(float zix, float ziy, float zjx, 
       const unsigned m = cfm[w][kk];
       const float E = (m >> lane) & 1u ? cfq[w][cfo[w][kk] + __popc(m & lt)] : 0.0f;
       float g, fp;
-      fixflux_eval<FF>(node_r2(j), F, E, g, fp);
+      fixflux_eval<FF, FERM>(node_r2(j), F, E, g, fp);
       if (j == 0) {
         g0 = g;
         f0 = fp;

@@ -136,7 +136,7 @@ __device__ __forceinline__ int block_end(int q) {
 // pairs: Gaussian spinor at 16 intervals, 333 instances on 1500 x 516, 4.83 ->
 // 2.65 ms.  One lane per instance, one CTA per chunk -> one warp per loop, 50
 // intervals: periodic, 128 instances on 1024 x 512, 103 -> 32.7 ms; fixflux, 64
-// instances on 512 x 512, 375 -> 92 ms.
+// instances on 512 x 512, 375 -> 92 ms (48 with its segment's smaller code).
 //   row: the partial-sum row of loop l0 (per_loop) or of the unit's chunk.
 // Returns false if a copy timed out.
 template <int P, bool FERM, int NINT, bool PAIR>
@@ -414,7 +414,12 @@ __device__ __forceinline__ void lat_seg2_far(float2 uix, float2 uiy, float2 ujx,
 // way).  Measured on the a = 2, 5, 10 lambda lattice workloads against one
 // walk per segment with a vote: boxes of 32 points with vote-free near walks
 // 11-13 % faster; boxes of 64, 128, 256 points 0.5-3 % slower than 32; the
-// near walk with the vote kept 4-9 % slower; unrolled by 4, 4-25 % slower.
+// near walk with the vote kept 4-9 % slower.  The warps of an SM are in
+// different walks at any time, so the walks' instructions have to stay in the
+// instruction cache together: with the far and near walks unrolled by two
+// groups "no instruction" was the top stall (3.2 cycles per issue); one group
+// each (the middle walk keeps two) took 512 instances on 1024 x 1024 points,
+// a = 5 lambda, spinor, from 15.5 to 10.6 ms.
 constexpr float kLatFarChunk = 19.0f;
 // A block whose box stays at x > 0.55 from the image centres has every node
 // at x >= 0.5 (the same margin argument), where the integrand takes its
@@ -704,14 +709,14 @@ __device__ __forceinline__ bool warp_unit_lat(const SweepArgs &A, int tile, int 
         if (__all_sync(am, xb > kLatFarChunk)) {
           // every node of the block's walk is far: reciprocals only, no
           // per-segment vote, four segments of straight-line work per group
-#pragma unroll 2
+#pragma unroll 1
           for (int q = q0; q < q1; ++q) group4(q, far_seg);
         } else if (MIDWALK && __all_sync(am, xb > kLatMidChunk)) {
           // no node near an image centre: the integrand's large-x form alone
 #pragma unroll 2
           for (int q = q0; q < q1; ++q) group4(q, mid_seg);
         } else {
-#pragma unroll 2
+#pragma unroll 1
           for (int q = q0; q < q1; ++q) group4(q, near_seg);
         }
       }
