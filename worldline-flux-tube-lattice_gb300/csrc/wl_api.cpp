@@ -1727,10 +1727,11 @@ double EV(double T, void *p, int *WLlist) {
     a.ferm = f.fermion ? params.Wsferm_d : nullptr;
     unsigned long long fp = 0;
     cudaError_t ce = L.fpd.reserve(1);
-    if (ce == cudaSuccess) ce = wl::launch_fingerprint(params.worldlines, npts, L.fpd.p, ctx->stream);
+    if (ce == cudaSuccess) ce = cudaMemsetAsync(L.fpd.p, 0, sizeof(fp), ctx->stream);
+    a.fingerprint = L.fpd.p;
+    if (ce == cudaSuccess) ce = wl::launch_loopwarp(kprof, f.fermion != 0, f.nint, a, ctx->stream);
     if (ce == cudaSuccess)
       ce = cudaMemcpyAsync(&fp, L.fpd.p, sizeof(fp), cudaMemcpyDeviceToHost, ctx->stream);
-    if (ce == cudaSuccess) ce = wl::launch_loopwarp(kprof, f.fermion != 0, f.nint, a, ctx->stream);
     if (ce == cudaSuccess && params.Wsscal_h)
       ce = cudaMemcpyAsync(params.Wsscal_h, params.Wsscal_d, params.Nl * sizeof(float4),
                            cudaMemcpyDeviceToHost, ctx->stream);

@@ -515,7 +515,10 @@ constexpr int soft_rcp_period() {
 // b = z_i.(z_j - z_i), c = |z_j - z_i|^2, composite Simpson with NINT
 // intervals.  Adds xyyx * sum_w(f/rho^2) to ph and sum_w(f') to sp; the
 // Simpson factor h/3 and the f' scale are applied once per loop.
-template <int P, bool FERM, int NINT>
+// SQ (smooth profile, run-time interval count): f' = g^2 enters the sums as the
+// compiler contracts it, rounded on its own, or fused.
+enum : int { kSqAny = 0, kSqRound = 1, kSqFuse = 2 };
+template <int P, bool FERM, int NINT, int SQ = kSqAny>
 __device__ __forceinline__ void segment(float zix, float ziy, float zjx, float zjy,
                                         const FieldDev &F, float &ph, float &sp) {
   static_assert(NINT == 0 || (NINT % 2 == 0 && NINT >= 2), "Simpson needs an even interval count");
@@ -541,6 +544,10 @@ __device__ __forceinline__ void segment(float zix, float ziy, float zjx, float z
   Profile<P>::eval(ae, F, g1, f1);
   float so = 0.0f, se = 0.0f, fo = 0.0f, fe = 0.0f;
   constexpr int kSoftRcp = soft_rcp_period<P, FERM, NINT>();
+  constexpr bool kSq = smooth_profile(P) && NINT == 0 && SQ != kSqAny;
+  auto square = [](float g, float sum) {
+    return SQ == kSqRound ? __fadd_rn(sum, __fmul_rn(g, g)) : fmaf(g, g, sum);
+  };
   auto node = [&](int j, float t) {
     float r2 = fmaf(fmaf(c, t, b2), t, as);
     if (kFloor) r2 = fmaxf(r2, F.clampI);
@@ -553,10 +560,10 @@ __device__ __forceinline__ void segment(float zix, float ziy, float zjx, float z
     }
     if (j & 1) {
       so += g;
-      if (FERM) fo += fp;
+      if (FERM) fo = kSq ? square(g, fo) : fo + fp;
     } else {
       se += g;
-      if (FERM) fe += fp;
+      if (FERM) fe = kSq ? square(g, fe) : fe + fp;
     }
   };
   if constexpr (NINT > 0) {
@@ -941,7 +948,7 @@ __device__ __noinline__ float2 segment_lattice(float zix, float ziy, float zjx, 
 }
 
 // the segment of profile P (the image range is used by the lattice only)
-template <int P, bool FERM, int NINT>
+template <int P, bool FERM, int NINT, int SQ = kSqAny>
 __device__ __forceinline__ void seg(float zix, float ziy, float zjx, float zjy,
                                     const FieldDev &F, const ImgRange &img, float &ph,
                                     float &sp) {
@@ -955,7 +962,7 @@ __device__ __forceinline__ void seg(float zix, float ziy, float zjx, float zjy,
     ph = r.x;
     sp = r.y;
   } else {
-    segment<P, FERM, NINT>(zix, ziy, zjx, zjy, F, ph, sp);
+    segment<P, FERM, NINT, SQ>(zix, ziy, zjx, zjy, F, ph, sp);
   }
 }
 
@@ -1101,6 +1108,21 @@ __device__ __forceinline__ void loop_epilogue(const df G[3], const df H[3], cons
       add(j, w0, w1, w2);
     }
   }
+}
+
+// content hash of one point (x, y) at index p of the ensemble: the splitmix64
+// finaliser (Steele, Lea and Flood, "Fast splittable pseudorandom number
+// generators", OOPSLA 2014) of its coordinate bits combined with its index; an
+// ensemble's fingerprint is the sum over its points modulo 2^64
+__device__ __forceinline__ unsigned long long point_hash(float2 v, size_t p) {
+  auto mix = [](unsigned long long z) {
+    z = (z ^ (z >> 30)) * 0xbf58476d1ce4e5b9ull;
+    z = (z ^ (z >> 27)) * 0x94d049bb133111ebull;
+    return z ^ (z >> 31);
+  };
+  const unsigned long long bits = (unsigned long long)__float_as_uint(v.x) |
+                                  ((unsigned long long)__float_as_uint(v.y) << 32);
+  return mix(bits ^ mix(p + 0x9e3779b97f4a7c15ull));
 }
 
 // ------------------------------------------ bulk copy + mbarrier (PTX) --

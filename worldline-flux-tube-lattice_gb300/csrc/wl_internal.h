@@ -186,6 +186,10 @@ struct LoopArgs {
   float4 *scal;     // optional [ninst][Nl] Wsscal of F[0]
   float4 *ferm;     // optional [ninst][Nl] Wsferm of F[0]
   const float4 *bbox;  // lattice: [Nl] unit-loop bounding boxes
+  // optional (one instance): the ensemble's fingerprint (point_hash, zeroed by
+  // the caller), from the very points the sweep reads
+  unsigned long long *fingerprint;
+  int split;  // two warps per (loop, instance)
 };
 
 // plain per-instance kernel (the batching baseline), light profiles only

@@ -44,7 +44,11 @@ cudaError_t launch_sweep(int profile, bool fermion, int nint, const SweepArgs &a
 
 cudaError_t launch_loopwarp(int profile, bool fermion, int nint, const LoopArgs &a,
                             cudaStream_t s) {
-  return dispatch(profile, fermion, nint, nullptr, &a, s);
+  LoopArgs b = a;
+  // two warps per (loop, instance) up to four waves of resident warps: 2 to 45 %
+  // faster below (the more, the fewer), even above
+  b.split = (long long)a.Nl * a.ninst <= 4 * kSweepSlots;
+  return dispatch(profile, fermion, nint, nullptr, &b, s);
 }
 
 // ---------------------------------------------------------- reductions --
@@ -228,29 +232,16 @@ __global__ void loop_bbox_kernel(const float4 *__restrict__ loops, int Nl, int p
 }
 
 // ------------------------------------------------------- fingerprint --
-// Content fingerprint of an ensemble's (x, y) coordinates: the sum modulo
-// 2^64 of the splitmix64 finaliser (Steele, Lea and Flood, "Fast splittable
-// pseudorandom number generators", OOPSLA 2014) applied to each point's
-// coordinate bits combined with its index.  Any change of a coordinate
-// changes the sum except with probability ~2^-64; the sum does not depend on
-// the order in which the points are added.
-__device__ __forceinline__ unsigned long long mix64(unsigned long long z) {
-  z = (z ^ (z >> 30)) * 0xbf58476d1ce4e5b9ull;
-  z = (z ^ (z >> 27)) * 0x94d049bb133111ebull;
-  return z ^ (z >> 31);
-}
-
+// Content fingerprint of an ensemble's (x, y) coordinates (point_hash).  Any
+// change of a coordinate changes the sum except with probability ~2^-64; the
+// sum does not depend on the order in which the points are added.
 __global__ void __launch_bounds__(256)
     fingerprint_kernel(const float2 *__restrict__ pts, size_t npts,
                        unsigned long long *__restrict__ out) {
   unsigned long long acc = 0;
   const size_t stride = (size_t)gridDim.x * blockDim.x;
   for (size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x; p < npts; p += stride) {
-    const float2 v = pts[2 * p];  // (x, y) of the float4 point p
-    const unsigned long long bits =
-        (unsigned long long)__float_as_uint(v.x) |
-        ((unsigned long long)__float_as_uint(v.y) << 32);
-    acc += mix64(bits ^ mix64(p + 0x9e3779b97f4a7c15ull));
+    acc += point_hash(pts[2 * p], p);  // (x, y) of the float4 point p
   }
   for (int off = 16; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
   if ((threadIdx.x & 31) == 0) atomicAdd(out, acc);

@@ -824,41 +824,69 @@ __global__ void __launch_bounds__(kSweepThreads, 4)
     warp_unit<P, FERM, NINT, PAIR>(A, tile, l0, l1, row, W);
 }
 
+// One warp per (loop, instance), or (A.split) two: the N/2 sub-loop's segments
+// on one, both N/4 sub-loops' on the other -- the same work each, and the same
+// sums, since the sub-loops' accumulators are separate.  Bound by latency when
+// few (loop, instance) pairs leave the SMs with a few warps each: one instance
+// on 512 loops of 512 points, fixflux at 50 intervals, 1.06 -> 0.59 ms with two.
+//   With A.fingerprint the warps also hash the points they read: EV() checks a
+// cached ensemble against that, and a pass of its own over the ensemble took
+// 20 us beside the 60 us of the sweep (5120 loops of 1024 points, 50
+// intervals); 79 such EV() sweeps of integrateT 10.8 -> 9.9 ms.
+//   (kSqRound / kSqFuse: the roundings the four calls were compiled to, written
+// out so that results keep their bits.)
 template <int P, bool FERM, int NINT>
 __global__ void __launch_bounds__(kLoopWarps * 32)
     loopwarp_kernel(const __grid_constant__ LoopArgs A) {
-  const int lane = threadIdx.x & 31;
-  const int l = blockIdx.x * kLoopWarps + (threadIdx.x >> 5);
+  __shared__ float quarter[kLoopWarps][4];  // split: sums of the N/4 sub-loops
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int l = A.split ? blockIdx.x * (kLoopWarps / 2) + (w >> 1) : blockIdx.x * kLoopWarps + w;
+  const bool half = !A.split || !(w & 1), quarters = !A.split || (w & 1);
   const int inst = blockIdx.y;
-  if (l >= A.Nl) return;  // whole warp
+  const bool on = l < A.Nl;  // whole warp
+  if (!A.split && !on) return;
   const float cx = A.cx[inst], cy = A.cy[inst], s = A.rtT[inst];
   const FieldDev &F = A.field;
-  const float2 *w = reinterpret_cast<const float2 *>(A.loops + (size_t)l * A.ppl);
+  const float2 *pts = reinterpret_cast<const float2 *>(A.loops + (size_t)(on ? l : 0) * A.ppl);
   auto pt = [&](int p, float &x, float &y) {
-    const float2 v = __ldg(&w[2 * p]);
+    const float2 v = __ldg(&pts[2 * p]);
     x = fmaf(s, v.x, cx);
     y = fmaf(s, v.y, cy);
+    return v;
   };
   // group q covers points 4q..4q+3 and the four segments ending there; the
   // previous points of group 0 wrap to the end of the loop (closing segments)
-  const int nq = A.ppl >> 2;
+  const int nq = on ? A.ppl >> 2 : 0;
   ImgRange img = {0, -1, 0, -1, 1};
-  if constexpr (P == kLattice) img = image_range(A.bbox[l], s, cx, cy, F);
+  if constexpr (P == kLattice)
+    if (on) img = image_range(A.bbox[l], s, cx, cy, F);
   float ph[3] = {0.f, 0.f, 0.f}, sp[3] = {0.f, 0.f, 0.f};
+  unsigned long long hash = 0;
   for (int q = lane; q < nq; q += 32) {
     const int pa = (q == 0 ? A.ppl : 4 * q) - 4;
-    float zAx, zAy, zBx, zBy, zOx, zOy, P0x, P0y, P1x, P1y, P2x, P2y, P3x, P3y;
-    pt(pa, zAx, zAy);
-    pt(pa + 2, zBx, zBy);
-    pt(pa + 3, zOx, zOy);
-    pt(4 * q, P0x, P0y);
-    pt(4 * q + 1, P1x, P1y);
-    pt(4 * q + 2, P2x, P2y);
-    pt(4 * q + 3, P3x, P3y);
-    seg<P, FERM, NINT>(zAx, zAy, P0x, P0y, F, img, ph[2], sp[2]);
-    seg<P, FERM, NINT>(zOx, zOy, P1x, P1y, F, img, ph[0], sp[0]);
-    seg<P, FERM, NINT>(zBx, zBy, P2x, P2y, F, img, ph[1], sp[1]);
-    seg<P, FERM, NINT>(P1x, P1y, P3x, P3y, F, img, ph[0], sp[0]);
+    float2 v[4];
+    if (half) {
+      float zOx, zOy, P1x, P1y, P3x, P3y;
+      pt(pa + 3, zOx, zOy);
+      v[1] = pt(4 * q + 1, P1x, P1y);
+      v[3] = pt(4 * q + 3, P3x, P3y);
+      seg<P, FERM, NINT, kSqRound>(zOx, zOy, P1x, P1y, F, img, ph[0], sp[0]);
+      seg<P, FERM, NINT, kSqRound>(P1x, P1y, P3x, P3y, F, img, ph[0], sp[0]);
+    }
+    if (quarters) {
+      float zAx, zAy, zBx, zBy, P0x, P0y, P2x, P2y;
+      pt(pa, zAx, zAy);
+      pt(pa + 2, zBx, zBy);
+      v[0] = pt(4 * q, P0x, P0y);
+      v[2] = pt(4 * q + 2, P2x, P2y);
+      seg<P, FERM, NINT, kSqFuse>(zAx, zAy, P0x, P0y, F, img, ph[2], sp[2]);
+      seg<P, FERM, NINT, kSqRound>(zBx, zBy, P2x, P2y, F, img, ph[1], sp[1]);
+    }
+    if (A.fingerprint) {
+      const size_t p = (size_t)l * A.ppl + 4 * q;
+      if (half) hash += point_hash(v[1], p + 1) + point_hash(v[3], p + 3);
+      if (quarters) hash += point_hash(v[0], p) + point_hash(v[2], p + 2);
+    }
   }
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) {
@@ -868,7 +896,26 @@ __global__ void __launch_bounds__(kLoopWarps * 32)
       if (FERM) sp[r] += __shfl_xor_sync(0xffffffffu, sp[r], off);
     }
   }
-  if (lane == 0) {
+  if (A.fingerprint) {
+    for (int off = 16; off > 0; off >>= 1) hash += __shfl_xor_sync(0xffffffffu, hash, off);
+    if (lane == 0 && on) atomicAdd(A.fingerprint, hash);
+  }
+  if (A.split) {
+    if (lane == 0 && quarters) {
+      quarter[w][0] = ph[1];
+      quarter[w][1] = ph[2];
+      quarter[w][2] = sp[1];
+      quarter[w][3] = sp[2];
+    }
+    __syncthreads();
+    if (lane == 0 && half) {
+      ph[1] = quarter[w + 1][0];
+      ph[2] = quarter[w + 1][1];
+      sp[1] = quarter[w + 1][2];
+      sp[2] = quarter[w + 1][3];
+    }
+  }
+  if (lane == 0 && half && on) {
     const df tq = {A.tqh[inst], A.tql[inst]};
     const df G[3] = {df{ph[0], 0.f}, df{ph[1], 0.f}, df{ph[2], 0.f}};
     const df H[3] = {df{sp[0], 0.f}, df{sp[1], 0.f}, df{sp[2], 0.f}};
@@ -945,7 +992,8 @@ cudaError_t sweep_dispatch(bool fermion, int nint, const SweepArgs &a, cudaStrea
 
 template <int P>
 cudaError_t loopwarp_dispatch(bool fermion, int nint, const LoopArgs &a, cudaStream_t s) {
-  const dim3 grid((a.Nl + kLoopWarps - 1) / kLoopWarps, a.ninst);
+  const int per = a.split ? kLoopWarps / 2 : kLoopWarps;  // loops per CTA
+  const dim3 grid((a.Nl + per - 1) / per, a.ninst);
 #define WL_LOOP_CASE(FE, NI)                                                       \
   if (fermion == FE && (NI == 0 || nint == NI)) {                                  \
     loopwarp_kernel<P, FE, NI><<<grid, kLoopWarps * 32, 0, s>>>(a);                \
