@@ -11,6 +11,7 @@
 #include <string.h>
 
 #include <algorithm>
+#include <initializer_list>
 #include <map>
 #include <mutex>
 #include <string>
@@ -81,6 +82,8 @@ struct wl_ctx {
   double last_batch_ms = 0.0;
   int last_batch_tiles = 0, last_batch_grid = 0;
   std::vector<float> h_inst;
+  bool staged = false;        // h_inst may still be read by its copy
+  std::vector<double> h_out;  // small results on their way to the caller
   std::string err;
   int last_launches = 0;
   const char *last_kind = "none";
@@ -296,6 +299,8 @@ int upload_instances(wl_ctx *ctx, int ninst, const double *cx, const double *cy,
       return fail(ctx, WL_ERR_INVALID, "instance %d: need finite centre and T > 0", i);
   }
   const int na = wl::kInstArrays;
+  if (ctx->staged)  // a call that failed after staging left its copy unawaited
+    WL_CHECK(ctx, cudaStreamSynchronize(ctx->stream));
   ctx->h_inst.resize((size_t)na * ninst);
   float *h = ctx->h_inst.data();
   for (int i = 0; i < ninst; ++i) {
@@ -310,10 +315,11 @@ int upload_instances(wl_ctx *ctx, int ninst, const double *cx, const double *cy,
     h[4 * ninst + i] = (float)(tq - (double)(float)tq);
   }
   WL_CHECK(ctx, ctx->inst.reserve((size_t)na * ninst));
-  // the staging vector is pageable and reused: copy synchronously
+  // the launches that follow need no wait; the call's results are awaited before
+  // the vector is refilled
+  ctx->staged = true;
   WL_CHECK(ctx, cudaMemcpyAsync(ctx->inst.p, h, sizeof(float) * na * ninst,
                                 cudaMemcpyHostToDevice, ctx->stream));
-  WL_CHECK(ctx, cudaStreamSynchronize(ctx->stream));
   return WL_OK;
 }
 
@@ -327,16 +333,59 @@ int plan_chunk(int group) {
   return lc;
 }
 
-int check_status(wl_ctx *ctx) {
-  int st = 0;
-  WL_CHECK(ctx, cudaMemcpyAsync(&st, ctx->status.p, sizeof(int), cudaMemcpyDeviceToHost,
-                                ctx->stream));
-  WL_CHECK(ctx, cudaStreamSynchronize(ctx->stream));
+// after the stream has been waited for
+int status_error(wl_ctx *ctx, int st) {
+  ctx->staged = false;
   if (st == wl::kDevTimeout)
     return fail(ctx, WL_ERR_TIMEOUT, "a shared-memory stage copy timed out on the device");
   if (st == wl::kDevBadInstance)
     return fail(ctx, WL_ERR_INVALID, "an instance has T <= 0 or a non-finite value");
   return WL_OK;
+}
+
+int check_status(wl_ctx *ctx) {
+  int st = 0;
+  WL_CHECK(ctx, cudaMemcpyAsync(&st, ctx->status.p, sizeof(int), cudaMemcpyDeviceToHost,
+                                ctx->stream));
+  WL_CHECK(ctx, cudaStreamSynchronize(ctx->stream));
+  return status_error(ctx, st);
+}
+
+// Results of a blocking call: n doubles at dev, cut into consecutive parts for
+// the caller's arrays (a NULL one is skipped), and the launch's status behind
+// them (dev[n], written by the last kernel).  Small results come back in one
+// copy -- every copy to pageable memory waits for the device, 10 us a time --
+// large ones straight into the caller's arrays.
+struct OutPart {
+  double *host;
+  size_t n;
+};
+int read_results(wl_ctx *ctx, const double *dev, size_t n, std::initializer_list<OutPart> parts) {
+  constexpr size_t kOneCopy = 32768;  // 256 KiB
+  double st = 0.0;
+  size_t at = 0;
+  if (n <= kOneCopy) {
+    ctx->h_out.resize(n + 1);
+    WL_CHECK(ctx, cudaMemcpyAsync(ctx->h_out.data(), dev, sizeof(double) * (n + 1),
+                                  cudaMemcpyDeviceToHost, ctx->stream));
+    WL_CHECK(ctx, cudaStreamSynchronize(ctx->stream));
+    for (const OutPart &p : parts) {
+      if (p.host) memcpy(p.host, ctx->h_out.data() + at, sizeof(double) * p.n);
+      at += p.n;
+    }
+    st = ctx->h_out[n];
+  } else {
+    for (const OutPart &p : parts) {
+      if (p.host)
+        WL_CHECK(ctx, cudaMemcpyAsync(p.host, dev + at, sizeof(double) * p.n,
+                                      cudaMemcpyDeviceToHost, ctx->stream));
+      at += p.n;
+    }
+    WL_CHECK(ctx, cudaMemcpyAsync(&st, dev + n, sizeof(double), cudaMemcpyDeviceToHost,
+                                  ctx->stream));
+    WL_CHECK(ctx, cudaStreamSynchronize(ctx->stream));
+  }
+  return status_error(ctx, (int)st);
 }
 
 }  // namespace
@@ -901,7 +950,8 @@ static int eval_prologue(wl_ctx *ctx, int handle, const wl_field *field, int nin
 // NULL).  Returns after enqueueing.
 static int run_eval(wl_ctx *ctx, const Ensemble &e, int kprof, const FieldDev &fd,
                     const float4 *bbox, const wl_field *field, int ninst, int nF,
-                    const double *host_F, int group, double *dg, double *dm, double *ds) {
+                    const double *host_F, int group, double *dg, double *dm, double *ds,
+                    double *status_out) {
   const bool fermion = field->fermion != 0;
   const int nint = field->nint;
   const bool use_sweep = ninst >= 32;
@@ -986,7 +1036,8 @@ static int run_eval(wl_ctx *ctx, const Ensemble &e, int kprof, const FieldDev &f
     ctx->last_kind = "loop-parallel";
   }
   const wl::ReduceShape rs = {ctx->partial.p, n_chunks, cpg, inner, group, ninst, nF};
-  WL_CHECK(ctx, wl::launch_group_reduce(rs, dg, dm, ds, ctx->stream));
+  WL_CHECK(ctx, wl::launch_group_reduce(rs, dg, dm, ds, status_out ? ctx->status.p : nullptr,
+                                        status_out, ctx->stream));
   return WL_OK;
 }
 
@@ -1004,26 +1055,19 @@ int wl_eval(wl_ctx *ctx, int handle, const wl_field *field, int ninst, const dou
   WL_CHECK(ctx, cudaMemsetAsync(ctx->status.p, 0, sizeof(int), ctx->stream));
   const int ng = e.Nl / group;
   const size_t nout = (size_t)ninst * nF * (ng + 2);
-  if (ctx->out.reserve(nout) != cudaSuccess) {
+  if (ctx->out.reserve(nout + 1) != cudaSuccess) {
     cudaGetLastError();
     return fail(ctx, WL_ERR_NOMEM, "cannot allocate %zu outputs", nout);
   }
   double *dg = ctx->out.p, *dm = dg + (size_t)ninst * nF * ng, *ds = dm + (size_t)ninst * nF;
   const float4 *bb = nullptr;
   if (kprof == wl::kLattice && (r = ensure_bbox(ctx, handle, &bb))) return r;
-  if ((r = run_eval(ctx, e, kprof, fd, bb, field, ninst, nF, host_F, group, dg, dm, ds)))
+  if ((r = run_eval(ctx, e, kprof, fd, bb, field, ninst, nF, host_F, group, dg, dm, ds,
+                    dg + nout)))
     return r;
   ctx->last_launches = 2;
-  if (out_group)
-    WL_CHECK(ctx, cudaMemcpyAsync(out_group, dg, sizeof(double) * ninst * nF * ng,
-                                  cudaMemcpyDeviceToHost, ctx->stream));
-  if (out_mean)
-    WL_CHECK(ctx, cudaMemcpyAsync(out_mean, dm, sizeof(double) * ninst * nF,
-                                  cudaMemcpyDeviceToHost, ctx->stream));
-  if (out_sem)
-    WL_CHECK(ctx, cudaMemcpyAsync(out_sem, ds, sizeof(double) * ninst * nF,
-                                  cudaMemcpyDeviceToHost, ctx->stream));
-  return check_status(ctx);
+  const size_t nm = (size_t)ninst * nF;
+  return read_results(ctx, dg, nout, {{out_group, nm * ng}, {out_mean, nm}, {out_sem, nm}});
 }
 
 int wl_eval_device(wl_ctx *ctx, int handle, const wl_field *field, int ninst,
@@ -1055,7 +1099,7 @@ int wl_eval_device(wl_ctx *ctx, int handle, const wl_field *field, int ninst,
   const float4 *bb = nullptr;
   if (kprof == wl::kLattice && (r = ensure_bbox(ctx, handle, &bb))) return r;
   if ((r = run_eval(ctx, e, kprof, fd, bb, field, ninst, nF, host_F, group, dev_out_group,
-                    dev_out_mean, dev_out_sem)))
+                    dev_out_mean, dev_out_sem, nullptr)))
     return r;
   ctx->last_launches = 3;
   return WL_OK;
@@ -1218,12 +1262,12 @@ static int tint_run(wl_ctx *ctx, int handle, const wl_field *field, int nrho,
   const float4 *bb = nullptr;
   if (kprof == wl::kLattice && (r = ensure_bbox(ctx, handle, &bb))) return r;
   if ((r = run_eval(ctx, e, kprof, fd, bb, field, ninst, nF, host_F, group, dg, nullptr,
-                    nullptr)))
+                    nullptr, nullptr)))
     return r;
-  // aux: rho | T | w | F | Ig | leff | err | igrand
+  // aux: rho | T | w | F | Ig | leff | err | status | igrand
   const size_t n_ig = (size_t)nrho * nF * ng, n_le = (size_t)nrho * nF;
   const size_t n_igr = want_igrand ? (size_t)nrho * nF * nT * ng : 0;
-  const size_t naux = (size_t)nrho + 2 * (size_t)nT + nF + n_ig + 2 * n_le + n_igr;
+  const size_t naux = (size_t)nrho + 2 * (size_t)nT + nF + n_ig + 2 * n_le + 1 + n_igr;
   if (ctx->aux.reserve(naux) != cudaSuccess) {
     cudaGetLastError();
     return fail(ctx, WL_ERR_NOMEM, "cannot allocate the proper-time buffers");
@@ -1246,7 +1290,9 @@ static int tint_run(wl_ctx *ctx, int handle, const wl_field *field, int nrho,
   ta.Ig = d + nrho + 2 * nT + nF;
   ta.leff = ta.Ig + n_ig;
   ta.err = ta.leff + n_le;
-  ta.igrand = want_igrand ? ta.err + n_le : nullptr;
+  ta.status = ctx->status.p;
+  ta.status_out = ta.err + n_le;
+  ta.igrand = want_igrand ? ta.status_out + 1 : nullptr;
   ta.nrho = nrho;
   ta.nT = nT;
   ta.nF = nF;
@@ -1279,14 +1325,10 @@ int wl_tint(wl_ctx *ctx, int handle, const wl_field *field, int nrho, const doub
                     nbins, out_igrand != nullptr, &ta)))
     return r;
   const size_t n_le = (size_t)nrho * nF, n_igr = (size_t)nrho * nF * nT * ta.ng;
-  WL_CHECK(ctx, cudaMemcpyAsync(out_leff, ta.leff, sizeof(double) * n_le, cudaMemcpyDeviceToHost,
-                                ctx->stream));
-  WL_CHECK(ctx, cudaMemcpyAsync(out_err, ta.err, sizeof(double) * n_le, cudaMemcpyDeviceToHost,
-                                ctx->stream));
   if (out_igrand)
     WL_CHECK(ctx, cudaMemcpyAsync(out_igrand, ta.igrand, sizeof(double) * n_igr,
                                   cudaMemcpyDeviceToHost, ctx->stream));
-  return check_status(ctx);
+  return read_results(ctx, ta.leff, 2 * n_le, {{out_leff, n_le}, {out_err, n_le}});
 }
 
 // Classical action of the profile (EffAct.c:228-279), e = 0.30282212.
@@ -1507,7 +1549,7 @@ int wl_eval_plain(wl_ctx *ctx, int handle, const wl_field *field, int ninst, con
   WL_CHECK(ctx, cudaEventRecord(e1, ctx->stream));
   double *dg = ctx->out.p, *dm = dg + (size_t)ninst * nF * ng, *ds = dm + (size_t)ninst * nF;
   const wl::ReduceShape rs = {ctx->partial.p, e.Nl, group, 1, group, ninst, nF};
-  WL_CHECK(ctx, wl::launch_group_reduce(rs, dg, dm, ds, ctx->stream));
+  WL_CHECK(ctx, wl::launch_group_reduce(rs, dg, dm, ds, nullptr, nullptr, ctx->stream));
   WL_CHECK(ctx, cudaEventSynchronize(e1));
   float ms = 0.0f;
   cudaEventElapsedTime(&ms, e0, e1);
@@ -1725,32 +1767,33 @@ double EV(double T, void *p, int *WLlist) {
     a.partial = L.w.p;
     a.scal = params.Wsscal_d;
     a.ferm = f.fermion ? params.Wsferm_d : nullptr;
-    unsigned long long fp = 0;
-    cudaError_t ce = L.fpd.reserve(1);
-    if (ce == cudaSuccess) ce = cudaMemsetAsync(L.fpd.p, 0, sizeof(fp), ctx->stream);
-    a.fingerprint = L.fpd.p;
+    // the groups' means and, behind them, the fingerprint: one copy brings both
+    const int ngrp = params.Nl / groupsize;
+    if (L.gres.reserve((size_t)ngrp + 1) != cudaSuccess) {
+      cudaGetLastError();
+      return legacy_fail("out of memory");
+    }
+    static_assert(sizeof(unsigned long long) == sizeof(double), "one array holds both");
+    a.fingerprint = (unsigned long long *)(L.gres.p + ngrp);
+    cudaError_t ce = cudaMemsetAsync(a.fingerprint, 0, sizeof(double), ctx->stream);
     if (ce == cudaSuccess) ce = wl::launch_loopwarp(kprof, f.fermion != 0, f.nint, a, ctx->stream);
     if (ce == cudaSuccess)
-      ce = cudaMemcpyAsync(&fp, L.fpd.p, sizeof(fp), cudaMemcpyDeviceToHost, ctx->stream);
+      ce = wl::launch_group_list_means(L.w.p, groupsize, ngrp, L.gres.p, ctx->stream);
     if (ce == cudaSuccess && params.Wsscal_h)
       ce = cudaMemcpyAsync(params.Wsscal_h, params.Wsscal_d, params.Nl * sizeof(float4),
                            cudaMemcpyDeviceToHost, ctx->stream);
     if (ce == cudaSuccess && f.fermion && params.Wsferm_h)
       ce = cudaMemcpyAsync(params.Wsferm_h, params.Wsferm_d, params.Nl * sizeof(float4),
                            cudaMemcpyDeviceToHost, ctx->stream);
-    const int ngrp = params.Nl / groupsize;
-    L.gev.assign((size_t)ngrp, NAN);
-    if (ce == cudaSuccess && L.gres.reserve((size_t)ngrp) != cudaSuccess) {
-      cudaGetLastError();
-      return legacy_fail("out of memory");
-    }
+    L.gev.assign((size_t)ngrp + 1, NAN);
     if (ce == cudaSuccess)
-      ce = wl::launch_group_list_means(L.w.p, groupsize, ngrp, L.gres.p, ctx->stream);
-    if (ce == cudaSuccess)
-      ce = cudaMemcpyAsync(L.gev.data(), L.gres.p, sizeof(double) * ngrp,
+      ce = cudaMemcpyAsync(L.gev.data(), L.gres.p, sizeof(double) * (ngrp + 1),
                            cudaMemcpyDeviceToHost, ctx->stream);
     if (ce == cudaSuccess) ce = cudaStreamSynchronize(ctx->stream);
     if (ce != cudaSuccess) return legacy_fail(cudaGetErrorString(ce));
+    unsigned long long fp;
+    memcpy(&fp, &L.gev[(size_t)ngrp], sizeof(fp));
+    L.gev.resize((size_t)ngrp);
     L.T = T;
     L.F = params.F;
     L.l2 = params.l2;

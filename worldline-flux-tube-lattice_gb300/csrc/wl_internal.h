@@ -203,8 +203,10 @@ cudaError_t launch_loopwarp(int profile, bool fermion, int nint, const LoopArgs 
                             cudaStream_t s);
 
 // partial sums -> per-group <W>, mean and SEM over groups
+// (status_out, may be NULL: receives the status word as a double)
 cudaError_t launch_group_reduce(const ReduceShape &r, double *out_group, double *out_mean,
-                                double *out_sem, cudaStream_t s);
+                                double *out_sem, const int *status, double *status_out,
+                                cudaStream_t s);
 
 // EV(): mean over an index list of per-loop W factors (partial with
 // ninst = 1, nF = 1) and the Richardson combination; writes one double.
@@ -243,6 +245,9 @@ struct TintArgs {
   double *igrand;  // optional [nrho][nF][nT][ng]
   double *Ig;      // [nrho][nF][ng]
   double *leff, *err;  // [nrho][nF]
+  // optional: the launch's status word, copied as a double behind the results
+  const int *status;
+  double *status_out;
 };
 cudaError_t launch_tint(const TintArgs &a, cudaStream_t s);
 

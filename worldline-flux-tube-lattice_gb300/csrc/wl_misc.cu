@@ -55,7 +55,10 @@ cudaError_t launch_loopwarp(int profile, bool fermion, int nint, const LoopArgs 
 // <W> per group (Integrand.c:400), mean and standard error over the groups
 __global__ void __launch_bounds__(kReduceThreads)
     group_reduce_kernel(const ReduceShape R, int ti, double *__restrict__ out_group,
-                        double *__restrict__ out_mean, double *__restrict__ out_sem) {
+                        double *__restrict__ out_mean, double *__restrict__ out_sem,
+                        const int *status, double *status_out) {
+  if (status_out && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0)
+    *status_out = (double)*status;
   reduce_block(R, blockIdx.x * ti, blockIdx.y, ti, out_group,
                [&](size_t at, double mean, double sem) {
                  if (out_mean) out_mean[at] = mean;
@@ -126,10 +129,12 @@ cudaError_t launch_order_instances(const float *cx, const float *cy, const float
 }
 
 cudaError_t launch_group_reduce(const ReduceShape &r, double *out_group, double *out_mean,
-                                double *out_sem, cudaStream_t s) {
+                                double *out_sem, const int *status, double *status_out,
+                                cudaStream_t s) {
   const int ti = reduce_instances(r.ninst, r.nF, r.n_chunks / r.cpg);
   const dim3 grid((r.ninst + ti - 1) / ti, r.nF);
-  group_reduce_kernel<<<grid, kReduceThreads, 0, s>>>(r, ti, out_group, out_mean, out_sem);
+  group_reduce_kernel<<<grid, kReduceThreads, 0, s>>>(r, ti, out_group, out_mean, out_sem,
+                                                       status, status_out);
   return cudaGetLastError();
 }
 

@@ -204,7 +204,7 @@ extern "C" int wl_eval_noalloc(const float *dev_loops, int Nl, int ppl, const wl
   }
   if (ce == cudaSuccess)
     ce = wl::launch_group_reduce({partial, n_chunks, cpg, inner, group, ninst, nF}, dev_out_group,
-                                 dev_out_mean, dev_out_sem, s);
+                                 dev_out_mean, dev_out_sem, nullptr, nullptr, s);
   int st = 0;
   if (ce == cudaSuccess) ce = cudaMemcpyAsync(&st, status, sizeof(int), cudaMemcpyDeviceToHost, s);
   if (ce == cudaSuccess) ce = cudaStreamSynchronize(s);

@@ -142,6 +142,7 @@ __global__ void tint_kernel(const TintArgs A) {
 // one thread per (rho, F): L_eff and its jackknife error over nbins bins
 __global__ void jackknife_kernel(const TintArgs A) {
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
+  if (idx == 0 && A.status_out) *A.status_out = (double)*A.status;
   if (idx >= A.nrho * A.nF) return;
   const double *I = A.Ig + (size_t)idx * A.ng;
   const int nb = A.nbins, per = A.ng / nb;
