@@ -1308,7 +1308,7 @@ static int tint_run(wl_ctx *ctx, int handle, const wl_field *field, int nrho,
   ta.m2 = 1.0;         // Integrand.c:12
   ta.e = 0.30282212;   // Integrand.c:14
   WL_CHECK(ctx, wl::launch_tint(ta, ctx->stream));
-  ctx->last_launches = 4;
+  ctx->last_launches = 3;  // sweep, reduction, proper-time integral
   return WL_OK;
 }
 

@@ -78,8 +78,13 @@ __device__ double magfield_d(const TintArgs &A, double rho2, double F) {
   return 2.0 * F / A.e * B;
 }
 
-// Tfunc's integrand for one group (Integrand.c:215-305)
-__device__ double igrand_d(TintArgs A, double rho, double T, double F, double W) {
+// Tfunc's integrand at (rho, T, F) (Integrand.c:215-305), up to the group's
+// <W>: v = pre (<W> - 1 -+ shift) where mc, else the constant v.
+struct TNode {
+  double pre, shift, v, w;  // w: the quadrature weight
+  int mc;
+};
+__device__ TNode igrand_d(TintArgs A, double rho, double T, double F) {
   const double rho2 = rho * rho, l2 = A.l2, m2 = A.m2, e = A.e;
   A.xcm_x = rho;
   const double B = magfield_d(A, rho2, F), TB = e * T * B;
@@ -99,52 +104,82 @@ __device__ double igrand_d(TintArgs A, double rho, double T, double F, double W)
       break;
     default: smallT = 0.5 * (l2 + rho2);
   }
-  const double pre = exp(-m2 * T) / (T * T * T);
+  TNode n;
+  n.mc = 0;
+  n.pre = exp(-m2 * T) / (T * T * T);
+  n.shift = TB * TB / (A.fermion ? 3.0 : 6.0);
+  n.v = 0.0;
   if (T < 0.1 && T < 0.01 * smallT) {  // small-T series (Integrand.c:142-172)
     const double B2 = e * e * B * B, B4 = B2 * B2, B6 = B2 * B4;
     const double T3 = T * T * T, T4 = T3 * T;
     if (A.fermion)
-      return B4 * T * (m2 * T - 1.0) / 45.0 + (2.0 * B6 / 945.0 - B4 * m2 * m2 / 90.0) * T3 +
-             (7.0 * B4 * m2 * m2 * m2 - 4.0 * B6 * m2) / 1890.0 * T4;
-    return 7.0 / 360.0 * B4 * T * (1.0 - m2 * T) + (147.0 * B4 * m2 * m2 - 31.0 * B6) / 15120.0 * T3 +
-           (31.0 * B6 * m2 - 49.0 * B4 * m2 * m2 * m2) / 15120.0 * T4;
+      n.v = B4 * T * (m2 * T - 1.0) / 45.0 + (2.0 * B6 / 945.0 - B4 * m2 * m2 / 90.0) * T3 +
+            (7.0 * B4 * m2 * m2 * m2 - 4.0 * B6 * m2) / 1890.0 * T4;
+    else
+      n.v = 7.0 / 360.0 * B4 * T * (1.0 - m2 * T) + (147.0 * B4 * m2 * m2 - 31.0 * B6) / 15120.0 * T3 +
+            (31.0 * B6 * m2 - 49.0 * B4 * m2 * m2 * m2) / 15120.0 * T4;
+  } else if (T < 0.01 * smallT) {  // constant field (Integrand.c:20-37)
+    if (!(TB > 1.0e-6) || B < 1.0e-40)
+      n.v = 0.0;
+    else if (A.fermion)
+      n.v = n.pre * (TB / tanh(TB) - 1.0 - TB * TB / 3.0);
+    else if (TB < 50.0)
+      n.v = n.pre * (TB / sinh(TB) - 1.0 + TB * TB / 6.0);
+    else
+      n.v = n.pre * (TB * TB / 6.0 - 1.0);
+  } else if (T > 49.0) {  // large T (Integrand.c:272-288)
+    n.v = A.fermion ? -exp(-m2 * T) / (3.0 * T) * e * e * B * B
+                    : exp(-m2 * T) / (6.0 * T) * e * e * B * B;
+  } else {
+    n.mc = 1;
   }
-  if (T < 0.01 * smallT) {  // constant field (Integrand.c:20-37)
-    if (!(TB > 1.0e-6) || B < 1.0e-40) return 0.0;
-    if (A.fermion) return pre * (TB / tanh(TB) - 1.0 - TB * TB / 3.0);
-    if (TB < 50.0) return pre * (TB / sinh(TB) - 1.0 + TB * TB / 6.0);
-    return pre * (TB * TB / 6.0 - 1.0);
-  }
-  if (T > 49.0)  // large T (Integrand.c:272-288)
-    return A.fermion ? -exp(-m2 * T) / (3.0 * T) * e * e * B * B
-                     : exp(-m2 * T) / (6.0 * T) * e * e * B * B;
-  return A.fermion ? pre * (W - 1.0 - TB * TB / 3.0) : pre * (W - 1.0 + TB * TB / 6.0);
+  if (isinf(n.v)) n.v = 0.0;  // Tint.c:132-149
+  return n;
 }
 
-// one thread per (rho, F, group): the T integral
-__global__ void tint_kernel(const TintArgs A) {
-  const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= A.nrho * A.nF * A.ng) return;
-  const int g = idx % A.ng, j = (idx / A.ng) % A.nF, r = idx / (A.ng * A.nF);
+// One CTA per (rho, F): the field and the regime of every proper time once,
+// one thread per T (they do not depend on the group), then one thread per group
+// for its T integral, and one for L_eff and its jackknife error over nbins bins.
+// Bound by FP64 latency: one thread per (rho, F, group) evaluated every T's
+// exponentials for itself, 395 us for 64 rho x 3 F x 40 groups x 128 T and 214
+// us for 40 rho x 40 groups x 79 T, with a jackknife launch of 20-28 us behind;
+// L_eff of 20 rho x 40 T on 1280 x 256 points 794 -> 481 us with the faster
+// sweep, the lattice (441 images per field value) 16.4 -> 5.5 ms.
+constexpr int kTintThreads = 128;
+__global__ void __launch_bounds__(kTintThreads) tint_kernel(const TintArgs A) {
+  __shared__ TNode node[kTintThreads];
+  const int idx = blockIdx.x, t = threadIdx.x;
+  const int j = idx % A.nF, r = idx / A.nF;
   const double rho = A.rho[r], F = A.F[j];
-  double s = 0.0;
-  for (int k = 0; k < A.nT; ++k) {
-    const int inst = r * A.nT + k;
-    const double W = A.groups[((size_t)inst * A.nF + j) * A.ng + g];
-    double v = igrand_d(A, rho, A.T[k], F, W);
-    if (isinf(v)) v = 0.0;  // Tint.c:132-149
-    if (A.igrand) A.igrand[(((size_t)r * A.nF + j) * A.nT + k) * A.ng + g] = v;
-    s += A.w[k] * v;
+  double *const I = A.Ig + (size_t)idx * A.ng;
+  if (idx == 0 && t == 0 && A.status_out) *A.status_out = (double)*A.status;
+  for (int k0 = 0; k0 < A.nT; k0 += kTintThreads) {
+    const int nk = min(kTintThreads, A.nT - k0);
+    __syncthreads();  // the nodes of the round before have been read
+    if (t < nk) {
+      node[t] = igrand_d(A, rho, A.T[k0 + t], F);
+      node[t].w = A.w[k0 + t];
+    }
+    __syncthreads();
+    for (int g = t; g < A.ng; g += kTintThreads) {
+      double s = k0 ? I[g] : 0.0;
+#pragma unroll 4
+      for (int k = 0; k < nk; ++k) {
+        const TNode n = node[k];
+        double v = n.v;
+        if (n.mc) {
+          const double W = A.groups[((size_t)(r * A.nT + k0 + k) * A.nF + j) * A.ng + g];
+          v = A.fermion ? n.pre * (W - 1.0 - n.shift) : n.pre * (W - 1.0 + n.shift);
+          if (isinf(v)) v = 0.0;  // Tint.c:132-149
+        }
+        if (A.igrand) A.igrand[((size_t)idx * A.nT + k0 + k) * A.ng + g] = v;
+        s += n.w * v;
+      }
+      I[g] = s;
+    }
   }
-  A.Ig[((size_t)r * A.nF + j) * A.ng + g] = s;
-}
-
-// one thread per (rho, F): L_eff and its jackknife error over nbins bins
-__global__ void jackknife_kernel(const TintArgs A) {
-  const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx == 0 && A.status_out) *A.status_out = (double)*A.status;
-  if (idx >= A.nrho * A.nF) return;
-  const double *I = A.Ig + (size_t)idx * A.ng;
+  __syncthreads();
+  if (t) return;
   const int nb = A.nbins, per = A.ng / nb;
   double tot = 0.0;
   for (int g = 0; g < nb * per; ++g) tot += I[g];
@@ -164,12 +199,7 @@ __global__ void jackknife_kernel(const TintArgs A) {
 }
 
 cudaError_t launch_tint(const TintArgs &a, cudaStream_t s) {
-  const int bs = 128;
-  const int n1 = a.nrho * a.nF * a.ng, n2 = a.nrho * a.nF;
-  tint_kernel<<<(n1 + bs - 1) / bs, bs, 0, s>>>(a);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  jackknife_kernel<<<(n2 + bs - 1) / bs, bs, 0, s>>>(a);
+  tint_kernel<<<a.nrho * a.nF, kTintThreads, 0, s>>>(a);
   return cudaGetLastError();
 }
 
