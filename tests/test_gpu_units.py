@@ -62,6 +62,25 @@ def test_single_loops_and_whole_chunks_agree_bit_for_bit(prof, fe, nint, n):
     assert torch.isfinite(out[0]).all() and torch.equal(out[0], out[1])
 
 
+@pytest.mark.parametrize("ppl", [4, 8, 36, 256, 260, 288, 1028])
+@pytest.mark.parametrize("prof,fe,ffv", [("periodic", 0, 0), ("periodic", 1, 0),
+                                         ("spline", 1, 0), ("fixflux", 1, 0),
+                                         ("fixflux", 0, 1)])
+def test_heavy_profiles_cut_at_their_blocks(prof, fe, ffv, ppl):
+    """wl_eval cuts these loops at their Kahan blocks (few units); among many
+    loops (two tiles of 2512) it walks them whole: the same bits."""
+    import wltube
+
+    fld = wltube.field(prof, fermion=fe, nint=4, lambda2=0.5, tubedist=1.0, ff_variant=ffv)
+    few = O.vloops(43, 9, ppl)
+    many = np.concatenate([few, O.vloops(44, 2503, ppl)])
+    cx, cy, T = instances(40, ppl)
+    with wltube.Context(0) as ctx:
+        g, _, _ = ctx.eval(ctx.upload(few), fld, cx, cy, T, [0.7], 1)
+        w, _, _ = ctx.eval(ctx.upload(many), fld, cx, cy, T, [0.7], 1)
+    assert np.isfinite(g).all() and np.array_equal(g, w[:, :, :9])
+
+
 def test_a_job_beside_a_large_one_equals_it_alone():
     """Alone the batch stores single loops, beside a job of 40960 units whole
     chunks."""

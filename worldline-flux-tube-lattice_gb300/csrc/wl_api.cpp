@@ -66,6 +66,7 @@ struct wl_ctx {
   int next_handle = 1;
   DevBuf<float> inst;       // cx, cy, rtT, tq  (4 * ninst)
   DevBuf<double> partial;   // sweep partial sums
+  DevBuf<float> blocks;     // heavy profiles' block sums (SweepArgs::parts)
   DevBuf<double> out;       // group values, means, SEMs
   DevBuf<int> status;       // device status word
   DevBuf<int> list;         // EV() loop list
@@ -778,6 +779,7 @@ int wl_ctx_destroy(wl_ctx *ctx) {
   }
   ctx->inst.release();
   ctx->partial.release();
+  ctx->blocks.release();
   ctx->out.release();
   ctx->status.release();
   ctx->list.release();
@@ -982,6 +984,12 @@ static int run_eval(wl_ctx *ctx, const Ensemble &e, int kprof, const FieldDev &f
       cudaGetLastError();
       wl::sweep_units(a, kprof, fermion, nint, wl::kNoSplit);
     }
+    const size_t nbl = wl::sweep_parts(a, wl::heavy_profile(kprof));
+    if (nbl && ctx->blocks.reserve(nbl) != cudaSuccess) {
+      cudaGetLastError();
+      a.parts = 0;
+    }
+    a.blocks = ctx->blocks.p;
   }
   const int inner = a.per_loop ? a.chunk_loops : 1;
   const size_t npart = (size_t)n_chunks * inner * nF * 3 * ninst;

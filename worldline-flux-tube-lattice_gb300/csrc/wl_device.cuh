@@ -193,11 +193,20 @@ template <>
 struct Profile<kPeriodic> {  // radial shells, intEV.cu:201-232 and 300-328
   static __device__ __forceinline__ void eval(float r2, const FieldDev &F, float &g,
                                               float &fp) {
+    float d;
+    eval_d(r2, F, g, d);
+    fp = factor(F) * d;
+  }
+  // f' = factor d
+  static __device__ __forceinline__ float factor(const FieldDev &F) {
+    return F.a / (2.0f * F.l2 * 0.69314718055994531f);
+  }
+  static __device__ __forceinline__ void eval_d(float r2, const FieldDev &F, float &g, float &d) {
     const float rho = sqrtf(r2), a = F.a, lam = F.lam;
     const float flraf = floorf(rho / a);
     const int i0 = (int)flraf - 2, i1 = (int)flraf + 2;
     float f = (i0 > 0) ? 0.5f * (flraf - 3.0f) * (flraf - 2.0f) : 0.0f;
-    float d = 0.0f;
+    d = 0.0f;
     // The shell at the axis (i = 0, when i0 <= 0 <= i1) comes first in the
     // loop's ascending order: it sets f and d, the shells i > 0 then add to
     // them.  Evaluated before the loop, its exp and log run once per warp
@@ -216,7 +225,6 @@ struct Profile<kPeriodic> {  // radial shells, intEV.cu:201-232 and 300-328
     }
     const float ln2 = 0.69314718055994531f;
     g = (a / (lam * ln2) * f + 1.0f) / r2;
-    fp = a / (2.0f * F.l2 * ln2) * d;
   }
   static __device__ __forceinline__ float fp_scale(const FieldDev &) { return 1.0f; }
   static constexpr bool kHeavy = true;
@@ -515,8 +523,9 @@ constexpr int soft_rcp_period() {
 // b = z_i.(z_j - z_i), c = |z_j - z_i|^2, composite Simpson with NINT
 // intervals.  Adds xyyx * sum_w(f/rho^2) to ph and sum_w(f') to sp; the
 // Simpson factor h/3 and the f' scale are applied once per loop.
-// SQ (smooth profile, run-time interval count): f' = g^2 enters the sums as the
-// compiler contracts it, rounded on its own, or fused.
+// SQ: how f' enters the sums -- as the compiler contracts it, or written out, so
+// that a segment gives the same bits wherever it is compiled: smooth at run-time
+// interval counts, g^2 rounded on its own or fused; periodic, factor x d rounded.
 enum : int { kSqAny = 0, kSqRound = 1, kSqFuse = 2 };
 template <int P, bool FERM, int NINT, int SQ = kSqAny>
 __device__ __forceinline__ void segment(float zix, float ziy, float zjx, float zjy,
@@ -539,9 +548,20 @@ __device__ __forceinline__ void segment(float zix, float ziy, float zjx, float z
   const float as = a + profile_shift<P>(F);
   float ae = (as + b2) + c;
   if (kFloor) ae = fmaxf(ae, F.clampE);
+  // periodic with SQ given: f holds d, its factor enters with the sums
+  constexpr bool kPer = P == kPeriodic && FERM && SQ != kSqAny;
+  float kf = 1.0f;
+  if constexpr (kPer) kf = Profile<P>::factor(F);
+  auto eval = [&](float r, float &g, float &f) {
+    if constexpr (kPer)
+      Profile<P>::eval_d(r, F, g, f);
+    else
+      Profile<P>::eval(r, F, g, f);
+  };
+  auto scaled = [&](float d, float sum) { return __fadd_rn(sum, __fmul_rn(kf, d)); };
   float g0, f0, g1, f1;
-  Profile<P>::eval(as, F, g0, f0);
-  Profile<P>::eval(ae, F, g1, f1);
+  eval(as, g0, f0);
+  eval(ae, g1, f1);
   float so = 0.0f, se = 0.0f, fo = 0.0f, fe = 0.0f;
   constexpr int kSoftRcp = soft_rcp_period<P, FERM, NINT>();
   constexpr bool kSq = smooth_profile(P) && NINT == 0 && SQ != kSqAny;
@@ -556,14 +576,14 @@ __device__ __forceinline__ void segment(float zix, float ziy, float zjx, float z
       g = rcp_newton(r2);
       fp = g * g;
     } else {
-      Profile<P>::eval(r2, F, g, fp);
+      eval(r2, g, fp);
     }
     if (j & 1) {
       so += g;
-      if (FERM) fo = kSq ? square(g, fo) : fo + fp;
+      if (FERM) fo = kSq ? square(g, fo) : kPer ? scaled(fp, fo) : fo + fp;
     } else {
       se += g;
-      if (FERM) fe = kSq ? square(g, fe) : fe + fp;
+      if (FERM) fe = kSq ? square(g, fe) : kPer ? scaled(fp, fe) : fe + fp;
     }
   };
   if constexpr (NINT > 0) {
@@ -577,7 +597,10 @@ __device__ __forceinline__ void segment(float zix, float ziy, float zjx, float z
   }
   const float S = fmaf(4.0f, so, fmaf(2.0f, se, g0 + g1));
   ph = fmaf(xyyx, S, ph);
-  if (FERM) sp += fmaf(4.0f, fo, fmaf(2.0f, fe, f0 + f1));
+  if (FERM) {
+    const float f01 = kPer ? fmaf(kf, f0, __fmul_rn(kf, f1)) : f0 + f1;
+    sp += fmaf(4.0f, fo, fmaf(2.0f, fe, f01));
+  }
 }
 
 // ------------------------------------------------ packed pairs (f32x2) --

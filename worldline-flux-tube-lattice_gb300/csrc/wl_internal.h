@@ -39,6 +39,10 @@ struct SweepArgs {
   int n_units;
   int per_loop;      // the partial sums are stored loop by loop
   int n_tiles;       // warps per unit (set at launch)
+  // heavy profiles with few units (sweep_parts): a loop's Kahan blocks go to
+  // `parts` warps, part_blocks each, through [Nl][blocks + 2][6][ninst] floats
+  int parts, part_blocks;
+  float *blocks;
   double *partial;   // [n_chunks][nF][3][ninst], per_loop: [Nl][nF][3][ninst]
   int *status;       // kDevOk / kDevTimeout
   uint32_t wait_tries;
@@ -118,6 +122,39 @@ inline void sweep_units(SweepArgs &a, int kprof, int fermion, int nint, double i
   a.n_units = (loops + a.unit_loops - 1) / a.unit_loops;
 }
 constexpr double kNoSplit = 1e300;  // items of a launch that keeps whole chunks
+
+// Kahan blocks of a loop's walk: 8 groups, counted from the loop's first walked
+// group (1) up to group 64 and from multiples of 64 groups (256 points) after it
+inline __host__ __device__ int loop_blocks(int nq) {
+  return nq <= 64 ? (nq + 6) / 8 : 8 + (nq - 64 + 7) / 8;
+}
+inline __host__ __device__ int block_begin(int b) { return b < 8 ? 1 + 8 * b : 8 * b; }
+
+// A heavy profile's launch of fewer than two waves of single-loop units: its
+// loops are cut further, at their Kahan blocks, into about four waves of warps
+// (at most 8 blocks, a landing zone, each); a second kernel adds the blocks in
+// the walk's order.  Sets a.parts (0: not cut) and returns the floats needed.
+//   Bound by latency there: fixflux, 64 instances on 512 x 512 points (1024
+// units on 2432 slots), issued in a fifth of the cycles: 48.2 -> 26.9 ms;
+// periodic, 128 instances on 1024 x 512 (4096 units): 32.7 -> 23.9 ms.
+inline size_t sweep_parts(SweepArgs &a, bool heavy) {
+  constexpr size_t kMost = (size_t)64 << 20;  // floats (256 MB)
+  const long long units = (long long)((a.ninst + 31) / 32) * a.n_chunks * a.chunk_loops;
+  a.parts = 0;
+  if (!heavy || !a.per_loop || units >= 2 * kSweepSlots) return 0;
+  const int nb = loop_blocks(a.ppl / 4);
+  int parts = (int)((4 * kSweepSlots + units - 1) / units);
+  if (parts < (nb + 7) / 8) parts = (nb + 7) / 8;
+  if (parts > nb) parts = nb;
+  const size_t need = (size_t)a.n_chunks * a.chunk_loops * (nb + 2) * 6 * a.ninst;
+  if (parts < 2 || need > kMost) return 0;
+  a.part_blocks = (nb + parts - 1) / parts;
+  a.parts = (nb + a.part_blocks - 1) / a.part_blocks;
+  return need;
+}
+inline bool heavy_profile(int kprof) {
+  return kprof == kPeriodic || kprof == kSpline || kprof == kFixflux || kprof == kFixfluxFF;
+}
 
 // Persistent multi-job sweep: a queue of tiles (job, instance tile, loop
 // chunk) drained by one CTA per slot; jobs differ in ensemble, profile,

@@ -103,7 +103,7 @@ template <int P, bool FERM, int NINT, bool EDGE = false>
 __device__ __forceinline__ void vseg(float zix, float ziy, float zjx, float zjy,
                                      const FieldDev &F, const ImgRange &img, float &ph,
                                      float &sp) {
-  seg<P, FERM, NINT>(zix, ziy, zjx, zjy, F, img, ph, sp);
+  seg<P, FERM, NINT, kSqRound>(zix, ziy, zjx, zjy, F, img, ph, sp);
 }
 template <int P, bool FERM, int NINT, bool EDGE = false>
 __device__ __forceinline__ void vseg(float2 zix, float2 ziy, float2 zjx, float2 zjy,
@@ -112,8 +112,7 @@ __device__ __forceinline__ void vseg(float2 zix, float2 ziy, float2 zjx, float2 
   seg2<P, FERM, NINT, EDGE>(zix, ziy, zjx, zjy, F, ph, sp);
 }
 
-// Kahan blocks: 8 groups, counted from the loop's first walked group (1) up to
-// group 64 and from multiples of 64 groups (256 points) after it
+// end of the Kahan block that holds group q (loop_blocks)
 __device__ __forceinline__ int block_end(int q) {
   return q < 64 ? min(((q - 1) & ~7) + 9, 64) : (q & ~7) + 8;
 }
@@ -824,6 +823,132 @@ __global__ void __launch_bounds__(kSweepThreads, 4)
     warp_unit<P, FERM, NINT, PAIR>(A, tile, l0, l1, row, W);
 }
 
+// One part of a heavy profile's loop (SweepArgs::parts): the FP32 sums of its
+// Kahan blocks, of the opening segment (part 0) and of the closing ones (last),
+// exactly as warp_unit forms them, stored for loop_finish_kernel.
+template <int P, bool FERM>
+__global__ void __launch_bounds__(kSweepThreads, 4)
+    sweep_part_kernel(const __grid_constant__ SweepArgs A) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  __shared__ __align__(8) uint64_t bars[kSweepWarps];
+  const int lane = threadIdx.x & 31;
+  const unsigned item = blockIdx.x * kSweepWarps + (threadIdx.x >> 5);
+  const unsigned u = item / (unsigned)A.n_tiles;
+  const int l = u / (unsigned)A.parts, part = u % (unsigned)A.parts;
+  if (l >= A.n_chunks * A.chunk_loops) return;  // whole warp
+  WarpStage W = warp_stage(smem, bars, kStageBytes);
+  warp_stage_init(W.bar);
+  const int slot = (item % (unsigned)A.n_tiles) * 32 + lane;
+  const bool live = slot < A.ninst;
+  const int ic = live ? slot : A.ninst - 1;
+  const FieldDev &F = A.field;
+  const float cx = A.cx[ic], cy = A.cy[ic], s = A.rtT[ic];
+  const int nq = A.ppl >> 2, nb = loop_blocks(nq);
+  const int b0 = part * A.part_blocks, b1 = min(b0 + A.part_blocks, nb);
+  const int q0 = block_begin(b0), q1 = min(block_begin(b1), nq);
+  const float4 *const loop = A.loops + (size_t)l * A.ppl;
+  if (lane == 0) {
+    const uint32_t bytes = (uint32_t)((q1 - q0) * 4 * (int)sizeof(float4));
+    mbar_arrive_expect_tx(W.bar, bytes);
+    bulk_g2s(W.land, loop + 4 * q0, bytes, W.bar);
+  }
+  auto scale = [&](float2 v, float &x, float &y) {
+    x = fmaf(s, v.x, cx);
+    y = fmaf(s, v.y, cy);
+  };
+  auto gpt = [&](int p, float &x, float &y) {
+    scale(__ldg(reinterpret_cast<const float2 *>(loop + p)), x, y);
+  };
+  auto pt = [&](int p, float &x, float &y) {
+    scale(*reinterpret_cast<const float2 *>(W.land + (p - 4 * q0)), x, y);
+  };
+  float *const out = A.blocks + (size_t)l * (nb + 2) * 6 * A.ninst + ic;
+  auto put = [&](int b, const float *ph, const float *sp) {
+    if (!live) return;
+    float *o = out + (size_t)b * 6 * A.ninst;
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+      o[(size_t)r * A.ninst] = ph[r];
+      if (FERM) o[(size_t)(3 + r) * A.ninst] = sp[r];
+    }
+  };
+  const ImgRange img = {0, -1, 0, -1, 1};
+  float zAx, zAy, zBx, zBy, zOx, zOy;  // previous point of each sub-loop
+  gpt(4 * q0 - 4, zAx, zAy);
+  gpt(4 * q0 - 2, zBx, zBy);
+  gpt(4 * q0 - 1, zOx, zOy);
+  if (part == 0) {
+    float ph[3] = {0.f, 0.f, 0.f}, sp[3] = {0.f, 0.f, 0.f}, x, y;
+    gpt(1, x, y);
+    seg<P, FERM, 0, kSqRound>(x, y, zOx, zOy, F, img, ph[0], sp[0]);  // N/2: 1 -> 3
+    put(0, ph, sp);
+  }
+  if (!warp_stage_wait(A, W)) return;
+#pragma unroll 1
+  for (int b = b0; b < b1; ++b) {
+    float bp[3] = {0.f, 0.f, 0.f}, bs[3] = {0.f, 0.f, 0.f};
+    const int qe = min(block_begin(b + 1), nq);
+#pragma unroll 1
+    for (int q = block_begin(b); q < qe; ++q) {
+      float P0x, P0y, P1x, P1y, P2x, P2y, P3x, P3y;
+      pt(4 * q, P0x, P0y);
+      pt(4 * q + 1, P1x, P1y);
+      pt(4 * q + 2, P2x, P2y);
+      pt(4 * q + 3, P3x, P3y);
+      seg<P, FERM, 0, kSqRound>(zAx, zAy, P0x, P0y, F, img, bp[2], bs[2]);  // N/4a: 4q-4 -> 4q
+      seg<P, FERM, 0, kSqRound>(zOx, zOy, P1x, P1y, F, img, bp[0], bs[0]);  // N/2 : 4q-1 -> 4q+1
+      seg<P, FERM, 0, kSqRound>(zBx, zBy, P2x, P2y, F, img, bp[1], bs[1]);  // N/4b: 4q-2 -> 4q+2
+      seg<P, FERM, 0, kSqRound>(P1x, P1y, P3x, P3y, F, img, bp[0], bs[0]);  // N/2 : 4q+1 -> 4q+3
+      zAx = P0x; zAy = P0y;
+      zBx = P2x; zBy = P2y;
+      zOx = P3x; zOy = P3y;
+    }
+    put(1 + b, bp, bs);
+  }
+  if (part == A.parts - 1) {
+    float tp[3] = {0.f, 0.f, 0.f}, ts[3] = {0.f, 0.f, 0.f}, x, y;
+    gpt(1, x, y);
+    seg<P, FERM, 0, kSqRound>(zOx, zOy, x, y, F, img, tp[0], ts[0]);  // N/2 : N-1 -> 1
+    gpt(2, x, y);
+    seg<P, FERM, 0, kSqRound>(zBx, zBy, x, y, F, img, tp[1], ts[1]);  // N/4b: N-2 -> 2
+    gpt(0, x, y);
+    seg<P, FERM, 0, kSqRound>(zAx, zAy, x, y, F, img, tp[2], ts[2]);  // N/4a: N-4 -> 0
+    put(1 + nb, tp, ts);
+  }
+}
+
+// the parts' sums of one (loop, instance) in the walk's order, and its epilogue
+// (one instantiation per profile: the units are compiled with different options)
+template <int P, bool FERM>
+__global__ void __launch_bounds__(128) loop_finish_kernel(const __grid_constant__ SweepArgs A) {
+  const long long at = (long long)blockIdx.x * 128 + threadIdx.x;
+  const int l = (int)(at / A.ninst), i = (int)(at % A.ninst);
+  if (l >= A.n_chunks * A.chunk_loops) return;
+  const int nb = loop_blocks(A.ppl >> 2);
+  const float *b = A.blocks + (size_t)l * (nb + 2) * 6 * A.ninst + i;
+  const size_t n = (size_t)A.ninst;
+  float ph[3] = {b[0], 0.f, 0.f}, pc[3] = {0.f, 0.f, 0.f};
+  float sp[3] = {FERM ? b[3 * n] : 0.f, 0.f, 0.f}, sc[3] = {0.f, 0.f, 0.f};
+#pragma unroll 2
+  for (int k = 0; k <= nb; ++k) {  // the blocks, then the closing segments
+    b += 6 * n;
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+      kahan_add(ph[r], pc[r], b[r * n]);
+      if (FERM) kahan_add(sp[r], sc[r], b[(3 + r) * n]);
+    }
+  }
+  const df G[3] = {fast_two_sum(ph[0], -pc[0]), fast_two_sum(ph[1], -pc[1]),
+                   fast_two_sum(ph[2], -pc[2])};
+  const df H[3] = {fast_two_sum(sp[0], -sc[0]), fast_two_sum(sp[1], -sc[1]),
+                   fast_two_sum(sp[2], -sc[2])};
+  const df tq = {A.tqh[i], A.tql[i]};
+  loop_epilogue<FERM>(G, H, A.cph_hi, A.cph_lo, A.csp_hi, A.csp_lo, tq, A.nF,
+                      [&](int j, double w0, double w1, double w2) {
+                        put_loop(A, l, j, i, false, w0, w1, w2);
+                      });
+}
+
 // One warp per (loop, instance), or (A.split) two: the N/2 sub-loop's segments
 // on one, both N/4 sub-loops' on the other -- the same work each, and the same
 // sums, since the sub-loops' accumulators are separate.  Bound by latency when
@@ -961,6 +1086,19 @@ cudaError_t sweep_launch(SweepArgs a, cudaStream_t s) {
   return cudaGetLastError();
 }
 
+template <int P, bool FERM>
+cudaError_t sweep_parts_launch(SweepArgs a, cudaStream_t s) {
+  a.n_tiles = (a.ninst + 31) / 32;
+  const long long loops = (long long)a.n_chunks * a.chunk_loops;
+  const long long items = loops * a.parts * a.n_tiles;
+  sweep_part_kernel<P, FERM><<<(unsigned)((items + kSweepWarps - 1) / kSweepWarps), kSweepThreads,
+                               sweep_smem_bytes(), s>>>(a);
+  const cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return e;
+  loop_finish_kernel<P, FERM><<<(unsigned)((loops * a.ninst + 127) / 128), 128, 0, s>>>(a);
+  return cudaGetLastError();
+}
+
 template <int P>
 cudaError_t sweep_dispatch(bool fermion, int nint, const SweepArgs &a, cudaStream_t s) {
   constexpr bool kLight = P == kSmooth || P == kStep || P == kQuadratic || P == kGaussian;
@@ -983,6 +1121,10 @@ cudaError_t sweep_dispatch(bool fermion, int nint, const SweepArgs &a, cudaStrea
     // smooth +20 % / +13 % (scalar / spinor), Gaussian +56 % / +54 %, step
     // +4 % / +31 %, quadratic +35 % / +24 %
     WL_SWEEP_CASE(50, true)
+  }
+  if constexpr (Profile<P>::kHeavy) {
+    if (a.parts)
+      return fermion ? sweep_parts_launch<P, true>(a, s) : sweep_parts_launch<P, false>(a, s);
   }
   // other interval counts, the heavy profiles one loop at a time
   WL_SWEEP_CASE(0, kLight)
