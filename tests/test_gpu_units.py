@@ -68,12 +68,12 @@ def test_single_loops_and_whole_chunks_agree_bit_for_bit(prof, fe, nint, n):
                                          ("fixflux", 0, 1)])
 def test_heavy_profiles_cut_at_their_blocks(prof, fe, ffv, ppl):
     """wl_eval cuts these loops at their Kahan blocks (few units); among many
-    loops (two tiles of 2512) it walks them whole: the same bits."""
+    loops (two tiles of 4912) it walks them whole: the same bits."""
     import wltube
 
     fld = wltube.field(prof, fermion=fe, nint=4, lambda2=0.5, tubedist=1.0, ff_variant=ffv)
     few = O.vloops(43, 9, ppl)
-    many = np.concatenate([few, O.vloops(44, 2503, ppl)])
+    many = np.concatenate([few, O.vloops(44, 4903, ppl)])
     cx, cy, T = instances(40, ppl)
     with wltube.Context(0) as ctx:
         g, _, _ = ctx.eval(ctx.upload(few), fld, cx, cy, T, [0.7], 1)

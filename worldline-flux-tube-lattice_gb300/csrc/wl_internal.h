@@ -130,20 +130,22 @@ inline __host__ __device__ int loop_blocks(int nq) {
 }
 inline __host__ __device__ int block_begin(int b) { return b < 8 ? 1 + 8 * b : 8 * b; }
 
-// A heavy profile's launch of fewer than two waves of single-loop units: its
-// loops are cut further, at their Kahan blocks, into about four waves of warps
-// (at most 8 blocks, a landing zone, each); a second kernel adds the blocks in
-// the walk's order.  Sets a.parts (0: not cut) and returns the floats needed.
+// A heavy profile's launch of fewer than two waves of single-loop units (8 CTAs
+// per SM, sweep_min_ctas): its loops are cut further, at their Kahan blocks, into
+// about four waves of warps (at most 8 blocks, a landing zone, each); a second
+// kernel adds the blocks in the walk's order.  Sets a.parts (0: not cut) and
+// returns the floats needed.
 //   Bound by latency there: fixflux, 64 instances on 512 x 512 points (1024
-// units on 2432 slots), issued in a fifth of the cycles: 48.2 -> 26.9 ms;
-// periodic, 128 instances on 1024 x 512 (4096 units): 32.7 -> 23.9 ms.
+// units), issued in a fifth of the cycles: 48.2 -> 26.9 ms, and 21 with 8 CTAs
+// per SM; periodic, 128 instances on 1024 x 512 (4096 units): 32.7 -> 23.9 ms.
+// Two waves instead of four 5 % slower, eight the same.
 inline size_t sweep_parts(SweepArgs &a, bool heavy) {
   constexpr size_t kMost = (size_t)64 << 20;  // floats (256 MB)
   const long long units = (long long)((a.ninst + 31) / 32) * a.n_chunks * a.chunk_loops;
   a.parts = 0;
-  if (!heavy || !a.per_loop || units >= 2 * kSweepSlots) return 0;
+  if (!heavy || !a.per_loop || units >= 4 * kSweepSlots) return 0;
   const int nb = loop_blocks(a.ppl / 4);
-  int parts = (int)((4 * kSweepSlots + units - 1) / units);
+  int parts = (int)((8 * kSweepSlots + units - 1) / units);
   if (parts < (nb + 7) / 8) parts = (nb + 7) / 8;
   if (parts > nb) parts = nb;
   const size_t need = (size_t)a.n_chunks * a.chunk_loops * (nb + 2) * 6 * a.ninst;

@@ -802,9 +802,19 @@ __device__ __forceinline__ size_t unit_loops(const SweepArgs &A, int u, int &l0,
   return A.per_loop ? (size_t)l0 : (size_t)u;
 }
 
+// CTAs per SM a sweep is compiled for.  The heavy profiles wait on chains of
+// divisions and exponentials, not on a pipe, and gain from more warps than from
+// registers (spills included): over 4 CTAs fixflux 8 per SM 19-21 % faster,
+// periodic 8 1-12 %, spline 6 9-22 % (512 instances on 512 loops, 8 and 50
+// intervals); the light profiles lose 2-6 % at 5 or 6.
+template <int P>
+constexpr int sweep_min_ctas() {
+  return !Profile<P>::kHeavy ? 4 : P == kSpline ? 6 : 8;
+}
+
 // warp -> (unit, instance tile), the tiles of a unit on consecutive warps
 template <int P, bool FERM, int NINT, bool PAIR>
-__global__ void __launch_bounds__(kSweepThreads, 4)
+__global__ void __launch_bounds__(kSweepThreads, sweep_min_ctas<P>())
     sweep_kernel(const __grid_constant__ SweepArgs A) {
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ __align__(8) uint64_t bars[kSweepWarps];
@@ -827,7 +837,7 @@ __global__ void __launch_bounds__(kSweepThreads, 4)
 // Kahan blocks, of the opening segment (part 0) and of the closing ones (last),
 // exactly as warp_unit forms them, stored for loop_finish_kernel.
 template <int P, bool FERM>
-__global__ void __launch_bounds__(kSweepThreads, 4)
+__global__ void __launch_bounds__(kSweepThreads, sweep_min_ctas<P>())
     sweep_part_kernel(const __grid_constant__ SweepArgs A) {
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ __align__(8) uint64_t bars[kSweepWarps];
