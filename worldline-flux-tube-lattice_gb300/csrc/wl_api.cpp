@@ -549,7 +549,7 @@ int batch_plan(wl_ctx *ctx, int njobs, const wl_job *jobs, int points, bool may_
     wl::ReduceJob &rj = P->rjobs[i];
     rj.shape = {nullptr, a.n_chunks, J.group / lcs[i], a.per_loop ? lcs[i] : 1,
                 J.group, n,          J.nF};
-    rj.ti = wl::reduce_instances(n, J.nF, e.Nl / J.group);
+    rj.ti = wl::reduce_instances(n, J.nF);
     rj.first = P->reduce_blocks;
     rj.out_group = (double *)(uintptr_t)(out_off[i]);
     P->reduce_blocks += wl::reduce_blocks(rj);
@@ -563,8 +563,13 @@ int batch_plan(wl_ctx *ctx, int njobs, const wl_job *jobs, int points, bool may_
     const int cost = (int)fmin(
         2e9, wl::profile_weight(kprofs[i], a.fermion, a.nint) * a.unit_loops * e.ppl *
                  (per_tile / wl::kSweepThreads));
-    for (int c = 0; c < a.n_units; ++c)
-      for (int t = 0; t < tiles_x; ++t) P->tiles.push_back({i, t, c, cost});
+    if (kprofs[i] == wl::kLattice) {  // the instance order puts the most images first
+      for (int t = 0; t < tiles_x; ++t)
+        for (int c = 0; c < a.n_units; ++c) P->tiles.push_back({i, t, c, cost});
+    } else {
+      for (int c = 0; c < a.n_units; ++c)
+        for (int t = 0; t < tiles_x; ++t) P->tiles.push_back({i, t, c, cost});
+    }
   }
   // longest tiles first: the queue then drains evenly (LPT order); ties keep
   // job order

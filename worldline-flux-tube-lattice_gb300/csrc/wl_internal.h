@@ -172,13 +172,13 @@ struct ReduceShape {
 };
 constexpr int kReduceThreads = 256;
 // Instances per CTA of a reduction: 32 (a warp reads 256 contiguous bytes)
-// when that fills the chip, else fewer, down to the 4 of a 32-byte sector, so
-// that more CTAs run and more groups are summed at once.
-inline int reduce_instances(int ninst, int nF, int ng) {
+// when that fills the chip, else fewer, down to the 4 of a 32-byte sector: the
+// FP64 additions (2 lanes per SM per clock) then run on all SMs, and more groups
+// at once.
+inline int reduce_instances(int ninst, int nF) {
   int ti = 32;
   while (ti > 1 && ti / 2 >= ninst) ti /= 2;
-  while (ti > 4 && (long long)((ninst + ti - 1) / ti) * nF < 304 && kReduceThreads / ti < ng)
-    ti /= 2;
+  while (ti > 4 && (long long)((ninst + ti - 1) / ti) * nF < 304) ti /= 2;
   return ti;
 }
 struct ReduceJob {  // per job: where its partial sums and outputs live

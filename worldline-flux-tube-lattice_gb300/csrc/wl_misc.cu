@@ -131,7 +131,7 @@ cudaError_t launch_order_instances(const float *cx, const float *cy, const float
 cudaError_t launch_group_reduce(const ReduceShape &r, double *out_group, double *out_mean,
                                 double *out_sem, const int *status, double *status_out,
                                 cudaStream_t s) {
-  const int ti = reduce_instances(r.ninst, r.nF, r.n_chunks / r.cpg);
+  const int ti = reduce_instances(r.ninst, r.nF);
   const dim3 grid((r.ninst + ti - 1) / ti, r.nF);
   group_reduce_kernel<<<grid, kReduceThreads, 0, s>>>(r, ti, out_group, out_mean, out_sem,
                                                        status, status_out);

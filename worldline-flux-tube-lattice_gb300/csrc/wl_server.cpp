@@ -485,7 +485,7 @@ bool admit(wl_server *s) {
     rj.out_mean = d_out + (size_t)n * nF * R->ng;
     rj.out_sem = rj.out_mean + (size_t)n * nF;
     rj.shape = {d_part, R->n_chunks, R->q.group / R->lc, 1, R->q.group, n, nF};
-    rj.ti = wl::reduce_instances(n, nF, R->ng);
+    rj.ti = wl::reduce_instances(n, nF);
     rj.first = 0;
     memcpy(pin + R->p_args, &a, sizeof(a));
     memcpy(pin + R->p_rj, &rj, sizeof(rj));
