@@ -380,15 +380,15 @@ constexpr uint32_t kVloopTag = 0x764C6F6Fu;  // counter word 2 ("vLoo")
 // four standard normals of step k of loop l (Box-Muller in FP64)
 __device__ __forceinline__ void step_normals(uint2 key, int k, int lg, double n[4]) {
   const uint4 r = philox4x32_10(make_uint4((uint32_t)k, (uint32_t)lg, kVloopTag, 0u), key);
-  const double two32 = 4294967296.0;
   const uint32_t v[4] = {r.x, r.y, r.z, r.w};
 #pragma unroll
   for (int p = 0; p < 2; ++p) {
-    const double u = ((double)v[2 * p] + 0.5) / two32;
-    const double w = ((double)v[2 * p + 1] + 0.5) / two32;
+    // u = (v + 1/2) / 2^32 and 2 w = (v' + 1/2) / 2^31, exact in one operation
+    const double u = fma((double)v[2 * p], 0x1p-32, 0x1p-33);
+    const double w2 = fma((double)v[2 * p + 1], 0x1p-31, 0x1p-32);
     const double rad = sqrt(-2.0 * log(u));
     double sn, cs;
-    sincospi(2.0 * w, &sn, &cs);
+    sincospi(w2, &sn, &cs);
     n[2 * p] = rad * cs;
     n[2 * p + 1] = rad * sn;
   }
@@ -406,7 +406,8 @@ __device__ __forceinline__ void step_normals(uint2 key, int k, int lg, double n[
 // a sincospi for two of a step's four normals).  Generating, evaluating and
 // releasing 2048 loops of 1024 points took 12.6 ms with one thread per loop,
 // both passes drawing (11.4 ms of it the generator, the same for any loop count
-// up to the chip's threads), and takes 2.05 ms with one CTA per loop.
+// up to the chip's threads), and 2.05 ms with one CTA per loop (1.81 now, half
+// of it the generator, 116 FP64 operations per pair of normals).
 constexpr int kVloopMaxThreads = 256;
 constexpr int kVloopMaxWarps = kVloopMaxThreads / 32;
 constexpr size_t kVloopMaxSmem = 200 * 1024;
@@ -473,8 +474,11 @@ __global__ void __launch_bounds__(kVloopMaxThreads)
     mean[d] = s / (double)ppl - tot[d] * ((double)(ppl - 1) / (2.0 * ppl));
   }
   float4 *o = out + (size_t)l * ppl;
+  // k / ppl: for a power of two the product with 1 / ppl is the same, exactly
+  const bool pow2 = (ppl & (ppl - 1)) == 0;
+  const double inv = 1.0 / (double)ppl;
   for (int k = k0; k < k1; ++k) {
-    const double fk = (double)k / (double)ppl;
+    const double fk = pow2 ? (double)k * inv : (double)k / (double)ppl;
     o[k] = make_float4((float)(pre[0] - fk * tot[0] - mean[0]), (float)(pre[1] - fk * tot[1] - mean[1]),
                        (float)(pre[2] - fk * tot[2] - mean[2]), (float)(pre[3] - fk * tot[3] - mean[3]));
     double n[4];
