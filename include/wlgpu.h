@@ -298,10 +298,10 @@ typedef struct {
 
 #define WL_BATCH_GRAPH 1 /* capture the device work as a CUDA graph and launch it */
 
-/* Evaluate njobs jobs of uneven size in one persistent launch: every CTA takes
- * (job, instance tile, loop chunk) tiles from a device queue ordered by
- * decreasing cost; a job's results are identical to those it gets alone in a
- * batch (the tile shape depends only on the job and the tuned parameters).
+/* Evaluate njobs jobs of uneven size in one persistent launch: every warp takes
+ * (job, instances, loops) units from a device queue ordered by decreasing cost;
+ * a job's results are identical to those it gets alone in a batch (its sums run
+ * over the same loops in the same order, whatever the units).
  * The loops per tile come from the context's tuned points-per-tile target
  * (wl_batch_autotune; default 16384), the persistent grid from its tuned CTAs
  * per SM (default: the occupancy limit).  Jobs of the periodic, spline and

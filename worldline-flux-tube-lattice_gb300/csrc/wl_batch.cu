@@ -15,54 +15,81 @@ namespace wl {
 
 namespace {
 
-// One warp's unit of a job: loop pairs for the light profiles at 4 and 50
-// intervals, two instances per lane for the lattice at 4 -- as the single-job
-// sweep, so such a job's loops match it bit for bit -- one instance per lane
-// otherwise.
+// The persistent kernel's CTAs are single warps (a slot of the launch's grid is
+// four of them): a warp that finds the queue empty leaves at once, where in a
+// CTA of four each waited for the slowest (an uneven batch of six jobs 18.7 ->
+// 18.4 ms).
+// Dynamic shared memory: the warp's stage, its barrier, its job's parameters.
+constexpr int kBatchBar = kLatStageBytes;
+constexpr int kBatchJob = kBatchBar + 16;
+constexpr int kBatchSmem = kBatchJob + 16 * (((int)sizeof(SweepArgs) + 15) / 16);
+extern __shared__ __align__(128) unsigned char batch_smem[];
+
+__device__ __forceinline__ SweepArgs &warp_job() {
+  return *reinterpret_cast<SweepArgs *>(batch_smem + kBatchJob);
+}
+__device__ __forceinline__ WarpStage batch_stage() {
+  float4 *const land = reinterpret_cast<float4 *>(batch_smem);
+  return WarpStage{land, land + kLandPts, reinterpret_cast<uint64_t *>(batch_smem + kBatchBar), 0u};
+}
+
 // A called function per kind: each is allocated registers on its own (inlined,
 // the 28 of them spilled 420 bytes and the kernel ran an uneven batch of six
 // jobs in 43.9 ms; called, and with the lattice units first, 20.0 ms; CTA tiles
-// of 256 instances, 33 ms).
+// of 256 instances, 33 ms).  It finds its stage and job in shared memory itself:
+// through pointer arguments the walk's loads were generic ones, and the field's
+// constants were loaded at every segment (4000 smooth instances on 4096 x 1024
+// points, scalar, 20.0 -> 18.5 ms).
+// Takes and returns the stage's count of copies; ~0u: a copy timed out.
 template <int P, bool FERM, int NINT, bool PAIR>
-__device__ __noinline__ bool unit_called(const SweepArgs &A, int tile, int l0, int l1, size_t row,
-                                         WarpStage &W) {
+__device__ __noinline__ uint32_t unit_called(int tile, int l0, int l1, size_t row,
+                                             uint32_t copies) {
+  const SweepArgs &A = warp_job();
+  WarpStage W = batch_stage();
+  W.copies = copies;
+  bool ok;
   if constexpr (P == kLattice && PAIR)
-    return warp_unit_lattice<FERM, false>(A, tile, l0, l1, row, W);
+    ok = warp_unit_lattice<FERM, false, const FieldDev>(A, tile, l0, l1, row, W);
   else
-    return warp_unit<P, FERM, NINT, PAIR>(A, tile, l0, l1, row, W);
+    ok = warp_unit<P, FERM, NINT, PAIR, const FieldDev>(A, tile, l0, l1, row, W);
+  return ok ? W.copies : ~0u;
 }
+
+// One warp's unit of a job: loop pairs for the light profiles, two instances
+// per lane for the lattice at 4 intervals -- as the single-job sweep, so such a
+// job's loops match it bit for bit -- one loop at a time otherwise.
 template <bool FERM, int NINT>
-__device__ __forceinline__ bool run_unit(const SweepArgs &A, int tile, int l0, int l1, size_t row,
-                                         WarpStage &W) {
-  constexpr bool kPair = true;  // loop pairs
-  switch (A.kprof) {
-    case kSmooth: return unit_called<kSmooth, FERM, NINT, kPair>(A, tile, l0, l1, row, W);
-    case kGaussian: return unit_called<kGaussian, FERM, NINT, kPair>(A, tile, l0, l1, row, W);
-    case kStep: return unit_called<kStep, FERM, NINT, kPair>(A, tile, l0, l1, row, W);
-    case kQuadratic: return unit_called<kQuadratic, FERM, NINT, kPair>(A, tile, l0, l1, row, W);
+__device__ __forceinline__ uint32_t run_unit(int kprof, int tile, int l0, int l1, size_t row,
+                                             uint32_t copies) {
+  switch (kprof) {
+    case kSmooth: return unit_called<kSmooth, FERM, NINT, true>(tile, l0, l1, row, copies);
+    case kSmoothWide:
+      if constexpr (NINT == 4)
+        return unit_called<kSmoothWide, FERM, 4, true>(tile, l0, l1, row, copies);
+      return copies;
+    case kGaussian: return unit_called<kGaussian, FERM, NINT, true>(tile, l0, l1, row, copies);
+    case kStep: return unit_called<kStep, FERM, NINT, true>(tile, l0, l1, row, copies);
+    case kQuadratic: return unit_called<kQuadratic, FERM, NINT, true>(tile, l0, l1, row, copies);
     case kLattice:
-      if constexpr (NINT == 4) return unit_called<kLattice, FERM, 4, true>(A, tile, l0, l1, row, W);
+      if constexpr (NINT == 4)
+        return unit_called<kLattice, FERM, 4, true>(tile, l0, l1, row, copies);
       if constexpr (NINT == 0)
-        return unit_called<kLattice, FERM, NINT, false>(A, tile, l0, l1, row, W);
-      return true;
-    default: return true;
+        return unit_called<kLattice, FERM, 0, false>(tile, l0, l1, row, copies);
+      return copies;
+    default: return copies;
   }
 }
 
-constexpr int kBatchMinBlocks = 4;
+constexpr int kBatchMinSlots = 4;  // per SM
 
-// Every warp takes units from the queue (a tile holds one unit for each of its
-// CTA's four warps' instances) and works alone, its job's parameters in shared
-// memory.
-__global__ void __launch_bounds__(kSweepThreads, kBatchMinBlocks)
+// Every warp takes units from the queue (a tile holds kSweepWarps of them) and
+// works alone.
+__global__ void __launch_bounds__(32, kBatchMinSlots * kSweepWarps)
     batch_kernel(const __grid_constant__ BatchArgs B) {
-  extern __shared__ __align__(128) unsigned char smem[];
-  __shared__ __align__(8) uint64_t bars[kSweepWarps];
-  __shared__ __align__(16) SweepArgs jobs[kSweepWarps];
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  SweepArgs &job = jobs[w];
-  WarpStage W = warp_stage(smem, bars, kLatStageBytes);
-  warp_stage_init(W.bar);
+  const int lane = threadIdx.x;
+  SweepArgs &job = warp_job();
+  warp_stage_init(batch_stage().bar);
+  uint32_t copies = 0;
   int have = -1;  // the job whose parameters this warp holds
   for (;;) {
     int t = 0;
@@ -81,21 +108,22 @@ __global__ void __launch_bounds__(kSweepThreads, kBatchMinBlocks)
     if (tile >= job.n_tiles) continue;
     int l0, l1;
     const size_t row = unit_loops(job, d.chunk, l0, l1);
-    // 4 and 50 intervals (the reference's): unrolled, pairs for the light
-    // profiles; any other count at run time
-    const bool n50 = job.nint == 50 && light_profile(job.kprof);
-    bool ok;
+    // 4 and 50 intervals (the reference's) unrolled, any other count at run time
+    const int k = job.kprof == kSmooth && job.nint == 4 && smooth_clamp_idle(job.field)
+                      ? kSmoothWide
+                      : job.kprof;
+    const bool n50 = job.nint == 50 && light_profile(k);
     if (job.fermion) {
-      if (job.nint == 4) ok = run_unit<true, 4>(job, tile, l0, l1, row, W);
-      else if (n50) ok = run_unit<true, 50>(job, tile, l0, l1, row, W);
-      else ok = run_unit<true, 0>(job, tile, l0, l1, row, W);
+      if (job.nint == 4) copies = run_unit<true, 4>(k, tile, l0, l1, row, copies);
+      else if (n50) copies = run_unit<true, 50>(k, tile, l0, l1, row, copies);
+      else copies = run_unit<true, 0>(k, tile, l0, l1, row, copies);
     } else {
-      if (job.nint == 4) ok = run_unit<false, 4>(job, tile, l0, l1, row, W);
-      else if (n50) ok = run_unit<false, 50>(job, tile, l0, l1, row, W);
-      else ok = run_unit<false, 0>(job, tile, l0, l1, row, W);
+      if (job.nint == 4) copies = run_unit<false, 4>(k, tile, l0, l1, row, copies);
+      else if (n50) copies = run_unit<false, 50>(k, tile, l0, l1, row, copies);
+      else copies = run_unit<false, 0>(k, tile, l0, l1, row, copies);
     }
-    if (!ok) break;  // a copy timed out: the status is set, stop taking units
-    __syncwarp();    // the job's parameters may be rewritten next
+    if (copies == ~0u) break;  // a copy timed out: the status is set, stop taking units
+    __syncwarp();              // the job's parameters may be rewritten next
   }
 }
 
@@ -207,28 +235,18 @@ bool batch_in_kernel(int kprof) { return light_profile(kprof) || kprof == kLatti
 
 bool plain_supports(int kprof) { return light_profile(kprof) || kprof == kLattice; }
 
-// the lattice units' staging may pass the 48 KiB a launch gets without opting
-// in; the attribute is per device, so it is set before every use
-static cudaError_t batch_smem_optin() {
-  return cudaFuncSetAttribute(batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)sweep_lat_smem_bytes());
-}
-
 int batch_max_ctas_per_sm() {
   int n = 0;
-  if (batch_smem_optin() != cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, batch_kernel, kSweepThreads,
-                                                    sweep_lat_smem_bytes()) != cudaSuccess) {
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, batch_kernel, 32, kBatchSmem) !=
+      cudaSuccess) {
     cudaGetLastError();
     return 1;
   }
-  return n > 0 ? n : 1;
+  return n >= kSweepWarps ? n / kSweepWarps : 1;
 }
 
 cudaError_t launch_batch(const BatchArgs &a, int grid, cudaStream_t s) {
-  const cudaError_t e = batch_smem_optin();
-  if (e != cudaSuccess) return e;
-  batch_kernel<<<grid, kSweepThreads, sweep_lat_smem_bytes(), s>>>(a);
+  batch_kernel<<<grid * kSweepWarps, 32, kBatchSmem, s>>>(a);
   return cudaGetLastError();
 }
 

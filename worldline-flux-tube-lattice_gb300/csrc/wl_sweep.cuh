@@ -21,6 +21,8 @@
 //   groups of four points; per-loop results (EV() and few-instance calls).
 #pragma once
 
+#include <type_traits>
+
 #include "wl_device.cuh"
 #include "wl_internal.h"
 
@@ -138,7 +140,7 @@ __device__ __forceinline__ int block_end(int q) {
 // instances on 512 x 512, 375 -> 92 ms (48 with its segment's smaller code).
 //   row: the partial-sum row of loop l0 (per_loop) or of the unit's chunk.
 // Returns false if a copy timed out.
-template <int P, bool FERM, int NINT, bool PAIR>
+template <int P, bool FERM, int NINT, bool PAIR, class Field = const FieldDev &>
 __device__ __forceinline__ bool warp_unit(const SweepArgs &A, int tile, int l0, int l1,
                                           size_t row, WarpStage &W) {
   using V = typename Vec<PAIR>::T;
@@ -146,8 +148,14 @@ __device__ __forceinline__ bool warp_unit(const SweepArgs &A, int tile, int l0, 
   constexpr int kPiece = kLandPts / kStep;     // points per staged piece
   // groups in straight-line code: 4 where they fit the registers (smooth, the
   // scalar step profile: 2-5 % over 2), 2 elsewhere (4 there up to 11 %
-  // slower), 1 around a run-time node loop
-  constexpr int kUnroll = NINT == 0 ? 1 : NINT == 4 && (smooth_profile(P) || (P == kStep && !FERM)) ? 4 : 2;
+  // slower), 1 around a run-time node loop.  The persistent kernel (Field by
+  // value) runs several kinds of unit on an SM at once, whose code then
+  // competes for the instruction cache: 1 for the kinds that get 4 here (served
+  // smooth and Gaussian requests 4.9e11 segments/s at 4, 5.4e11 at 2, 5.57e11
+  // at 1; the other kinds at 1 too 5.52e11)
+  constexpr bool kMixed = !std::is_reference<Field>::value;
+  constexpr bool kShort = NINT == 4 && (smooth_profile(P) || (P == kStep && !FERM));
+  constexpr int kUnroll = NINT == 0 ? 1 : kShort ? (kMixed ? 1 : 4) : 2;
   const int lane = threadIdx.x & 31;
   const int slot = tile * 32 + lane;
   const bool live = slot < A.ninst;
@@ -155,7 +163,7 @@ __device__ __forceinline__ bool warp_unit(const SweepArgs &A, int tile, int l0, 
   // every per-instance read and the partial-sum write go through ic: a lane's
   // result does not depend on which slot it runs in
   const int ic = A.perm ? A.perm[sl] : sl;
-  const FieldDev &F = A.field;
+  Field F = A.field;  // by value where A is not in the constant bank
   const V cx = vset(V(), A.cx[ic]), cy = vset(V(), A.cy[ic]), s = vset(V(), A.rtT[ic]);
 
   auto issue = [&](int l, int p0) {  // points p0.. of the kStep loops from l
@@ -470,7 +478,7 @@ constexpr int kLatPts = kLandPts + 8, kLatFirst = kLandPts + 4;
 // (the single-job kernel; inside the persistent batch kernel the extra walk
 // measured 3 % slower on the uneven batch, so its units keep two walks --
 // the sums are the same bits either way)
-template <bool FERM, bool MIDWALK>
+template <bool FERM, bool MIDWALK, class Field = const FieldDev &>
 __device__ __forceinline__ bool warp_unit_lat(const SweepArgs &A, int tile, int l0, int l1,
                                               size_t row, WarpStage &W, float (*tot)[32],
                                               float4 *box) {
@@ -483,7 +491,7 @@ __device__ __forceinline__ bool warp_unit_lat(const SweepArgs &A, int tile, int 
   const int iA = A.perm ? A.perm[slA] : slA, iB = A.perm ? A.perm[slB] : slB;
   const int npc = (A.ppl + kLandPts - 1) / kLandPts;
   const int K = (l1 - l0) * npc;
-  const FieldDev &F = A.field;
+  Field F = A.field;
 
   auto issue = [&](int k) {
     const int l = l0 + k / npc, p0 = k % npc * kLandPts;
@@ -787,11 +795,11 @@ __device__ __forceinline__ WarpStage warp_stage(unsigned char *smem, uint64_t *b
 }
 
 // the lattice's totals and block boxes behind its compact points
-template <bool FERM, bool MIDWALK>
+template <bool FERM, bool MIDWALK, class Field = const FieldDev &>
 __device__ __forceinline__ bool warp_unit_lattice(const SweepArgs &A, int tile, int l0, int l1,
                                                   size_t row, WarpStage &W) {
   float4 *const box = W.comp + kLatPts;
-  return warp_unit_lat<FERM, MIDWALK>(A, tile, l0, l1, row, W,
+  return warp_unit_lat<FERM, MIDWALK, Field>(A, tile, l0, l1, row, W,
                                       reinterpret_cast<float(*)[32]>(box + kLatNSub), box);
 }
 
@@ -1116,8 +1124,7 @@ template <int P>
 cudaError_t sweep_dispatch(bool fermion, int nint, const SweepArgs &a, cudaStream_t s) {
   constexpr bool kLight = P == kSmooth || P == kStep || P == kQuadratic || P == kGaussian;
   if constexpr (P == kSmooth) {
-    const float c = a.field.clampA;
-    if (nint == 4 && (c < 0.0f || a.field.l2 + c == a.field.l2))
+    if (nint == 4 && smooth_clamp_idle(a.field))
       return fermion ? sweep_launch<kSmoothWide, true, 4, true>(a, s)
                      : sweep_launch<kSmoothWide, false, 4, true>(a, s);
   }

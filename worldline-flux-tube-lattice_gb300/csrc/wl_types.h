@@ -44,4 +44,13 @@ struct FieldDev {
   float sp_h, sp_piarg;
 };
 
+// whether the smooth profile's clamp of |z|^2 cannot act (kSmoothWide): there
+// is none, or l2 + clamp rounds to l2
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+inline bool smooth_clamp_idle(const FieldDev &f) {
+  return f.clampA < 0.0f || f.l2 + f.clampA == f.l2;
+}
+
 }  // namespace wl
