@@ -86,40 +86,6 @@ __device__ __forceinline__ float expint_lentz(float x) {
   return 0.0f;
 }
 
-__device__ __forceinline__ float bump_d(float x) {  // intEV.cu:151-159
-  return (x * x < 0.999f) ? expf(-1.0f / (1.0f - x * x)) : 0.0f;
-}
-
-template <bool FF>
-__device__ __forceinline__ float phi_d(float x) {  // intEV.cu:161-174 / intEVff.cu:147-157
-  const float onemx2 = 1.0f - x * x;
-  if (x < (FF ? 1.0f : 0.999f))
-    return 1.0f - (0.5f / 0.0742478f) *
-                      (onemx2 * expf(-1.0f / onemx2) + expint_lentz(-1.0f / onemx2));
-  return 1.0f;
-}
-
-template <bool FF>
-__device__ __forceinline__ float chi_d(float x, float n, float lam, float a) {
-  // intEV.cu:176-198 (logistic fit) / intEVff.cu:159-176 (cosh-ratio fit)
-  const float onemx2 = 1.0f - x * x, x2 = x * x, x4 = x2 * x2;
-  if (x <= (FF ? -1.0f : -0.999f)) return 0.0f;
-  if (x2 < (FF ? 1.0f : 0.999f)) {
-    float ans = 0.5f * (-onemx2 * expf(-1.0f / onemx2) - expint_lentz(-1.0f / onemx2));
-    if (FF)
-      ans += 2.0f * n * a / lam *
-             (0.218f + 0.393f * x * coshf(0.806f * x4 - 0.696f * x2 + 0.0902f) /
-                           coshf(0.825f * x2 - 0.0234f * x + 0.375f));
-    else
-      ans += 2.0f * n * a / lam * 0.444f /
-             (1.0f + expf(-(3.31f * x + 5.25f * x * x2 * sinf(x) *
-                                            cosf(-0.907f * x2 - 1.29f * x4 * x4)) /
-                          cosf(x)));
-    return ans;
-  }
-  return 2.0f * n * a * 0.443991f / lam;
-}
-
 template <int P>
 struct Profile;
 
@@ -254,36 +220,16 @@ struct Profile<kSpline> {  // interp (intEV.cu:64-107), fplambda spline (intEV.c
   static constexpr bool kHeavy = true;
 };
 
-template <bool FF>
-struct FixfluxProfile {  // intEV.cu:236-257, 333-357; intEVff.cu:194-250
-  static __device__ __forceinline__ void eval(float r2, const FieldDev &F, float &g,
-                                              float &fp) {
-    const float a = F.a, lam = F.lam, lml = F.lml, aml = F.aml;
-    const float rho = sqrtf(r2);
-    const float n = floorf((rho + 0.5f * a) / a);
-    float f;
-    if (r2 <= 0.25f * a * a) {
-      f = (1.0f - 0.75f * lml) * phi_d<FF>(2.0f * sqrtf(r2 * F.inv_l2)) +
-          3.0f * r2 / (a * a) * lml;
-    } else {
-      f = 1.0f + 0.75f * (4.0f * r2 / (a * a) - 1.0f) * lml + 3.0f * n * (n - 1.0f) * aml;
-      f += 3.0f * lam / (0.443991f * a) * aml *
-           chi_d<FF>(2.0f * (rho - n * a) / lam, n, lam, a);
-    }
-    g = f / r2;
-    const float bbg = 3.0f / (a * a) * lml;
-    if (rho <= 0.5f * a)
-      fp = bbg + 2.0f / (F.l2 * 0.0742478f) * (1.0f - 0.75f * lml) * bump_d(2.0f * rho / lam);
-    else
-      fp = bbg + 6.0f / (0.443991f * lam * a) * aml * bump_d(2.0f * (rho - n * a) / lam);
-  }
+// fixflux (intEV.cu:236-257, 333-357; intEVff.cu:194-250): nodes in
+// segment_fixflux below
+struct FixfluxProfile {
   static __device__ __forceinline__ float fp_scale(const FieldDev &) { return 1.0f; }
   static constexpr bool kHeavy = true;
 };
 template <>
-struct Profile<kFixflux> : FixfluxProfile<false> {};
+struct Profile<kFixflux> : FixfluxProfile {};
 template <>
-struct Profile<kFixfluxFF> : FixfluxProfile<true> {};
+struct Profile<kFixfluxFF> : FixfluxProfile {};
 
 // The fixflux profile with its Lentz continued fraction split out.  The
 // fraction (up to ~17 iterations of two divisions) is needed only where the
@@ -295,7 +241,7 @@ struct Profile<kFixfluxFF> : FixfluxProfile<true> {};
 // lane finishes its own nodes in the usual order.
 //
 // fixflux_cf: whether the node at r2 needs a fraction, and its argument
-// -1/(1 - x^2) (x as phi_d / chi_d compute it)
+// -1/(1 - x^2) (x as the phi and chi fits compute it, intEV.cu:161-198)
 template <bool FF>
 __device__ __forceinline__ bool fixflux_cf(float r2, const FieldDev &F, float &arg) {
   const float a = F.a;
@@ -313,8 +259,10 @@ __device__ __forceinline__ bool fixflux_cf(float r2, const FieldDev &F, float &a
   return true;
 }
 
-// FixfluxProfile::eval with the node's fraction value E given (used only
-// where fixflux_cf says the node needs it).  f is a called function and few
+// f / rho^2 and f' at rho^2 = r2 with the node's fraction value E given (used
+// only where fixflux_cf says the node needs it); phi, intEV.cu:161-174 /
+// intEVff.cu:147-157, chi, intEV.cu:176-198 (logistic fit) / intEVff.cu:159-176
+// (cosh-ratio fit), the bump, intEV.cu:151-159.  f is a called function and few
 // nodes are unrolled around it: its exponentials, sine and cosines are long,
 // and with eight inlined copies the warps of an SM waited for instructions 3.8
 // cycles per issue (64 instances on 512 x 512 points, spinor, 50 intervals:
@@ -384,9 +332,8 @@ constexpr int kFfBatch = 8;
 constexpr int kFfWarps = 4;  // warps per CTA of the kernels that call it (128 threads)
 
 // segment<> for the fixflux profiles (run-time interval count), with the
-// continued fractions gathered per warp; the same node values and sums as
-// segment<> evaluating FixfluxProfile<FF>::eval node by node.  Not inlined:
-// one copy for the dozen call sites of the sweep.
+// continued fractions gathered per warp; the sums of segment<> over the nodes
+// of fixflux_eval.  Not inlined: one copy for the dozen call sites of the sweep.
 template <bool FF, bool FERM>
 __device__ __noinline__ float2 segment_fixflux(float zix, float ziy, float zjx, float zjy,
                                                const FieldDev &F, float ph, float sp) {
