@@ -1,0 +1,250 @@
+/* The C-ABI runtime (csrc/wl_api.cpp) on the host alone: the CUDA runtime and
+ * the kernel launchers are replaced by stand-ins that record what the library
+ * asks for.  Asynchronous copies are carried out only when their stream is
+ * waited for -- the latest moment the CUDA runtime may read or write their host
+ * side -- and a host buffer that is rewritten or released before is reported.
+ * Usage: host_runtime <scenario>; prints "name value" lines. */
+#include <cuda_runtime.h>
+#include <math.h>
+#include <stdio.h>
+#include <stdlib.h>
+#include <string.h>
+#include <sys/mman.h>
+
+#include <new>
+#include <string>
+
+#include "wl_internal.h"
+#include "wl_legacy.h"
+#include "wlgpu.h"
+
+namespace {
+
+struct Block {
+  char *p;
+  size_t n;
+};
+struct Copy {
+  char *dst;
+  const char *src;
+  size_t n;
+  bool to_host;
+  unsigned char *seen;  // the source's contents when the copy was enqueued
+};
+constexpr int kMany = 4096;
+Block g_dev[kMany];
+int g_ndev = 0;
+Copy g_copy[kMany];
+int g_ncopy = 0;
+long g_released = 0, g_rewritten = 0, g_syncs = 0, g_kernels = 0;
+size_t g_bytes = 0, g_largest = 0;  // device memory held, the largest allocation
+bool g_report = true;
+wl::SweepArgs g_jobs[64];
+int g_sweeps_cut = 0;
+
+void run_copies() {
+  for (int i = 0; i < g_ncopy; ++i) {
+    Copy &c = g_copy[i];
+    if (!c.to_host && memcmp(c.seen, c.src, c.n)) ++g_rewritten;
+    memcpy(c.dst, c.src, c.n);
+    free(c.seen);
+  }
+  g_ncopy = 0;
+}
+void host_released(const void *p, size_t n) {
+  for (int i = 0; i < g_ncopy; ++i) {
+    const char *h = g_copy[i].to_host ? g_copy[i].dst : g_copy[i].src;
+    if (h >= (const char *)p && h < (const char *)p + n) ++g_released;
+  }
+}
+bool on_device(const void *p) {
+  for (int i = 0; i < g_ndev; ++i)
+    if ((const char *)p >= g_dev[i].p && (const char *)p < g_dev[i].p + g_dev[i].n) return true;
+  return false;
+}
+
+}  // namespace
+
+// every host buffer of the library comes from here: 16 bytes in front hold its size
+void *operator new(size_t n) {
+  char *p = (char *)malloc(n + 16);
+  if (!p) abort();
+  memcpy(p, &n, sizeof(n));
+  return p + 16;
+}
+void operator delete(void *q) noexcept {
+  if (!q) return;
+  char *p = (char *)q - 16;
+  size_t n;
+  memcpy(&n, p, sizeof(n));
+  host_released(q, n);
+  free(p);
+}
+void operator delete(void *q, size_t) noexcept { operator delete(q); }
+
+extern "C" {
+cudaError_t cudaGetDeviceCount(int *n) { return *n = 1, cudaSuccess; }
+cudaError_t cudaGetDevice(int *d) { return *d = 0, cudaSuccess; }
+cudaError_t cudaSetDevice(int) { return cudaSuccess; }
+cudaError_t cudaDeviceGetAttribute(int *v, cudaDeviceAttr, int) { return *v = 152, cudaSuccess; }
+cudaError_t cudaGetLastError(void) { return cudaSuccess; }
+const char *cudaGetErrorString(cudaError_t) { return "error"; }
+cudaError_t cudaGetDriverEntryPointByVersion(const char *, void **, unsigned int,
+                                             unsigned long long,
+                                             cudaDriverEntryPointQueryResult *) {
+  return cudaErrorNotSupported;
+}
+cudaError_t cudaMalloc(void **out, size_t n) {
+  *out = mmap(nullptr, n, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS | MAP_NORESERVE, -1, 0);
+  if (*out == MAP_FAILED || g_ndev == kMany) return cudaErrorMemoryAllocation;
+  g_dev[g_ndev++] = {(char *)*out, n};
+  g_bytes += n;
+  if (n > g_largest) g_largest = n;
+  return cudaSuccess;
+}
+cudaError_t cudaFree(void *p) {
+  run_copies();  // cudaFree waits for the device
+  for (int i = 0; i < g_ndev; ++i)
+    if (g_dev[i].p == p) {
+      g_bytes -= g_dev[i].n;
+      munmap(p, g_dev[i].n);
+      g_dev[i] = g_dev[--g_ndev];
+      break;
+    }
+  return cudaSuccess;
+}
+cudaError_t cudaPointerGetAttributes(cudaPointerAttributes *a, const void *p) {
+  memset(a, 0, sizeof(*a));
+  a->type = on_device(p) ? cudaMemoryTypeDevice : cudaMemoryTypeUnregistered;
+  return cudaSuccess;
+}
+cudaError_t cudaMemcpy(void *d, const void *s, size_t n, cudaMemcpyKind) {
+  run_copies();
+  memcpy(d, s, n);
+  return cudaSuccess;
+}
+cudaError_t cudaMemcpyAsync(void *d, const void *s, size_t n, cudaMemcpyKind k, cudaStream_t) {
+  if (g_ncopy == kMany) return cudaErrorUnknown;
+  Copy c = {(char *)d, (const char *)s, n, k == cudaMemcpyDeviceToHost, nullptr};
+  c.seen = (unsigned char *)malloc(n + 1);
+  memcpy(c.seen, s, n);
+  g_copy[g_ncopy++] = c;
+  return cudaSuccess;
+}
+cudaError_t cudaMemset(void *d, int v, size_t n) { return memset(d, v, n), cudaSuccess; }
+cudaError_t cudaMemsetAsync(void *d, int v, size_t n, cudaStream_t) {
+  return memset(d, v, n), cudaSuccess;
+}
+cudaError_t cudaStreamCreateWithFlags(cudaStream_t *s, unsigned) {
+  return *s = (cudaStream_t)0x10, cudaSuccess;
+}
+cudaError_t cudaStreamDestroy(cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaStreamSynchronize(cudaStream_t) { return run_copies(), ++g_syncs, cudaSuccess; }
+cudaError_t cudaStreamBeginCapture(cudaStream_t, cudaStreamCaptureMode) { return cudaSuccess; }
+cudaError_t cudaStreamEndCapture(cudaStream_t, cudaGraph_t *g) { return *g = nullptr, cudaSuccess; }
+cudaError_t cudaGraphInstantiate(cudaGraphExec_t *e, cudaGraph_t, unsigned long long) {
+  return *e = nullptr, cudaSuccess;
+}
+cudaError_t cudaGraphLaunch(cudaGraphExec_t, cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaGraphExecDestroy(cudaGraphExec_t) { return cudaSuccess; }
+cudaError_t cudaGraphDestroy(cudaGraph_t) { return cudaSuccess; }
+cudaError_t cudaEventCreate(cudaEvent_t *e) { return *e = (cudaEvent_t)0x20, cudaSuccess; }
+cudaError_t cudaEventDestroy(cudaEvent_t) { return cudaSuccess; }
+cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaEventSynchronize(cudaEvent_t) { return run_copies(), cudaSuccess; }
+cudaError_t cudaEventElapsedTime(float *ms, cudaEvent_t, cudaEvent_t) { return *ms = 1.0f, cudaSuccess; }
+}
+
+namespace wl {
+static cudaError_t kernels(int n) { return g_kernels += n, cudaSuccess; }
+cudaError_t launch_tint(const TintArgs &, cudaStream_t) { return kernels(1); }
+cudaError_t launch_batch(const BatchArgs &b, int, cudaStream_t) {
+  int n = 0;
+  for (int t = 0; t < b.ntiles; ++t)
+    if (b.tiles[t].job >= n) n = b.tiles[t].job + 1;
+  for (int j = 0; j < n && j < 64; ++j) g_jobs[j] = b.jobs[j];
+  return kernels(1);
+}
+cudaError_t launch_plain(int, bool, int, const LoopArgs &, int, cudaStream_t) { return kernels(1); }
+cudaError_t launch_sweep(int, bool, int, const SweepArgs &a, cudaStream_t) {
+  g_sweeps_cut += a.parts > 0;
+  return kernels(a.parts > 0 ? 2 : 1);  // a cut sweep adds its blocks in a second kernel
+}
+cudaError_t launch_vloops(uint64_t, int, int, int, float4 *, cudaStream_t) { return kernels(1); }
+bool batch_supports(int, int) { return true; }
+bool plain_supports(int k) { return light_profile(k) || k == kLattice; }
+bool batch_in_kernel(int k) { return light_profile(k) || k == kLattice; }
+int batch_max_ctas_per_sm() { return 4; }
+cudaError_t launch_loopwarp(int, bool, int, const LoopArgs &, cudaStream_t) { return kernels(1); }
+cudaError_t launch_list_mean(const double *, const int *, int, double *, cudaStream_t) { return kernels(1); }
+cudaError_t launch_loop_bbox(const float4 *, int, int, float4 *, cudaStream_t) { return kernels(1); }
+cudaError_t launch_peak_probe(int, int, int, int, float *, cudaStream_t) { return kernels(1); }
+cudaError_t launch_fingerprint(const float4 *, size_t, unsigned long long *, cudaStream_t) { return kernels(1); }
+cudaError_t launch_batch_reduce(const ReduceJob *, int, int, cudaStream_t) { return kernels(1); }
+cudaError_t launch_group_reduce(const ReduceShape &, double *, double *, double *, const int *,
+                                double *, cudaStream_t) {
+  return kernels(1);
+}
+cudaError_t launch_wait_selftest(int *, unsigned, int, cudaStream_t) { return kernels(1); }
+cudaError_t launch_instance_setup(const double *, const double *, const double *, int, int, float *,
+                                  int *, cudaStream_t) {
+  return kernels(1);
+}
+cudaError_t launch_order_instances(const float *, const float *, const float *, int, float, int *,
+                                   cudaStream_t) {
+  return kernels(1);
+}
+cudaError_t launch_group_list_means(const double *, int, int, double *, cudaStream_t) { return kernels(1); }
+}  // namespace wl
+
+// ------------------------------------------------------------ scenarios --
+static void say(const char *name, double v) { printf("%s %.17g\n", name, v); }
+static void need(int status, const char *what) {
+  if (status == WL_OK) return;
+  fprintf(stderr, "%s: status %d\n", what, status);
+  exit(2);
+}
+static wl_field field_of(int profile, int fermion, int nint) {
+  wl_field f;
+  memset(&f, 0, sizeof(f));
+  f.profile = profile;
+  f.fermion = fermion;
+  f.nint = nint;
+  f.mode = profile == WL_PROFILE_LATTICE ? WL_MODE_EXACT : WL_MODE_REFCOMPAT;
+  f.lambda2 = 0.5;
+  f.tubedist = 2.0;
+  f.lmin = 0.2;
+  f.rimage = 24.0;
+  return f;
+}
+static int ensemble(wl_ctx *c, int Nl, int ppl) {
+  int h = 0;
+  need(wl_ensemble_generate(c, 1, 0, Nl, ppl, &h), "generate");
+  return h;
+}
+
+// host buffers of the proper-time integral's copies
+static void tint_staging(wl_ctx *c) {
+  const int h = ensemble(c, 256, 64);
+  const wl_field f = field_of(WL_PROFILE_SMOOTH, 0, 4);
+  double rho[5], T[9], F[2] = {0.5, 1.0}, leff[10], err[10];
+  for (int i = 0; i < 5; ++i) rho[i] = 0.5 * i;
+  for (int k = 0; k < 9; ++k) T[k] = exp(0.3 * k);
+  for (int rep = 0; rep < 2; ++rep)
+    need(wl_tint(c, h, &f, 5, rho, 9, T, 2, F, 64, 2, leff, err, nullptr), "tint");
+  need(wl_effective_action(c, h, &f, 1.0, WL_TRULE_SUBST, 5, nullptr, 64, 3, leff, err, nullptr,
+                           nullptr),
+       "effective action");
+  say("released", (double)g_released);
+  say("rewritten", (double)g_rewritten);
+}
+
+int main(int argc, char **argv) {
+  const std::string s = argc > 1 ? argv[1] : "";
+  wl_ctx *c = nullptr;
+  need(wl_ctx_create(0, &c), "context");
+  if (s == "tint_staging") tint_staging(c);
+  else return 3;
+  wl_ctx_destroy(c);
+  return 0;
+}

@@ -1,0 +1,40 @@
+"""The C-ABI runtime on the host alone (tests/c/host_runtime.cpp): the CUDA
+runtime and the kernel launchers replaced by stand-ins that record what the
+library asks for.  Copies happen as late as the CUDA runtime may do them, so a
+host buffer that does not outlive its copy shows here and nowhere else."""
+import os
+import shutil
+import subprocess
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+PKG = os.path.join(ROOT, "worldline-flux-tube-lattice_gb300")
+
+
+@pytest.fixture(scope="module")
+def runtime(tmp_path_factory):
+    import build as pkg_build
+
+    cxx = shutil.which("g++")
+    if not cxx:
+        pytest.skip("no C++ compiler")
+    exe = str(tmp_path_factory.mktemp("host") / "host_runtime")
+    subprocess.run([cxx, "-std=c++17", "-O1", "-I" + os.path.join(PKG, "csrc"),
+                    "-I" + os.path.join(ROOT, "include"), "-I" + pkg_build.cuda_include(),
+                    os.path.join(PKG, "csrc", "wl_api.cpp"),
+                    os.path.join(PKG, "csrc", "wl_spline.cpp"),
+                    os.path.join(ROOT, "tests", "c", "host_runtime.cpp"), "-o", exe],
+                   check=True, capture_output=True, text=True)
+
+    def run(scenario):
+        r = subprocess.run([exe, scenario], capture_output=True, text=True, timeout=60)
+        assert r.returncode == 0, r.stderr
+        return {k: float(v) for k, v in (line.split() for line in r.stdout.splitlines())}
+
+    return run
+
+
+def test_proper_time_inputs_outlive_their_copy(runtime):
+    r = runtime("tint_staging")
+    assert r["released"] == 0 and r["rewritten"] == 0

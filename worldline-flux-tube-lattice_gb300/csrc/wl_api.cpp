@@ -83,7 +83,8 @@ struct wl_ctx {
   double last_batch_ms = 0.0;
   int last_batch_tiles = 0, last_batch_grid = 0;
   std::vector<float> h_inst;
-  bool staged = false;        // h_inst may still be read by its copy
+  std::vector<double> h_aux;  // proper-time integral: rho | T | w | F
+  bool staged = false;        // h_inst or h_aux may still be read by its copy
   std::vector<double> h_out;  // small results on their way to the caller
   std::string err;
   int last_launches = 0;
@@ -317,7 +318,7 @@ int upload_instances(wl_ctx *ctx, int ninst, const double *cx, const double *cy,
   }
   WL_CHECK(ctx, ctx->inst.reserve((size_t)na * ninst));
   // the launches that follow need no wait; the call's results are awaited before
-  // the vector is refilled
+  // the vector (and tint_run's) is refilled
   ctx->staged = true;
   WL_CHECK(ctx, cudaMemcpyAsync(ctx->inst.p, h, sizeof(float) * na * ninst,
                                 cudaMemcpyHostToDevice, ctx->stream));
@@ -1285,7 +1286,8 @@ static int tint_run(wl_ctx *ctx, int handle, const wl_field *field, int nrho,
     cudaGetLastError();
     return fail(ctx, WL_ERR_NOMEM, "cannot allocate the proper-time buffers");
   }
-  std::vector<double> h((size_t)nrho + 2 * (size_t)nT + nF);
+  std::vector<double> &h = ctx->h_aux;  // outlives its copy, as h_inst does
+  h.resize((size_t)nrho + 2 * (size_t)nT + nF);
   memcpy(h.data(), host_rho, sizeof(double) * nrho);
   memcpy(h.data() + nrho, host_T, sizeof(double) * nT);
   memcpy(h.data() + nrho + nT, host_w, sizeof(double) * nT);
