@@ -239,11 +239,39 @@ static void tint_staging(wl_ctx *c) {
   say("rewritten", (double)g_rewritten);
 }
 
+// waits of the stream per EV() sweep and per wl_loops() call
+static void loop_waits(wl_ctx *c) {
+  const int Nl = 256, ppl = 64, h = ensemble(c, Nl, ppl);
+  const wl_field f = field_of(WL_PROFILE_SMOOTH, 0, 50);
+  const float *loops = nullptr;
+  need(wl_ensemble_info(c, h, &loops, nullptr, nullptr), "info");
+  struct Wparams p;
+  memset(&p, 0, sizeof(p));
+  p.Nl = Nl;
+  p.Nppl = ppl;
+  p.F = 1.0;
+  p.l2 = 0.5;
+  p.ng = Nl / 128;
+  p.worldlines = (float4 *)loops;
+  cudaMalloc((void **)&p.Wsscal_d, sizeof(float4) * Nl);
+  int list[128];
+  for (int j = 0; j < 128; ++j) list[j] = j;
+  EV(0.5, &p, list);  // the first call makes the context
+  long before = g_syncs;
+  for (int k = 0; k < 10; ++k) EV(1.0 + k, &p, list);
+  say("ev", (double)(g_syncs - before) / 10);
+  before = g_syncs;
+  for (int k = 0; k < 10; ++k) need(wl_loops(c, h, &f, 0.1, 0, 1.0 + k, 1.0, nullptr, nullptr), "loops");
+  say("loops", (double)(g_syncs - before) / 10);
+  say("rewritten", (double)g_rewritten);
+}
+
 int main(int argc, char **argv) {
   const std::string s = argc > 1 ? argv[1] : "";
   wl_ctx *c = nullptr;
   need(wl_ctx_create(0, &c), "context");
   if (s == "tint_staging") tint_staging(c);
+  else if (s == "loop_waits") loop_waits(c);
   else return 3;
   wl_ctx_destroy(c);
   return 0;

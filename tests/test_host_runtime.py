@@ -38,3 +38,8 @@ def runtime(tmp_path_factory):
 def test_proper_time_inputs_outlive_their_copy(runtime):
     r = runtime("tint_staging")
     assert r["released"] == 0 and r["rewritten"] == 0
+
+
+def test_one_wait_per_sweep_of_the_loop_parallel_calls(runtime):
+    r = runtime("loop_waits")
+    assert r["ev"] == 1 and r["loops"] == 1 and r["rewritten"] == 0

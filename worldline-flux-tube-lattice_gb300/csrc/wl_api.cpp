@@ -1640,6 +1640,7 @@ int wl_loops(wl_ctx *ctx, int handle, const wl_field *field, double cx, double c
     WL_CHECK(ctx, cudaMemcpyAsync(host_ferm, df, sizeof(float4) * e.Nl, cudaMemcpyDeviceToHost,
                                   ctx->stream));
   WL_CHECK(ctx, cudaStreamSynchronize(ctx->stream));
+  ctx->staged = false;
   return WL_OK;
 }
 
@@ -1806,6 +1807,7 @@ double EV(double T, void *p, int *WLlist) {
                            cudaMemcpyDeviceToHost, ctx->stream);
     if (ce == cudaSuccess) ce = cudaStreamSynchronize(ctx->stream);
     if (ce != cudaSuccess) return legacy_fail(cudaGetErrorString(ce));
+    ctx->staged = false;
     unsigned long long fp;
     memcpy(&fp, &L.gev[(size_t)ngrp], sizeof(fp));
     L.gev.resize((size_t)ngrp);
