@@ -278,8 +278,9 @@ int wl_ctx_stream(wl_ctx *ctx, void **stream);
 int wl_loops(wl_ctx *ctx, int handle, const wl_field *field, double cx, double cy,
              double T, double F, float *host_scal, float *host_ferm);
 
-/* How the last wl_eval on this context was run: kernel launches issued and
- * which sweep kernel ("instance-parallel" or "loop-parallel"). */
+/* How the last call on this context was run: kernel launches issued (without
+ * what an ensemble needs once, its loops' bounding boxes) and which sweep kernel
+ * ("instance-parallel" or "loop-parallel"). */
 int wl_last_launches(wl_ctx *ctx, int *launches, const char **sweep_kind);
 
 /* ---- uneven batches in one persistent launch ---------------------------- */

@@ -266,12 +266,68 @@ static void loop_waits(wl_ctx *c) {
   say("rewritten", (double)g_rewritten);
 }
 
+// wl_last_launches() against the kernels that were enqueued
+static void launches(wl_ctx *c) {
+  static double cx[64], cy[64], T[64], out[4096];
+  for (int i = 0; i < 64; ++i) cx[i] = 0.05 * i, T[i] = 0.1 + 0.1 * i;
+  const double F[1] = {1.0}, rho[2] = {0.1, 0.5};
+  double *dev = nullptr;
+  cudaMalloc((void **)&dev, sizeof(double) * 64);
+  for (int i = 0; i < 64; ++i) dev[i] = T[i];
+  const int h = ensemble(c, 256, 512);
+  int worst = 0;
+  long before;
+  auto count = [&](int status, const char *what) {
+    need(status, what);
+    int n = -1;
+    wl_last_launches(c, &n, nullptr);
+    const int off = abs(n - (int)(g_kernels - before));
+    if (off > worst) worst = off;
+    before = g_kernels;
+  };
+  const int profiles[] = {WL_PROFILE_SMOOTH, WL_PROFILE_LATTICE, WL_PROFILE_FIXFLUX,
+                          WL_PROFILE_PERIODIC, WL_PROFILE_SPLINE};
+  for (int p : profiles) {
+    const wl_field f = field_of(p, 0, 4);
+    // first use: the lattice's boxes and the spline's table
+    need(wl_eval(c, h, &f, 1, cx, cy, T, 1, F, 128, nullptr, out, nullptr), "eval");
+    before = g_kernels;
+    for (int n : {1, 40})
+      count(wl_eval(c, h, &f, n, cx, cy, T, 1, F, 128, nullptr, out, nullptr), "eval");
+    count(wl_eval_device(c, h, &f, 40, dev, dev, dev, 1, F, 128, nullptr, nullptr, nullptr),
+          "eval_device");
+    count(wl_tint(c, h, &f, 2, rho, 2 * 16 + 1, [] {
+            static double t[33];
+            for (int k = 0; k < 33; ++k) t[k] = exp(0.1 * k);
+            return t;
+          }(), 1, F, 128, 2, out, out + 2, nullptr), "tint");
+    wl_job J[2];
+    memset(J, 0, sizeof(J));
+    for (wl_job &j : J) {
+      j.handle = h;
+      j.ninst = 40;
+      j.cx = cx;
+      j.cy = cy;
+      j.T = T;
+      j.nF = 1;
+      j.F[0] = 1.0;
+      j.group = 128;
+      j.field = f;
+    }
+    J[1].field = field_of(WL_PROFILE_SMOOTH, 1, 4);
+    count(wl_batch_eval(c, 2, J, 0), "batch");
+  }
+  say("cut", (double)g_sweeps_cut);  // the heavy profiles did take the cut path
+  say("off", (double)worst);
+}
+
 int main(int argc, char **argv) {
   const std::string s = argc > 1 ? argv[1] : "";
   wl_ctx *c = nullptr;
   need(wl_ctx_create(0, &c), "context");
   if (s == "tint_staging") tint_staging(c);
   else if (s == "loop_waits") loop_waits(c);
+  else if (s == "launches") launches(c);
   else return 3;
   wl_ctx_destroy(c);
   return 0;

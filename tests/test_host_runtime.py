@@ -43,3 +43,8 @@ def test_proper_time_inputs_outlive_their_copy(runtime):
 def test_one_wait_per_sweep_of_the_loop_parallel_calls(runtime):
     r = runtime("loop_waits")
     assert r["ev"] == 1 and r["loops"] == 1 and r["rewritten"] == 0
+
+
+def test_reported_launches_are_the_kernels_enqueued(runtime):
+    r = runtime("launches")
+    assert r["cut"] > 0 and r["off"] == 0

@@ -651,8 +651,10 @@ int batch_run(wl_ctx *ctx, int njobs, const wl_job *jobs, int flags, int points,
   int grid = per_sm * ctx->num_sms;
   if (grid > B.ntiles) grid = B.ntiles;
   const wl::ReduceJob *rjd = (const wl::ReduceJob *)(meta + off_rj);
-  // kernels per run: the persistent kernel, the side sweeps, the reduction
-  const int launches = (B.ntiles > 0 ? 1 : 0) + (int)P.side.size() + 1;
+  // the lattice jobs' instance orders, the persistent kernel, the side sweeps,
+  // the reduction
+  int launches = (B.ntiles > 0 ? 1 : 0) + (int)P.side.size() + 1;
+  for (int i = 0; i < njobs; ++i) launches += P.jobs[i].perm != nullptr;
 
   cudaEvent_t e0, e1;
   WL_CHECK(ctx, cudaEventCreate(&e0));
@@ -955,7 +957,7 @@ static int eval_prologue(wl_ctx *ctx, int handle, const wl_field *field, int nin
 
 // Sweep + reduction on the context stream; instances are already staged in
 // ctx->inst as [cx | cy | rtT | tq].  Outputs are device pointers (may be
-// NULL).  Returns after enqueueing.
+// NULL).  Returns after enqueueing, its kernels counted in last_launches.
 static int run_eval(wl_ctx *ctx, const Ensemble &e, int kprof, const FieldDev &fd,
                     const float4 *bbox, const wl_field *field, int ninst, int nF,
                     const double *host_F, int group, double *dg, double *dm, double *ds,
@@ -963,6 +965,7 @@ static int run_eval(wl_ctx *ctx, const Ensemble &e, int kprof, const FieldDev &f
   const bool fermion = field->fermion != 0;
   const int nint = field->nint;
   const bool use_sweep = ninst >= 32;
+  ctx->last_launches = 0;
   if (kprof == wl::kSpline && (!fd.sp_rho2 || !fd.sp_coef))
     return fail(ctx, WL_ERR_INVALID, "spline profile without its table");
   int n_chunks, cpg;
@@ -1026,8 +1029,10 @@ static int run_eval(wl_ctx *ctx, const Ensemble &e, int kprof, const FieldDev &f
       WL_CHECK(ctx, wl::launch_order_instances(a.cx, a.cy, a.rtT, ninst, 1.0f / fd.a,
                                                ctx->perm.p, ctx->stream));
       a.perm = ctx->perm.p;
+      ctx->last_launches += 1;
     }
     WL_CHECK(ctx, wl::launch_sweep(kprof, fermion, nint, a, ctx->stream));
+    ctx->last_launches += a.parts ? 2 : 1;  // a cut sweep adds its blocks in a second kernel
     ctx->last_kind = "instance-parallel";
   } else {
     wl::LoopArgs b;
@@ -1047,11 +1052,13 @@ static int run_eval(wl_ctx *ctx, const Ensemble &e, int kprof, const FieldDev &f
     b.partial = ctx->partial.p;
     b.bbox = bbox;
     WL_CHECK(ctx, wl::launch_loopwarp(kprof, fermion, nint, b, ctx->stream));
+    ctx->last_launches += 1;
     ctx->last_kind = "loop-parallel";
   }
   const wl::ReduceShape rs = {ctx->partial.p, n_chunks, cpg, inner, group, ninst, nF};
   WL_CHECK(ctx, wl::launch_group_reduce(rs, dg, dm, ds, status_out ? ctx->status.p : nullptr,
                                         status_out, ctx->stream));
+  ctx->last_launches += 1;
   return WL_OK;
 }
 
@@ -1079,7 +1086,6 @@ int wl_eval(wl_ctx *ctx, int handle, const wl_field *field, int ninst, const dou
   if ((r = run_eval(ctx, e, kprof, fd, bb, field, ninst, nF, host_F, group, dg, dm, ds,
                     dg + nout)))
     return r;
-  ctx->last_launches = 2;
   const size_t nm = (size_t)ninst * nF;
   return read_results(ctx, dg, nout, {{out_group, nm * ng}, {out_mean, nm}, {out_sem, nm}});
 }
@@ -1115,7 +1121,7 @@ int wl_eval_device(wl_ctx *ctx, int handle, const wl_field *field, int ninst,
   if ((r = run_eval(ctx, e, kprof, fd, bb, field, ninst, nF, host_F, group, dev_out_group,
                     dev_out_mean, dev_out_sem, nullptr)))
     return r;
-  ctx->last_launches = 3;
+  ctx->last_launches += 1;  // the instance setup
   return WL_OK;
 }
 
@@ -1323,7 +1329,7 @@ static int tint_run(wl_ctx *ctx, int handle, const wl_field *field, int nrho,
   ta.m2 = 1.0;         // Integrand.c:12
   ta.e = 0.30282212;   // Integrand.c:14
   WL_CHECK(ctx, wl::launch_tint(ta, ctx->stream));
-  ctx->last_launches = 3;  // sweep, reduction, proper-time integral
+  ctx->last_launches += 1;
   return WL_OK;
 }
 
