@@ -321,6 +321,37 @@ static void launches(wl_ctx *c) {
   say("off", (double)worst);
 }
 
+static wl_job job_of(int h, const wl_field &f, int n, int nF, const double *v, const double *T) {
+  wl_job j;
+  memset(&j, 0, sizeof(j));
+  j.handle = h;
+  j.field = f;
+  j.ninst = n;
+  j.cx = j.cy = v;
+  j.T = T;
+  j.nF = nF;
+  for (int k = 0; k < nF; ++k) j.F[k] = 0.5;
+  j.group = 128;
+  return j;
+}
+
+// device memory of a batch whose chunks are whole groups (ppl 64, groups of
+// 128), just under the number of units at which jobs stop being cut
+static void batch_scratch(wl_ctx *c) {
+  const int n = 31100, Nl = 5120, h = ensemble(c, Nl, 64);
+  double *v = new double[n], *T = new double[n];
+  for (int i = 0; i < n; ++i) v[i] = 0.1, T[i] = 1.0;
+  g_largest = 0;
+  wl_job j = job_of(h, field_of(WL_PROFILE_GAUSSIAN, 1, 50), n, 4, v, T);
+  need(wl_batch_eval(c, 1, &j, 0), "batch");
+  say("largest", (double)g_largest);
+  say("chunk_sums", 8.0 * Nl / 128 * 4 * 3 * n);
+  // small jobs are still cut into single loops
+  wl_job k = job_of(h, field_of(WL_PROFILE_SMOOTH, 1, 50), 40, 1, v, T);
+  need(wl_batch_eval(c, 1, &k, 0), "batch");
+  say("small_per_loop", g_jobs[0].per_loop);
+}
+
 int main(int argc, char **argv) {
   const std::string s = argc > 1 ? argv[1] : "";
   wl_ctx *c = nullptr;
@@ -328,6 +359,7 @@ int main(int argc, char **argv) {
   if (s == "tint_staging") tint_staging(c);
   else if (s == "loop_waits") loop_waits(c);
   else if (s == "launches") launches(c);
+  else if (s == "batch_scratch") batch_scratch(c);
   else return 3;
   wl_ctx_destroy(c);
   return 0;

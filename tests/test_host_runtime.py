@@ -48,3 +48,9 @@ def test_one_wait_per_sweep_of_the_loop_parallel_calls(runtime):
 def test_reported_launches_are_the_kernels_enqueued(runtime):
     r = runtime("launches")
     assert r["cut"] > 0 and r["off"] == 0
+
+
+def test_batch_scratch_is_bounded(runtime):
+    r = runtime("batch_scratch")
+    assert r["largest"] <= r["chunk_sums"] + 256 * 2 ** 20
+    assert r["small_per_loop"] == 1

@@ -441,6 +441,12 @@ int batch_loops_per_tile(int points_per_tile, int ppl, int group) {
   return lc;
 }
 
+// Partial sums that a batch may store loop by loop (doubles, 256 MB): a chunk
+// holds up to a whole group here, so that the 16 waves of units below which
+// sweep_units cuts it would be 3.8 GB per flux value at groups of 128 loops.
+// The jobs past the bound keep their chunks.
+constexpr size_t kMaxLoopSums = (size_t)32 << 20;
+
 struct BatchPlan {
   size_t perm_total = 0;  // lattice jobs' instance orders
   std::vector<wl::SweepArgs> jobs;
@@ -449,7 +455,7 @@ struct BatchPlan {
   std::vector<wl::ReduceJob> rjobs;
   std::vector<float> inst;
   size_t part_total = 0, out_total = 0;
-  bool split = false;  // some job's partial sums are stored loop by loop
+  size_t split_total = 0;  // of them, sums stored loop by loop instead of by chunk
   int reduce_blocks = 0;
 };
 
@@ -484,18 +490,18 @@ int batch_plan(wl_ctx *ctx, int njobs, const wl_job *jobs, int points, bool may_
     P->out_total += (size_t)J.ninst * J.nF * (e.Nl / J.group + 2);
   }
   // units over the whole launch (a heavy profile's own launch follows it)
-  P->split = false;
+  P->split_total = 0;
   for (int i = 0; i < njobs; ++i) {
     const wl_job &J = jobs[i];
+    const size_t loop_sums = (size_t)cut[i].n_chunks * lcs[i] * J.nF * 3 * J.ninst;
     wl::sweep_units(cut[i], kprofs[i], J.field.fermion != 0, J.field.nint,
-                    !may_split ? wl::kNoSplit
+                    !may_split || P->split_total + loop_sums > kMaxLoopSums ? wl::kNoSplit
                     : wl::batch_in_kernel(kprofs[i])
                         ? items
                         : wl::sweep_chunk_items(cut[i], kprofs[i], J.field.nint));
-    const int rows = cut[i].n_chunks * (cut[i].per_loop ? lcs[i] : 1);
-    P->split |= cut[i].per_loop && lcs[i] > 1;
+    if (cut[i].per_loop && lcs[i] > 1) P->split_total += loop_sums;
     part_off[i] = P->part_total;
-    P->part_total += (size_t)rows * J.nF * 3 * J.ninst;
+    P->part_total += cut[i].per_loop ? loop_sums : loop_sums / lcs[i];
   }
   P->inst.resize(inst_total);
   P->jobs.resize(njobs);
@@ -584,7 +590,7 @@ int batch_run(wl_ctx *ctx, int njobs, const wl_job *jobs, int flags, int points,
   BatchPlan P;
   int r = batch_plan(ctx, njobs, jobs, points, true, &P);
   if (r) return r;
-  if (P.split && ctx->b_part.reserve(P.part_total) != cudaSuccess) {
+  if (P.split_total && ctx->b_part.reserve(P.part_total) != cudaSuccess) {
     cudaGetLastError();  // loop by loop needs more memory than whole chunks
     P = BatchPlan();
     if ((r = batch_plan(ctx, njobs, jobs, points, false, &P))) return r;

@@ -110,7 +110,7 @@ inline double sweep_chunk_items(const SweepArgs &a, int kprof, int nint) {
 // bytes of HBM traffic per (loop, instance), 6 nF / ppl of the time of its ppl
 // segments at the measured rates (8.5e11 segments/s of weight 1, 6.8 TB/s).
 // Above 16 waves the partial sums would also outgrow the gain (0.24 GB per flux
-// value).  Measured: 96 instances x 3 fluxes on 5120 x 2048 points (1 wave)
+// value at wl_eval's 8 loops per chunk; a batch's larger chunks: batch_plan).  Measured: 96 instances x 3 fluxes on 5120 x 2048 points (1 wave)
 // 1.20 ms against 3.14 ms in 128-thread tiles of 256 instances.
 inline void sweep_units(SweepArgs &a, int kprof, int fermion, int nint, double items) {
   const int loops = a.n_chunks * a.chunk_loops, unit = sweep_loop_pairs(kprof, nint) ? 2 : 1;
