@@ -352,6 +352,19 @@ static void batch_scratch(wl_ctx *c) {
   say("small_per_loop", g_jobs[0].per_loop);
 }
 
+// a light job's cut, alone and beside a heavy job that runs in a launch of its own
+static void batch_side(wl_ctx *c) {
+  const int n = 4000, Nl = 5120, h = ensemble(c, Nl, 4096), h2 = ensemble(c, 1024, 1024);
+  double *v = new double[n], *T = new double[n];
+  for (int i = 0; i < n; ++i) v[i] = 0.1, T[i] = 1.0;
+  wl_job j[2] = {job_of(h2, field_of(WL_PROFILE_SMOOTH, 0, 4), 300, 1, v, T),
+                 job_of(h, field_of(WL_PROFILE_FIXFLUX, 0, 50), n, 1, v, T)};
+  for (int k = 1; k <= 2; ++k) {
+    need(wl_batch_eval(c, k, j, 0), "batch");
+    say(k == 1 ? "alone" : "beside", g_jobs[0].per_loop);
+  }
+}
+
 int main(int argc, char **argv) {
   const std::string s = argc > 1 ? argv[1] : "";
   wl_ctx *c = nullptr;
@@ -360,6 +373,7 @@ int main(int argc, char **argv) {
   else if (s == "loop_waits") loop_waits(c);
   else if (s == "launches") launches(c);
   else if (s == "batch_scratch") batch_scratch(c);
+  else if (s == "batch_side") batch_side(c);
   else return 3;
   wl_ctx_destroy(c);
   return 0;

@@ -54,3 +54,8 @@ def test_batch_scratch_is_bounded(runtime):
     r = runtime("batch_scratch")
     assert r["largest"] <= r["chunk_sums"] + 256 * 2 ** 20
     assert r["small_per_loop"] == 1
+
+
+def test_heavy_jobs_do_not_decide_the_cut_of_the_others(runtime):
+    r = runtime("batch_side")
+    assert r["alone"] == 1 and r["beside"] == 1

@@ -485,11 +485,13 @@ int batch_plan(wl_ctx *ctx, int njobs, const wl_job *jobs, int points, bool may_
     cut[i].ppl = e.ppl;
     cut[i].chunk_loops = lcs[i];
     cut[i].n_chunks = e.Nl / lcs[i];
-    items += wl::sweep_chunk_items(cut[i], kprofs[i], J.field.nint);
+    if (wl::batch_in_kernel(kprofs[i]))  // of the persistent launch
+      items += wl::sweep_chunk_items(cut[i], kprofs[i], J.field.nint);
     out_off[i] = P->out_total;
     P->out_total += (size_t)J.ninst * J.nF * (e.Nl / J.group + 2);
   }
-  // units over the whole launch (a heavy profile's own launch follows it)
+  // units over the whole launch (a heavy profile's own launch follows it and
+  // counts by itself)
   P->split_total = 0;
   for (int i = 0; i < njobs; ++i) {
     const wl_job &J = jobs[i];
