@@ -417,7 +417,8 @@ int wl_server_destroy(wl_server *srv);
 /* ---- legacy EV() configuration ----------------------------------------- */
 /* The reference selects the profile at compile time (intT.h "profile"); the
  * library's EV() uses the profile, lattice spacing, Simpson intervals and
- * clamp mode set here (default: smooth, a = 1, 50 intervals, ref-compat).   */
+ * clamp mode set here (default: smooth, a = 1, 50 intervals, ref-compat).
+ * The square lattice is wl_eval's alone: EV() returns NaN for it.           */
 int wl_legacy_configure(int profile, double tubedist, double lmin, int nint,
                         int mode);
 /* the configuration EV() uses (any pointer may be NULL) */

@@ -365,6 +365,28 @@ static void batch_side(wl_ctx *c) {
   }
 }
 
+// EV() configured for the lattice: launches nothing, returns NaN
+static void ev_lattice(wl_ctx *c) {
+  const int Nl = 128, ppl = 64, h = ensemble(c, Nl, ppl);
+  const float *loops = nullptr;
+  need(wl_ensemble_info(c, h, &loops, nullptr, nullptr), "info");
+  need(wl_legacy_configure(WL_PROFILE_LATTICE, 2.0, 0.1, 4, WL_MODE_EXACT), "configure");
+  struct Wparams p;
+  memset(&p, 0, sizeof(p));
+  p.Nl = Nl;
+  p.Nppl = ppl;
+  p.F = 1.0;
+  p.l2 = 0.5;
+  p.ng = 1;
+  p.worldlines = (float4 *)loops;
+  cudaMalloc((void **)&p.Wsscal_d, sizeof(float4) * Nl);
+  int list[128];
+  for (int j = 0; j < 128; ++j) list[j] = j;
+  const long before = g_kernels;
+  say("nan", isnan(EV(0.5, &p, list)));
+  say("kernels", (double)(g_kernels - before));
+}
+
 int main(int argc, char **argv) {
   const std::string s = argc > 1 ? argv[1] : "";
   wl_ctx *c = nullptr;
@@ -374,6 +396,7 @@ int main(int argc, char **argv) {
   else if (s == "launches") launches(c);
   else if (s == "batch_scratch") batch_scratch(c);
   else if (s == "batch_side") batch_side(c);
+  else if (s == "ev_lattice") ev_lattice(c);
   else return 3;
   wl_ctx_destroy(c);
   return 0;

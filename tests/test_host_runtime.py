@@ -59,3 +59,9 @@ def test_batch_scratch_is_bounded(runtime):
 def test_heavy_jobs_do_not_decide_the_cut_of_the_others(runtime):
     r = runtime("batch_side")
     assert r["alone"] == 1 and r["beside"] == 1
+
+
+def test_ev_launches_nothing_for_the_lattice(runtime):
+    """The legacy call holds no bounding boxes, which the lattice's kernels read."""
+    r = runtime("ev_lattice")
+    assert r["nan"] == 1 and r["kernels"] == 0

@@ -1746,6 +1746,8 @@ double EV(double T, void *p, int *WLlist) {
   int kprof;
   FieldDev fd;
   if (field_to_dev(ctx, &f, &kprof, &fd)) return legacy_fail(ctx->err.c_str());
+  if (kprof == wl::kLattice)  // its images need the ensemble's bounding boxes
+    return legacy_fail("the lattice profile is evaluated by wl_eval, not by EV()");
   if (kprof == wl::kSpline && ensure_spline(ctx, &f, &fd)) return legacy_fail(ctx->err.c_str());
   const size_t npts = (size_t)params.Nl * params.Nppl;
   bool hit = L.valid && L.T == T && L.F == params.F && L.l2 == params.l2 &&
