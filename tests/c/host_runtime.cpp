@@ -387,6 +387,19 @@ static void ev_lattice(wl_ctx *c) {
   say("kernels", (double)(g_kernels - before));
 }
 
+// every launch the host lets through has its last warp's unit index in 32 bits
+static void sweep_grid() {
+  bool ok = wl::sweep_ctas(1) == 1 && wl::sweep_ctas(4) == 1 && wl::sweep_ctas(5) == 2;
+  for (int b = 3; b < 62; ++b)
+    for (int d = -1; d <= 1; ++d) {
+      const long long items = (1ll << b) + d;
+      const unsigned ctas = wl::sweep_ctas(items);
+      if (items <= 1ll << 32) ok &= (long long)ctas * wl::kSweepWarps >= items;
+      ok &= (unsigned long long)ctas * wl::kSweepWarps <= 1ull << 32;
+    }
+  say("ok", ok);
+}
+
 int main(int argc, char **argv) {
   const std::string s = argc > 1 ? argv[1] : "";
   wl_ctx *c = nullptr;
@@ -397,6 +410,7 @@ int main(int argc, char **argv) {
   else if (s == "batch_scratch") batch_scratch(c);
   else if (s == "batch_side") batch_side(c);
   else if (s == "ev_lattice") ev_lattice(c);
+  else if (s == "sweep_grid") sweep_grid();
   else return 3;
   wl_ctx_destroy(c);
   return 0;

@@ -65,3 +65,7 @@ def test_ev_launches_nothing_for_the_lattice(runtime):
     """The legacy call holds no bounding boxes, which the lattice's kernels read."""
     r = runtime("ev_lattice")
     assert r["nan"] == 1 and r["kernels"] == 0
+
+
+def test_sweep_grids_keep_the_unit_index_in_32_bits(runtime):
+    assert runtime("sweep_grid")["ok"] == 1

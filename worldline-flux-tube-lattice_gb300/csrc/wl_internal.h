@@ -95,6 +95,13 @@ inline double profile_weight(int kprof, int fermion, int nint) {
   return (fermion ? w * 1.15 : w) * (nint + 1) / 5.0;
 }
 
+// CTAs of a sweep of so many warp units (0: too many; a warp finds its unit as
+// blockIdx.x * kSweepWarps + warp in 32 bits)
+inline unsigned sweep_ctas(long long items) {
+  const long long ctas = (items + kSweepWarps - 1) / kSweepWarps;
+  return ctas > (1ll << 32) / kSweepWarps ? 0u : (unsigned)ctas;
+}
+
 // warp units of a sweep by whole chunks
 inline double sweep_chunk_items(const SweepArgs &a, int kprof, int nint) {
   const int per = warp_instances(kprof, nint);

@@ -1094,8 +1094,8 @@ cudaError_t sweep_launch(SweepArgs a, cudaStream_t s) {
   const int per = kLat4 ? 64 : 32;
   a.n_tiles = (a.ninst + per - 1) / per;
   const long long items = (long long)a.n_tiles * a.n_units;
-  const long long ctas = (items + kSweepWarps - 1) / kSweepWarps;
-  if (ctas > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
+  const unsigned ctas = sweep_ctas(items);
+  if (!ctas) return cudaErrorInvalidConfiguration;
   constexpr size_t smem = kLat4 ? sweep_lat_smem_bytes() : sweep_smem_bytes();
   auto k = sweep_kernel<P, FERM, NINT, PAIR>;
   if (smem > 48 * 1024) {  // a per-device attribute
@@ -1103,7 +1103,7 @@ cudaError_t sweep_launch(SweepArgs a, cudaStream_t s) {
         cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
   }
-  k<<<(unsigned)ctas, kSweepThreads, smem, s>>>(a);
+  k<<<ctas, kSweepThreads, smem, s>>>(a);
   return cudaGetLastError();
 }
 
@@ -1112,8 +1112,9 @@ cudaError_t sweep_parts_launch(SweepArgs a, cudaStream_t s) {
   a.n_tiles = (a.ninst + 31) / 32;
   const long long loops = (long long)a.n_chunks * a.chunk_loops;
   const long long items = loops * a.parts * a.n_tiles;
-  sweep_part_kernel<P, FERM><<<(unsigned)((items + kSweepWarps - 1) / kSweepWarps), kSweepThreads,
-                               sweep_smem_bytes(), s>>>(a);
+  const unsigned ctas = sweep_ctas(items);
+  if (!ctas) return cudaErrorInvalidConfiguration;
+  sweep_part_kernel<P, FERM><<<ctas, kSweepThreads, sweep_smem_bytes(), s>>>(a);
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   loop_finish_kernel<P, FERM><<<(unsigned)((loops * a.ninst + 127) / 128), 128, 0, s>>>(a);
