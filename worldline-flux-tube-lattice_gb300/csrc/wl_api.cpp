@@ -981,7 +981,8 @@ static int run_eval(wl_ctx *ctx, const Ensemble &e, int kprof, const FieldDev &f
     const int lc = plan_chunk(group);
     n_chunks = e.Nl / lc;
     if (n_chunks > 65535)
-      return fail(ctx, WL_ERR_INVALID, "group %d too small for Nl = %d (grid limit)", group, e.Nl);
+      return fail(ctx, WL_ERR_INVALID, "group %d too small for Nl = %d (more than 65535 sums)", group,
+                  e.Nl);
     cpg = group / lc;
   } else {
     n_chunks = e.Nl;
