@@ -400,6 +400,29 @@ static void sweep_grid() {
   say("ok", ok);
 }
 
+// smooth_clamp_idle(): where it says so, lambda^2 + max(a, clamp) and lambda^2 + a
+// are the same float for every a below the clamp; elsewhere they differ somewhere
+static void clamp_idle() {
+  int wrong = 0, idle = 0;
+  const float widths[] = {1e-7f, 0.01f, 0.2f, 0.24999999f, 0.25f, 0.3f, 0.49999997f, 0.5f, 1.0f, 300.0f};
+  for (float l2 : widths)
+    for (float clamp : {1e-8f, 1e-30f, -INFINITY}) {
+      wl::FieldDev f;
+      memset(&f, 0, sizeof(f));
+      f.l2 = l2;
+      f.clampA = clamp;
+      bool same = true;
+      for (float a = 0.0f; clamp > 0.0f && a <= clamp; a = a * 1.01f + 1e-44f) {
+        volatile float x = l2 + fmaxf(a, clamp), y = l2 + a;
+        same &= x == y;
+      }
+      wrong += same != wl::smooth_clamp_idle(f);
+      idle += same;
+    }
+  say("wrong", wrong);
+  say("idle", idle);
+}
+
 int main(int argc, char **argv) {
   const std::string s = argc > 1 ? argv[1] : "";
   wl_ctx *c = nullptr;
@@ -411,6 +434,7 @@ int main(int argc, char **argv) {
   else if (s == "batch_side") batch_side(c);
   else if (s == "ev_lattice") ev_lattice(c);
   else if (s == "sweep_grid") sweep_grid();
+  else if (s == "clamp_idle") clamp_idle();
   else return 3;
   wl_ctx_destroy(c);
   return 0;

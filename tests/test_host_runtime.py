@@ -69,3 +69,9 @@ def test_ev_launches_nothing_for_the_lattice(runtime):
 
 def test_sweep_grids_keep_the_unit_index_in_32_bits(runtime):
     assert runtime("sweep_grid")["ok"] == 1
+
+
+def test_the_clamp_is_left_out_only_where_it_changes_no_bit(runtime):
+    """smooth_clamp_idle() itself, against float32 sums over |z|^2 below the clamp."""
+    r = runtime("clamp_idle")
+    assert r["wrong"] == 0 and r["idle"] > 0
