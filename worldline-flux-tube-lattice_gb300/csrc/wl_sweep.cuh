@@ -119,6 +119,26 @@ __device__ __forceinline__ int block_end(int q) {
   return q < 64 ? min(((q - 1) & ~7) + 9, 64) : (q & ~7) + 8;
 }
 
+// Groups of a walk in straight-line code: 4 where they fit the registers (smooth,
+// the scalar step profile: 5 % over 2 at 512 points per loop), 2 elsewhere (scalar
+// quadratic 1-4 % over 4, 9-12 % at four fluxes), 1 around a run-time node loop.  The
+// persistent kernel (MIXED) runs several kinds of unit on an SM at once, whose
+// code then competes for the instruction cache: 1 for the kinds that get 4 here
+// (served smooth and Gaussian requests 4.9e11 segments/s at 4, 5.4e11 at 2,
+// 5.57e11 at 1; the other kinds at 1 too 5.52e11).
+template <int P, bool FERM, int NINT, bool MIXED>
+constexpr int walk_unroll() {
+  if (NINT == 0) return 1;
+  if (NINT == 4 && (smooth_profile(P) || (P == kStep && !FERM))) return MIXED ? 1 : 4;
+  return 2;
+}
+static_assert(walk_unroll<kStep, false, 4, false>() == 4 &&
+                  walk_unroll<kStep, false, 4, true>() == 1 &&
+                  walk_unroll<kStep, true, 4, false>() == 2 &&
+                  walk_unroll<kQuadratic, false, 4, false>() == 2 &&
+                  walk_unroll<kSmoothWide, true, 4, false>() == 4,
+              "profiles as the comment names them");
+
 // One unit of a warp: instances [32 tile, +32), one per lane, over loops
 // [l0, l1).  PAIR: the lane walks loops l and l + 1 together as a packed pair:
 // every FP32 operation of a segment is one f32x2 operation on the two loops
@@ -144,18 +164,9 @@ template <int P, bool FERM, int NINT, bool PAIR, class Field = const FieldDev &>
 __device__ __forceinline__ bool warp_unit(const SweepArgs &A, int tile, int l0, int l1,
                                           size_t row, WarpStage &W) {
   using V = typename Vec<PAIR>::T;
-  constexpr int kStep = PAIR ? 2 : 1;          // loops walked together
-  constexpr int kPiece = kLandPts / kStep;     // points per staged piece
-  // groups in straight-line code: 4 where they fit the registers (smooth, the
-  // scalar step profile: 2-5 % over 2), 2 elsewhere (4 there up to 11 %
-  // slower), 1 around a run-time node loop.  The persistent kernel (Field by
-  // value) runs several kinds of unit on an SM at once, whose code then
-  // competes for the instruction cache: 1 for the kinds that get 4 here (served
-  // smooth and Gaussian requests 4.9e11 segments/s at 4, 5.4e11 at 2, 5.57e11
-  // at 1; the other kinds at 1 too 5.52e11)
-  constexpr bool kMixed = !std::is_reference<Field>::value;
-  constexpr bool kShort = NINT == 4 && (smooth_profile(P) || (P == kStep && !FERM));
-  constexpr int kUnroll = NINT == 0 ? 1 : kShort ? (kMixed ? 1 : 4) : 2;
+  constexpr int kLoops = PAIR ? 2 : 1;         // loops walked together
+  constexpr int kPiece = kLandPts / kLoops;    // points per staged piece
+  constexpr int kUnroll = walk_unroll<P, FERM, NINT, !std::is_reference<Field>::value>();
   const int lane = threadIdx.x & 31;
   const int slot = tile * 32 + lane;
   const bool live = slot < A.ninst;
@@ -166,7 +177,7 @@ __device__ __forceinline__ bool warp_unit(const SweepArgs &A, int tile, int l0, 
   Field F = A.field;  // by value where A is not in the constant bank
   const V cx = vset(V(), A.cx[ic]), cy = vset(V(), A.cy[ic]), s = vset(V(), A.rtT[ic]);
 
-  auto issue = [&](int l, int p0) {  // points p0.. of the kStep loops from l
+  auto issue = [&](int l, int p0) {  // points p0.. of the kLoops loops from l
     const uint32_t bytes = (uint32_t)(min(kPiece, A.ppl - p0) * (int)sizeof(float4));
     const bool two = PAIR && l + 1 < l1;
     mbar_arrive_expect_tx(W.bar, two ? 2 * bytes : bytes);
@@ -205,7 +216,7 @@ __device__ __forceinline__ bool warp_unit(const SweepArgs &A, int tile, int l0, 
         reinterpret_cast<float2 *>(W.comp)[i] = *reinterpret_cast<const float2 *>(W.land + i);
     }
     __syncwarp();
-    const int ln = last ? l + kStep : l, pn = last ? 0 : p0 + kPiece;
+    const int ln = last ? l + kLoops : l, pn = last ? 0 : p0 + kPiece;
     if (lane == 0 && ln < l1) issue(ln, pn);
 
     auto pt = [&](int p, V &x, V &y) {
@@ -298,7 +309,7 @@ __device__ __forceinline__ bool warp_unit(const SweepArgs &A, int tile, int l0, 
       }
       const df tq = {A.tqh[ic], A.tql[ic]};
 #pragma unroll 1
-      for (int h = 0; h < kStep; ++h) {  // per-loop epilogue of each half
+      for (int h = 0; h < kLoops; ++h) {  // per-loop epilogue of each half
         if (l + h >= l1) break;
         const df G[3] = {fast_two_sum(vlane(ph[0], h), -vlane(pc[0], h)),
                          fast_two_sum(vlane(ph[1], h), -vlane(pc[1], h)),
