@@ -986,22 +986,28 @@ __global__ void __launch_bounds__(128) loop_finish_kernel(const __grid_constant_
 // sums, since the sub-loops' accumulators are separate.  Bound by latency when
 // few (loop, instance) pairs leave the SMs with a few warps each: one instance
 // on 512 loops of 512 points, fixflux at 50 intervals, 1.06 -> 0.59 ms with two.
+//   LEAN: one warp per pair and no fingerprint, the form of launches that fill the
+// chip.  The role tests and hashes of the other took the light profiles from 32-40
+// to 40-48 registers and the lattice from 72 to 92, and with them the SM's warps:
+// 25 instances on 512 x 1820 points, lattice spinor, 224 -> 233 us.
 //   With A.fingerprint the warps also hash the points they read: EV() checks a
 // cached ensemble against that, and a pass of its own over the ensemble took
 // 20 us beside the 60 us of the sweep (5120 loops of 1024 points, 50
 // intervals); 79 such EV() sweeps of integrateT 10.8 -> 9.9 ms.
 //   (kSqRound / kSqFuse: the roundings the four calls were compiled to, written
 // out so that results keep their bits.)
-template <int P, bool FERM, int NINT>
+template <int P, bool FERM, int NINT, bool LEAN>
 __global__ void __launch_bounds__(kLoopWarps * 32)
     loopwarp_kernel(const __grid_constant__ LoopArgs A) {
   __shared__ float quarter[kLoopWarps][4];  // split: sums of the N/4 sub-loops
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int l = A.split ? blockIdx.x * (kLoopWarps / 2) + (w >> 1) : blockIdx.x * kLoopWarps + w;
-  const bool half = !A.split || !(w & 1), quarters = !A.split || (w & 1);
+  const bool split = !LEAN && A.split;
+  unsigned long long *const fingerprint = LEAN ? nullptr : A.fingerprint;
+  const int l = split ? blockIdx.x * (kLoopWarps / 2) + (w >> 1) : blockIdx.x * kLoopWarps + w;
+  const bool half = !split || !(w & 1), quarters = !split || (w & 1);
   const int inst = blockIdx.y;
   const bool on = l < A.Nl;  // whole warp
-  if (!A.split && !on) return;
+  if (!split && !on) return;
   const float cx = A.cx[inst], cy = A.cy[inst], s = A.rtT[inst];
   const FieldDev &F = A.field;
   const float2 *pts = reinterpret_cast<const float2 *>(A.loops + (size_t)(on ? l : 0) * A.ppl);
@@ -1019,30 +1025,45 @@ __global__ void __launch_bounds__(kLoopWarps * 32)
     if (on) img = image_range(A.bbox[l], s, cx, cy, F);
   float ph[3] = {0.f, 0.f, 0.f}, sp[3] = {0.f, 0.f, 0.f};
   unsigned long long hash = 0;
+  // a point that this group is the first to read: hashed before its segments, so
+  // that no coordinate lives through them
+  auto own = [&](int p, float &x, float &y) {
+    const float2 v = pt(p, x, y);
+    if (fingerprint) hash += point_hash(v, (size_t)l * A.ppl + p);
+  };
   for (int q = lane; q < nq; q += 32) {
     const int pa = (q == 0 ? A.ppl : 4 * q) - 4;
-    float2 v[4];
-    if (half) {
-      float zOx, zOy, P1x, P1y, P3x, P3y;
-      pt(pa + 3, zOx, zOy);
-      v[1] = pt(4 * q + 1, P1x, P1y);
-      v[3] = pt(4 * q + 3, P3x, P3y);
-      seg<P, FERM, NINT, kSqRound>(zOx, zOy, P1x, P1y, F, img, ph[0], sp[0]);
-      seg<P, FERM, NINT, kSqRound>(P1x, P1y, P3x, P3y, F, img, ph[0], sp[0]);
-    }
-    if (quarters) {
-      float zAx, zAy, zBx, zBy, P0x, P0y, P2x, P2y;
+    if constexpr (LEAN) {
+      float zAx, zAy, zBx, zBy, zOx, zOy, P0x, P0y, P1x, P1y, P2x, P2y, P3x, P3y;
       pt(pa, zAx, zAy);
       pt(pa + 2, zBx, zBy);
-      v[0] = pt(4 * q, P0x, P0y);
-      v[2] = pt(4 * q + 2, P2x, P2y);
+      pt(pa + 3, zOx, zOy);
+      pt(4 * q, P0x, P0y);
+      pt(4 * q + 1, P1x, P1y);
+      pt(4 * q + 2, P2x, P2y);
+      pt(4 * q + 3, P3x, P3y);
       seg<P, FERM, NINT, kSqFuse>(zAx, zAy, P0x, P0y, F, img, ph[2], sp[2]);
+      seg<P, FERM, NINT, kSqRound>(zOx, zOy, P1x, P1y, F, img, ph[0], sp[0]);
       seg<P, FERM, NINT, kSqRound>(zBx, zBy, P2x, P2y, F, img, ph[1], sp[1]);
-    }
-    if (A.fingerprint) {
-      const size_t p = (size_t)l * A.ppl + 4 * q;
-      if (half) hash += point_hash(v[1], p + 1) + point_hash(v[3], p + 3);
-      if (quarters) hash += point_hash(v[0], p) + point_hash(v[2], p + 2);
+      seg<P, FERM, NINT, kSqRound>(P1x, P1y, P3x, P3y, F, img, ph[0], sp[0]);
+    } else {
+      if (half) {
+        float zOx, zOy, P1x, P1y, P3x, P3y;
+        pt(pa + 3, zOx, zOy);
+        own(4 * q + 1, P1x, P1y);
+        own(4 * q + 3, P3x, P3y);
+        seg<P, FERM, NINT, kSqRound>(zOx, zOy, P1x, P1y, F, img, ph[0], sp[0]);
+        seg<P, FERM, NINT, kSqRound>(P1x, P1y, P3x, P3y, F, img, ph[0], sp[0]);
+      }
+      if (quarters) {
+        float zAx, zAy, zBx, zBy, P0x, P0y, P2x, P2y;
+        pt(pa, zAx, zAy);
+        pt(pa + 2, zBx, zBy);
+        own(4 * q, P0x, P0y);
+        own(4 * q + 2, P2x, P2y);
+        seg<P, FERM, NINT, kSqFuse>(zAx, zAy, P0x, P0y, F, img, ph[2], sp[2]);
+        seg<P, FERM, NINT, kSqRound>(zBx, zBy, P2x, P2y, F, img, ph[1], sp[1]);
+      }
     }
   }
 #pragma unroll
@@ -1053,11 +1074,11 @@ __global__ void __launch_bounds__(kLoopWarps * 32)
       if (FERM) sp[r] += __shfl_xor_sync(0xffffffffu, sp[r], off);
     }
   }
-  if (A.fingerprint) {
+  if (fingerprint) {
     for (int off = 16; off > 0; off >>= 1) hash += __shfl_xor_sync(0xffffffffu, hash, off);
-    if (lane == 0 && on) atomicAdd(A.fingerprint, hash);
+    if (lane == 0 && on) atomicAdd(fingerprint, hash);
   }
-  if (A.split) {
+  if (split) {
     if (lane == 0 && quarters) {
       quarter[w][0] = ph[1];
       quarter[w][1] = ph[2];
@@ -1168,9 +1189,14 @@ template <int P>
 cudaError_t loopwarp_dispatch(bool fermion, int nint, const LoopArgs &a, cudaStream_t s) {
   const int per = a.split ? kLoopWarps / 2 : kLoopWarps;  // loops per CTA
   const dim3 grid((a.Nl + per - 1) / per, a.ninst);
+  // a heavy profile's segments hold more registers than either form
+  const bool lean = !Profile<P>::kHeavy && !a.split && !a.fingerprint;
 #define WL_LOOP_CASE(FE, NI)                                                       \
   if (fermion == FE && (NI == 0 || nint == NI)) {                                  \
-    loopwarp_kernel<P, FE, NI><<<grid, kLoopWarps * 32, 0, s>>>(a);                \
+    if (lean)                                                                      \
+      loopwarp_kernel<P, FE, NI, !Profile<P>::kHeavy><<<grid, kLoopWarps * 32, 0, s>>>(a); \
+    else                                                                           \
+      loopwarp_kernel<P, FE, NI, false><<<grid, kLoopWarps * 32, 0, s>>>(a);       \
     return cudaGetLastError();                                                     \
   }
   if constexpr (!Profile<P>::kHeavy) {
