@@ -31,5 +31,5 @@ def test_clamped_widths_match_the_oracle(lam2, fe, mode):
     ref, S = O.eval_groups(loops, cx, cx, T, [1.0],
                            O.field("smooth", fermion=fe, nint=4, lambda2=lam2, mode=mode),
                            group=16, return_scale=True)
-    assert np.max(np.abs(g - ref) / np.maximum(np.abs(ref), 1e-2 * S)) < W_TOL
-    assert np.array_equal(g, b)
+    for w in (g, b):  # b sums its groups of 16 as one chunk, g as two
+        assert np.max(np.abs(w - ref) / np.maximum(np.abs(ref), 1e-2 * S)) < W_TOL
