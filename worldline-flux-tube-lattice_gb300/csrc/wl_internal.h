@@ -317,11 +317,4 @@ cudaError_t launch_vloops(uint64_t seed, int first, int Nl, int ppl, float4 *out
 
 constexpr int kInstArrays = 5;  // cx, cy, rtT, tq_hi, tq_lo
 
-// per CTA: each warp's landing zone and compact piece
-constexpr size_t sweep_smem_bytes() { return (size_t)kSweepWarps * kLandPts * (16 + 8); }
-// lattice at 4 intervals: landing zone, compact points, block boxes, loop totals
-constexpr size_t sweep_lat_smem_bytes() {
-  return (size_t)kSweepWarps * (kLandPts * 16 + (kLandPts + 8) * 16 + 8 * 16 + 24 * 32 * 4);
-}
-
 }  // namespace wl

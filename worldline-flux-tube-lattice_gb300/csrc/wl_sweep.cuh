@@ -33,14 +33,19 @@ static_assert(kSweepThreads == 32 * kFfWarps && kLoopWarps == kFfWarps,
               "fixflux queues: 4 warps per CTA");
 
 // ------------------------------------------------------ staging per warp --
-// A warp's staging area: the landing zone of its bulk copies and the compact
-// copy of a piece's coordinates that the lanes walk.  `copies` counts the
-// pieces this warp has waited for (its barrier's phase continues across units).
+// A warp's staging area: the landing zone of its bulk copies, the compact copy of
+// a piece's coordinates that the lanes walk, and for sweep_kernel's loop pairs the
+// first points of the loops and the chunk's running sums.  `copies` counts the pieces this
+// warp has waited for (its barrier's phase continues across units).
 struct WarpStage {
   float4 *land;   // [kLandPts] float4 points as the ensemble holds them
   float4 *comp;   // the piece's coordinates, laid out for its walk
   uint64_t *bar;  // the warp's mbarrier
   uint32_t copies;
+  // pairs: points 0..2 of the walked loops, as in comp
+  __device__ float4 *first() const { return land + kLandPts * 3 / 2; }
+  // pairs: [kMaxF][3][32 lanes]
+  __device__ double *sums() const { return reinterpret_cast<double *>(first() + 4); }
 };
 
 __device__ __forceinline__ void warp_stage_init(uint64_t *bar) {
@@ -80,6 +85,31 @@ __device__ __forceinline__ void put_loop(const SweepArgs &A, size_t row, int j, 
   o[0] = d0;
   o[n] = d1;
   o[2 * n] = d2;
+}
+
+// The same for sweep_kernel's loop pairs, a chunk's sums kept in the warp's shared memory
+// until its last loop (`last`).  Added to in global memory they took a round trip
+// per loop and flux, one after another (the stores may alias the next loads): 1024
+// Gaussian instances at four fluxes on 1024 loops of 64 points 321 -> 306 us.
+__device__ __forceinline__ void put_pair_loop(const SweepArgs &A, const WarpStage &W, size_t row,
+                                              int j, int ic, bool live, bool acc, bool last,
+                                              double d0, double d1, double d2) {
+  double *const s = W.sums() + j * 96 + (threadIdx.x & 31);
+  if (acc) {
+    d0 += s[0];
+    d1 += s[32];
+    d2 += s[64];
+  }
+  if (!last) {
+    s[0] = d0;
+    s[32] = d1;
+    s[64] = d2;
+  } else if (live) {
+    double *o = A.partial + (row * A.nF + j) * 3 * A.ninst + ic;
+    o[0] = d0;
+    o[A.ninst] = d1;
+    o[2 * (size_t)A.ninst] = d2;
+  }
 }
 
 // scalar and pair arithmetic of the walk under one name
@@ -166,7 +196,17 @@ __device__ __forceinline__ bool warp_unit(const SweepArgs &A, int tile, int l0, 
   using V = typename Vec<PAIR>::T;
   constexpr int kLoops = PAIR ? 2 : 1;         // loops walked together
   constexpr int kPiece = kLandPts / kLoops;    // points per staged piece
-  constexpr int kUnroll = walk_unroll<P, FERM, NINT, !std::is_reference<Field>::value>();
+  // the persistent kernel (Field by value) keeps the longer forms below: called
+  // units of long loops lose 3 % by the shorter ones (served smooth requests 8.04e11
+  // -> 7.82e11 segments/s, an uneven batch of six jobs 18.0 -> 18.6 ms)
+  constexpr bool kMixed = !std::is_reference<Field>::value;
+  constexpr int kUnroll = walk_unroll<P, FERM, NINT, kMixed>();
+  constexpr bool kSums = PAIR && !kMixed;  // put_pair_loop
+  // the loops' first points kept in shared memory for their closing segments; read
+  // again from the ensemble a pair waits for them (50 intervals: Gaussian scalar 3 %,
+  // smooth spinor 1 %), but the smooth scalar kernel at 50 compiles to a faster walk
+  // that way (3160 instances on 2048 x 1024 points 56.8 ms, 57.7 with them kept)
+  constexpr bool kFirst = kSums && !(smooth_profile(P) && !FERM && NINT == 50);
   const int lane = threadIdx.x & 31;
   const int slot = tile * 32 + lane;
   const bool live = slot < A.ninst;
@@ -209,7 +249,9 @@ __device__ __forceinline__ bool warp_unit(const SweepArgs &A, int tile, int l0, 
       for (int i = lane; i < np; i += 32) {
         const float2 a = *reinterpret_cast<const float2 *>(W.land + i);
         const float2 b = *reinterpret_cast<const float2 *>(W.land + o + i);
-        W.comp[i] = make_float4(a.x, b.x, a.y, b.y);
+        const float4 v = make_float4(a.x, b.x, a.y, b.y);
+        W.comp[i] = v;
+        if (kFirst && p0 == 0 && i < 3) W.first()[i] = v;
       }
     } else {
       for (int i = lane; i < np; i += 32)
@@ -280,17 +322,22 @@ __device__ __forceinline__ bool warp_unit(const SweepArgs &A, int tile, int l0, 
     }
 
     if (last) {  // last piece: closing segments back to points 1, 0, 2
-      // (read again from the ensemble: kept since the first piece they would
-      // hold six registers, twelve on a pair, through the whole walk)
+      // (kept since the first piece in registers they would take six, twelve on a
+      // pair, through the whole walk)
       V tp[3] = {zero, zero, zero}, ts[3] = {zero, zero, zero};
       const float2 *g = reinterpret_cast<const float2 *>(A.loops + (size_t)l * A.ppl);
       auto gpt = [&](int p, V &x, V &y) {
-        const float2 a = __ldg(&g[2 * p]);
-        if constexpr (PAIR) {
+        if constexpr (kFirst) {
+          const float4 v = W.first()[p];
+          x = fma2(s, make_float2(v.x, v.y), cx);
+          y = fma2(s, make_float2(v.z, v.w), cy);
+        } else if constexpr (PAIR) {
+          const float2 a = __ldg(&g[2 * p]);
           const float2 b = l + 1 < l1 ? __ldg(&g[2 * ((size_t)A.ppl + p)]) : a;
           x = fma2(s, make_float2(a.x, b.x), cx);
           y = fma2(s, make_float2(a.y, b.y), cy);
         } else {
+          const float2 a = __ldg(&g[2 * p]);
           x = fmaf(s, a.x, cx);
           y = fmaf(s, a.y, cy);
         }
@@ -321,7 +368,11 @@ __device__ __forceinline__ bool warp_unit(const SweepArgs &A, int tile, int l0, 
         const bool acc = !A.per_loop && l + h > l0;
         loop_epilogue<FERM>(G, H, A.cph_hi, A.cph_lo, A.csp_hi, A.csp_lo, tq, A.nF,
                             [&](int j, double w0, double w1, double w2) {
-                              if (live) put_loop(A, at, j, ic, acc, w0, w1, w2);
+                              if constexpr (kSums)
+                                put_pair_loop(A, W, at, j, ic, live, acc,
+                                              A.per_loop || l + h == l1 - 1, w0, w1, w2);
+                              else if (live)
+                                put_loop(A, at, j, ic, acc, w0, w1, w2);
                             });
       }
     }
@@ -793,11 +844,13 @@ __device__ __forceinline__ bool warp_unit_lat(const SweepArgs &A, int tile, int 
 // ------------------------------------------------------------- kernels --
 // bytes of dynamic shared memory per warp
 constexpr int kStageBytes = kLandPts * 16 + kLandPts * 8;
+constexpr int kPairStageBytes = kStageBytes + 4 * 16 + kMaxF * 3 * 32 * 8;
 constexpr int kLatStageBytes =
     kLandPts * 16 + kLatPts * 16 + kLatTotRows * 32 * 4 + kLatNSub * 16;
-static_assert(kSweepWarps * kStageBytes == (int)sweep_smem_bytes() &&
-                  kSweepWarps * kLatStageBytes == (int)sweep_lat_smem_bytes(),
-              "the launch's shared memory");
+template <int P, bool PAIR>
+constexpr int stage_bytes() {
+  return !PAIR ? kStageBytes : P == kLattice ? kLatStageBytes : kPairStageBytes;
+}
 
 __device__ __forceinline__ WarpStage warp_stage(unsigned char *smem, uint64_t *bars, int bytes) {
   const int w = threadIdx.x >> 5;
@@ -845,7 +898,7 @@ __global__ void __launch_bounds__(kSweepThreads, sweep_min_ctas<P>())
   const unsigned u = kLat4 ? item % (unsigned)A.n_units : item / (unsigned)A.n_tiles;
   const int tile = kLat4 ? item / (unsigned)A.n_units : item % (unsigned)A.n_tiles;
   if (u >= (unsigned)A.n_units || tile >= A.n_tiles) return;  // whole warp
-  WarpStage W = warp_stage(smem, bars, kLat4 ? kLatStageBytes : kStageBytes);
+  WarpStage W = warp_stage(smem, bars, stage_bytes<P, PAIR>());
   warp_stage_init(W.bar);
   int l0, l1;
   const size_t row = unit_loops(A, u, l0, l1);
@@ -1128,7 +1181,7 @@ cudaError_t sweep_launch(SweepArgs a, cudaStream_t s) {
   const long long items = (long long)a.n_tiles * a.n_units;
   const unsigned ctas = sweep_ctas(items);
   if (!ctas) return cudaErrorInvalidConfiguration;
-  constexpr size_t smem = kLat4 ? sweep_lat_smem_bytes() : sweep_smem_bytes();
+  constexpr size_t smem = (size_t)kSweepWarps * stage_bytes<P, PAIR>();
   auto k = sweep_kernel<P, FERM, NINT, PAIR>;
   if (smem > 48 * 1024) {  // a per-device attribute
     const cudaError_t e =
@@ -1146,7 +1199,7 @@ cudaError_t sweep_parts_launch(SweepArgs a, cudaStream_t s) {
   const long long items = loops * a.parts * a.n_tiles;
   const unsigned ctas = sweep_ctas(items);
   if (!ctas) return cudaErrorInvalidConfiguration;
-  sweep_part_kernel<P, FERM><<<ctas, kSweepThreads, sweep_smem_bytes(), s>>>(a);
+  sweep_part_kernel<P, FERM><<<ctas, kSweepThreads, kSweepWarps * kStageBytes, s>>>(a);
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   loop_finish_kernel<P, FERM><<<(unsigned)((loops * a.ninst + 127) / 128), 128, 0, s>>>(a);
