@@ -1012,6 +1012,15 @@ __device__ __forceinline__ double coshm1_df(df x) {
   return 0.5 * exp((double)a + (double)e) - 1.0;
 }
 
+// cosm1_df and coshm1_df as calls of one copy (loop_epilogue's SMALL)
+template <bool ONE>
+__device__ __noinline__ float cosm1_called(df x) {
+  return cosm1_df(x);
+}
+template <bool ONE>
+__device__ __noinline__ double coshm1_called(df x) {
+  return coshm1_df(x);
+}
 // Per-loop factors of EVMean (Integrand.c:352-390) from the sub-loop phases
 // p[k] and spin exponents q[k] (k: N/2, N/4b, N/4a), returned as deviations
 // d = w - 1 (the sums of deviations keep <W> - 1 accurate):
@@ -1019,13 +1028,14 @@ __device__ __forceinline__ double coshm1_df(df x) {
 //   w1 = W_N/2 = cos(p0)                [* cosh(q0)]
 //   w2 = W_N/4 = cos((p1+p2)/2)         [* cosh(same of q)]
 // with the reference's 1e10 sentinel when a spin exponent truncates above 600.
-template <bool FERM>
+template <bool FERM, bool ONE>
 __device__ __forceinline__ void wfactors(const df p[3], const df q[3], double &d0, double &d1,
                                          double &d2) {
   const df nb4 = df_add(p[1], p[2]);
-  const float c0 = cosm1_df(df_add(df_scale2(p[0], 0.5f), df_scale2(nb4, 0.25f)));
-  const float c1 = cosm1_df(p[0]);
-  const float c2 = cosm1_df(df_scale2(nb4, 0.5f));
+  const df a0 = df_add(df_scale2(p[0], 0.5f), df_scale2(nb4, 0.25f)), a2 = df_scale2(nb4, 0.5f);
+  const float c0 = ONE ? cosm1_called<ONE>(a0) : cosm1_df(a0);
+  const float c1 = ONE ? cosm1_called<ONE>(p[0]) : cosm1_df(p[0]);
+  const float c2 = ONE ? cosm1_called<ONE>(a2) : cosm1_df(a2);
   d0 = c0;
   d1 = c1;
   d2 = c2;
@@ -1037,9 +1047,10 @@ __device__ __forceinline__ void wfactors(const df p[3], const df q[3], double &d
       d2 = (1.0 + (double)c2) * 1.0e10 - 1.0;
     } else {
       // cos * cosh - 1 = (cos - 1) cosh + (cosh - 1)
-      const double h0 = coshm1_df(df_add(df_scale2(q[0], 0.5f), df_scale2(nb4f, 0.25f)));
-      const double h1 = coshm1_df(q[0]);
-      const double h2 = coshm1_df(df_scale2(nb4f, 0.5f));
+      const df b0 = df_add(df_scale2(q[0], 0.5f), df_scale2(nb4f, 0.25f)), b2 = df_scale2(nb4f, 0.5f);
+      const double h0 = ONE ? coshm1_called<ONE>(b0) : coshm1_df(b0);
+      const double h1 = ONE ? coshm1_called<ONE>(q[0]) : coshm1_df(q[0]);
+      const double h2 = ONE ? coshm1_called<ONE>(b2) : coshm1_df(b2);
       d0 = (double)c0 * (1.0 + h0) + h0;
       d1 = (double)c1 * (1.0 + h1) + h1;
       d2 = (double)c2 * (1.0 + h2) + h2;
@@ -1054,13 +1065,24 @@ __device__ __forceinline__ void wfactors(const df p[3], const df q[3], double &d
 // instance's, so the phase is F G h/3 and the spin exponent 2 F T sum/(N/2)
 // (N/2 loop) or 2 F T sum/(N/4) (N/4 loops).  add(j, d0, d1, d2) receives the
 // W factors minus one (accumulated in FP64 by the caller).
-template <bool FERM, class Add>
+//   SMALL: the flux values by one copy of the code, and for spinor QED one called
+// copy of the cosine and of the cosh, for walks of a few nodes: the warps of an SM
+// are at different places of their loops, and the epilogue's code competes with the
+// walks' for the instruction cache (smooth spinor, 1024 instances at four fluxes on
+// 1024 loops of 128 points: no instruction 0.46 cycles per issue with the warps of a
+// CTA in step, 0.84-1.08 apart).  By whole chunks there, three calls in flight, the
+// former tiles' time over this: spinor 0.90 -> 1.02 (0.98 with the factors inlined),
+// 0.88 -> 1.04 at 64 points; scalar 0.94 -> 0.98 and 0.92 -> 0.97 (as calls 0.95 and
+// 0.94).  At 50 intervals the long form is 1 to 6 % faster.
+// (Both written out: sharing the body through a lambda compiled the persistent
+// kernel's smooth units to 3 % slower code, 20.8 -> 21.5 ms.)
+template <bool FERM, bool SMALL = false, class Add>
 __device__ __forceinline__ void loop_epilogue(const df G[3], const df H[3], const float *cph_hi,
                                               const float *cph_lo, const float *csp_hi,
                                               const float *csp_lo, df tq, int nF, Add &&add) {
-#pragma unroll
-  for (int j = 0; j < kMaxF; ++j) {
-    if (j < nF) {
+  if constexpr (SMALL) {
+#pragma unroll 1
+    for (int j = 0; j < nF; ++j) {
       const df cph = {cph_hi[j], cph_lo[j]};
       df p[3], q[3];
 #pragma unroll
@@ -1074,8 +1096,29 @@ __device__ __forceinline__ void loop_epilogue(const df G[3], const df H[3], cons
         q[0] = q[1] = q[2] = df{0.0f, 0.0f};
       }
       double w0, w1, w2;
-      wfactors<FERM>(p, q, w0, w1, w2);
+      wfactors<FERM, FERM>(p, q, w0, w1, w2);
       add(j, w0, w1, w2);
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < kMaxF; ++j) {
+      if (j < nF) {
+        const df cph = {cph_hi[j], cph_lo[j]};
+        df p[3], q[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) p[k] = df_mul(cph, G[k]);
+        if (FERM) {
+          const df csp = df_mul(df{csp_hi[j], csp_lo[j]}, tq);
+          q[0] = df_mul(csp, H[0]);
+          q[1] = df_scale2(df_mul(csp, H[1]), 2.0f);
+          q[2] = df_scale2(df_mul(csp, H[2]), 2.0f);
+        } else {
+          q[0] = q[1] = q[2] = df{0.0f, 0.0f};
+        }
+        double w0, w1, w2;
+        wfactors<FERM, false>(p, q, w0, w1, w2);
+        add(j, w0, w1, w2);
+      }
     }
   }
 }

@@ -366,7 +366,7 @@ __device__ __forceinline__ bool warp_unit(const SweepArgs &A, int tile, int l0, 
                          fast_two_sum(vlane(sp[2], h), -vlane(sc[2], h))};
         const size_t at = A.per_loop ? row + (l - l0) + h : row;
         const bool acc = !A.per_loop && l + h > l0;
-        loop_epilogue<FERM>(G, H, A.cph_hi, A.cph_lo, A.csp_hi, A.csp_lo, tq, A.nF,
+        loop_epilogue<FERM, kSums && NINT != 50>(G, H, A.cph_hi, A.cph_lo, A.csp_hi, A.csp_lo, tq, A.nF,
                             [&](int j, double w0, double w1, double w2) {
                               if constexpr (kSums)
                                 put_pair_loop(A, W, at, j, ic, live, acc,
