@@ -423,6 +423,38 @@ static void clamp_idle() {
   say("idle", idle);
 }
 
+// which launches are cut into single loops: 10 alone on the chip, 1 among others
+static void cut_rule() {
+  struct Case {
+    const char *name;
+    int profile, fermion, nint, ninst, nF, Nl, ppl, chunk;
+  };
+  const Case cases[] = {
+      {"short_loops_full_chip", WL_PROFILE_SMOOTH, 0, 4, 1024, 1, 1024, 64, 8},
+      {"four_fluxes", WL_PROFILE_SMOOTH, 0, 4, 512, 4, 1024, 256, 8},
+      {"scan", WL_PROFILE_SMOOTH, 1, 4, 96, 3, 5120, 2048, 8},
+      {"long_loops_full_chip", WL_PROFILE_SMOOTH, 0, 4, 1024, 1, 1024, 1024, 8},
+      {"heavier_nodes", WL_PROFILE_GAUSSIAN, 1, 16, 333, 2, 1500, 516, 5},
+      {"just_above_a_wave", WL_PROFILE_SMOOTH, 0, 4, 513, 2, 1152, 232, 8},
+      {"few_units", WL_PROFILE_SMOOTH, 0, 4, 40, 4, 1024, 64, 8},
+      {"many_waves", WL_PROFILE_SMOOTH, 1, 4, 8192, 3, 5120, 2048, 8}};
+  for (const Case &k : cases) {
+    wl::SweepArgs a;
+    memset(&a, 0, sizeof(a));
+    a.ninst = k.ninst;
+    a.nF = k.nF;
+    a.ppl = k.ppl;
+    a.chunk_loops = k.chunk;
+    a.n_chunks = k.Nl / k.chunk;
+    const double items = wl::sweep_chunk_items(a, k.profile, k.nint);
+    wl::sweep_units(a, k.profile, k.fermion, k.nint, items, true);
+    const int alone = a.per_loop;
+    wl::sweep_units(a, k.profile, k.fermion, k.nint, items, false);
+    say(k.name, 10 * alone + a.per_loop);
+    if (a.n_units != (k.Nl + a.unit_loops - 1) / a.unit_loops) exit(4);
+  }
+}
+
 int main(int argc, char **argv) {
   const std::string s = argc > 1 ? argv[1] : "";
   wl_ctx *c = nullptr;
@@ -435,6 +467,7 @@ int main(int argc, char **argv) {
   else if (s == "ev_lattice") ev_lattice(c);
   else if (s == "sweep_grid") sweep_grid();
   else if (s == "clamp_idle") clamp_idle();
+  else if (s == "cut_rule") cut_rule();
   else return 3;
   wl_ctx_destroy(c);
   return 0;

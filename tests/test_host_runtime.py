@@ -75,3 +75,12 @@ def test_the_clamp_is_left_out_only_where_it_changes_no_bit(runtime):
     """smooth_clamp_idle() itself, against float32 sums over |z|^2 below the clamp."""
     r = runtime("clamp_idle")
     assert r["wrong"] == 0 and r["idle"] > 0
+
+
+def test_which_launches_are_cut_into_single_loops(runtime):
+    """(10: a launch alone on the chip, 1: one among others.)  Full chips of short
+    loops, or of several fluxes, keep whole chunks: their loops' sums would cost up
+    to a quarter of the walk."""
+    assert runtime("cut_rule") == {"short_loops_full_chip": 0, "four_fluxes": 10, "scan": 11,
+                                   "long_loops_full_chip": 11, "heavier_nodes": 11,
+                                   "just_above_a_wave": 10, "few_units": 11, "many_waves": 0}

@@ -966,10 +966,11 @@ static int eval_prologue(wl_ctx *ctx, int handle, const wl_field *field, int nin
 // Sweep + reduction on the context stream; instances are already staged in
 // ctx->inst as [cx | cy | rtT | tq].  Outputs are device pointers (may be
 // NULL).  Returns after enqueueing, its kernels counted in last_launches.
+// alone: the caller waits for the results (sweep_units).
 static int run_eval(wl_ctx *ctx, const Ensemble &e, int kprof, const FieldDev &fd,
                     const float4 *bbox, const wl_field *field, int ninst, int nF,
                     const double *host_F, int group, double *dg, double *dm, double *ds,
-                    double *status_out) {
+                    double *status_out, bool alone) {
   const bool fermion = field->fermion != 0;
   const int nint = field->nint;
   const bool use_sweep = ninst >= 32;
@@ -996,7 +997,7 @@ static int run_eval(wl_ctx *ctx, const Ensemble &e, int kprof, const FieldDev &f
     a.nF = nF;
     a.chunk_loops = e.Nl / n_chunks;
     a.n_chunks = n_chunks;
-    wl::sweep_units(a, kprof, fermion, nint, wl::sweep_chunk_items(a, kprof, nint));
+    wl::sweep_units(a, kprof, fermion, nint, wl::sweep_chunk_items(a, kprof, nint), alone);
     // loop by loop needs chunk_loops times the memory: by chunks if there is none
     if (a.per_loop && ctx->partial.reserve((size_t)e.Nl * nF * 3 * ninst) != cudaSuccess) {
       cudaGetLastError();
@@ -1093,7 +1094,7 @@ int wl_eval(wl_ctx *ctx, int handle, const wl_field *field, int ninst, const dou
   const float4 *bb = nullptr;
   if (kprof == wl::kLattice && (r = ensure_bbox(ctx, handle, &bb))) return r;
   if ((r = run_eval(ctx, e, kprof, fd, bb, field, ninst, nF, host_F, group, dg, dm, ds,
-                    dg + nout)))
+                    dg + nout, true)))
     return r;
   const size_t nm = (size_t)ninst * nF;
   return read_results(ctx, dg, nout, {{out_group, nm * ng}, {out_mean, nm}, {out_sem, nm}});
@@ -1128,7 +1129,7 @@ int wl_eval_device(wl_ctx *ctx, int handle, const wl_field *field, int ninst,
   const float4 *bb = nullptr;
   if (kprof == wl::kLattice && (r = ensure_bbox(ctx, handle, &bb))) return r;
   if ((r = run_eval(ctx, e, kprof, fd, bb, field, ninst, nF, host_F, group, dev_out_group,
-                    dev_out_mean, dev_out_sem, nullptr)))
+                    dev_out_mean, dev_out_sem, nullptr, false)))
     return r;
   ctx->last_launches += 1;  // the instance setup
   return WL_OK;
@@ -1291,7 +1292,7 @@ static int tint_run(wl_ctx *ctx, int handle, const wl_field *field, int nrho,
   const float4 *bb = nullptr;
   if (kprof == wl::kLattice && (r = ensure_bbox(ctx, handle, &bb))) return r;
   if ((r = run_eval(ctx, e, kprof, fd, bb, field, ninst, nF, host_F, group, dg, nullptr,
-                    nullptr, nullptr)))
+                    nullptr, nullptr, true)))
     return r;
   // aux: rho | T | w | F | Ig | leff | err | status | igrand
   const size_t n_ig = (size_t)nrho * nF * ng, n_le = (size_t)nrho * nF;

@@ -112,18 +112,30 @@ inline double sweep_chunk_items(const SweepArgs &a, int kprof, int nint) {
 // few units to fill the chip evenly, into the smallest units (a loop, or the
 // two of a packed pair) whose loops are stored one by one; the reduction adds
 // them in the same order, so a result does not depend on the choice.
-//   items: the launch's units by whole chunks.  Chunks leave about half a wave
-// of warps idle at the end, 0.5 / waves of the time; loop by loop costs 48 nF
-// bytes of HBM traffic per (loop, instance), 6 nF / ppl of the time of its ppl
-// segments at the measured rates (8.5e11 segments/s of weight 1, 6.8 TB/s).
-// Above 16 waves the partial sums would also outgrow the gain (0.24 GB per flux
-// value at wl_eval's 8 loops per chunk; a batch's larger chunks: batch_plan).  Measured: 96 instances x 3 fluxes on 5120 x 2048 points (1 wave)
-// 1.20 ms against 3.14 ms in 128-thread tiles of 256 instances.
-inline void sweep_units(SweepArgs &a, int kprof, int fermion, int nint, double items) {
+//   items: the launch's units by whole chunks, w = items / kSweepSlots waves of
+// them.  Chunks leave part of the last wave idle: a launch alone on the chip gains
+// 10 % from single loops at 0.84 waves or just above one, 4 % at 1.7, and most of
+// the chip below a quarter; one beside other launches, which fill the idle part,
+// nothing.  Single loops cost 48 nF bytes of traffic per (loop, instance) and 3 nF
+// of the reduction's FP64 additions, which in a chunk's walk overlap its FP32 work:
+// with x = nF / (ppl weight), among others 28 % of the time at x = 1/16, 9-14 % at
+// 1/64, 3-4 % at 1/128, 1 % at 1/256.  alone: the call waits for its results, so
+// its launches share the chip with other contexts' only; the lines lie where the
+// two sides meet alone (0.012) and where a launch among others loses at most 3 %
+// (0.005; the Gaussian profile's longer walks wait for instructions by chunks,
+// spinor, 1024 instances x 64 points 194 us by single loops, 208 by chunks: 0.015
+// for it).  Smooth scalar on 1024 loops, three wl_eval_device calls in flight, by
+// single loops -> chunks: 1024 instances x 64 points 92 -> 80 us, 512 x 4 F x 256
+// points 176 -> 156; 96 instances x 3 F on 5120 x 2048 stay single loops (1.20 ms,
+// 3.14 in 128-thread tiles of 256 instances).  Above 16 waves the sums would also
+// outgrow the gain (0.24 GB per flux value at wl_eval's 8 loops per chunk; a
+// batch's larger chunks: batch_plan).
+inline void sweep_units(SweepArgs &a, int kprof, int fermion, int nint, double items,
+                        bool alone = true) {
   const int loops = a.n_chunks * a.chunk_loops, unit = sweep_loop_pairs(kprof, nint) ? 2 : 1;
-  const bool split = items <= 16.0 * kSweepSlots &&
-                     items * 12.0 * a.nF <
-                         (double)kSweepSlots * a.ppl * profile_weight(kprof, fermion, nint);
+  const double w = items / kSweepSlots, x = a.nF / (a.ppl * profile_weight(kprof, fermion, nint));
+  const double line = kprof == kGaussian ? 0.015 : alone ? 0.012 : 0.005;
+  const bool split = w <= 16.0 && x * w * (w < 1.0 ? w : 1.0) < line;
   a.per_loop = a.chunk_loops == 1 || split;
   a.unit_loops = a.per_loop ? unit : a.chunk_loops;
   a.n_units = (loops + a.unit_loops - 1) / a.unit_loops;
