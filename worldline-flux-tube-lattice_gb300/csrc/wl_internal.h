@@ -1,5 +1,5 @@
 // wl_internal.h -- launch interfaces between the C-ABI runtime (wl_api.cpp)
-// and the kernels (wl_sweep.cu, wl_loopwarp.cu, wl_misc.cu).
+// and the kernels (wl_sweep_*.cu, wl_batch.cu, wl_misc.cu, wl_tint.cu).
 #pragma once
 
 #include <cuda_runtime.h>
@@ -57,10 +57,7 @@ inline __host__ __device__ bool light_profile(int kprof) {
   return kprof == kSmooth || kprof == kStep || kprof == kQuadratic || kprof == kGaussian;
 }
 // two loops per lane as packed f32x2 pairs (wl_sweep.cuh)
-inline __host__ __device__ bool sweep_loop_pairs(int kprof, int nint) {
-  (void)nint;
-  return light_profile(kprof);
-}
+inline __host__ __device__ bool sweep_loop_pairs(int kprof) { return light_profile(kprof); }
 // instances per warp (the lattice at 4 intervals: two per lane)
 inline __host__ __device__ int warp_instances(int kprof, int nint) {
   return nint == 4 && kprof == kLattice ? 64 : 32;
@@ -71,11 +68,16 @@ inline __host__ __device__ int sweep_tile_instances(int kprof, int nint) {
 }
 
 // Device time of one tile-point relative to the smooth profile at 4
-// intervals (tile order, processor-sharing split and rate estimates only): the
-// node count times the profile's cost relative to the smooth one at the same
-// interval count, measured on the GB300 through wl_eval (512 instances on
-// Nl 1024 x ppl 1024, scalar QED) at 4, 8 and 50 intervals and interpolated
-// linearly in nint between them (flat outside).
+// intervals (tile order, the cut into single loops, processor-sharing split and
+// rate estimates): the node count times the profile's cost relative to the smooth
+// one at the same interval count, interpolated linearly in nint between 4, 8 and
+// 50 (flat outside).  The figures were measured with the CTA tiles (512 instances
+// on Nl 1024 x ppl 1024, scalar QED); with the warp units the ratios are, in that
+// order, Gaussian 2.1, 2.1, 2.6, lattice at a = 5 lambda 12, 31, 40, periodic 30,
+// 30, 34, spline 16, 15, 21, fixflux 73, 70, 91, step and quadratic 1.1 to 1.4.
+// They stay because sweep_units' lines are drawn in them and a batch's order by
+// the new ones is no better (six uneven jobs 17.9 -> 18.3 ms: Gaussian units ahead
+// of smooth ones of the same length).
 inline double profile_weight(int kprof, int fermion, int nint) {
   double r[3] = {1.0, 1.0, 1.0};  // at 4, 8, 50 intervals
   switch (kprof) {
@@ -132,7 +134,7 @@ inline double sweep_chunk_items(const SweepArgs &a, int kprof, int nint) {
 // batch's larger chunks: batch_plan).
 inline void sweep_units(SweepArgs &a, int kprof, int fermion, int nint, double items,
                         bool alone = true) {
-  const int loops = a.n_chunks * a.chunk_loops, unit = sweep_loop_pairs(kprof, nint) ? 2 : 1;
+  const int loops = a.n_chunks * a.chunk_loops, unit = sweep_loop_pairs(kprof) ? 2 : 1;
   const double w = items / kSweepSlots, x = a.nF / (a.ppl * profile_weight(kprof, fermion, nint));
   const double line = kprof == kGaussian ? 0.015 : alone ? 0.012 : 0.005;
   const bool split = w <= 16.0 && x * w * (w < 1.0 ? w : 1.0) < line;

@@ -137,8 +137,8 @@ __device__ TNode igrand_d(TintArgs A, double rho, double T, double F) {
   return n;
 }
 
-// One CTA per (rho, F): the field and the regime of every proper time once,
-// one thread per T (they do not depend on the group), then one thread per group
+// One CTA per (rho, F): the field and the regime at every proper time, one thread
+// per T (not again for every group), then one thread per group
 // for its T integral, and one for L_eff and its jackknife error over nbins bins.
 // Bound by FP64 latency: one thread per (rho, F, group) evaluated every T's
 // exponentials for itself, 395 us for 64 rho x 3 F x 40 groups x 128 T and 214
